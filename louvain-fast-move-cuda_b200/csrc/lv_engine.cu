@@ -415,17 +415,22 @@ class Run {
       ho[1] = n_;
     }
     allocate(G_, n_, E64);
-    const cudaMemcpyKind kin = in_mem == LV_MEM_DEVICE ? cudaMemcpyDeviceToDevice : cudaMemcpyHostToDevice;
-    if (w) LV_CUDA(cudaMemcpyAsync(D.w, w, (size_t)E * 4, kin, st));
-    choose_weight_mode(w != nullptr);
-    LV_CUDA(cudaMemcpyAsync(D.col, col, (size_t)E * 4, kin, st));
-    LV_CUDA(cudaMemcpyAsync(row64(), row_ptr, (size_t)(n + 1) * 8, kin, st));
+    // host arrays are uploaded into the engine's buffers; device arrays are read where they lie
+    // (k_prep writes the engine's copy of the columns and weights as it validates them)
+    PrepIn in{reinterpret_cast<const long long*>(row_ptr), reinterpret_cast<const uint32_t*>(col), w, nullptr, 0};
+    if (in_mem != LV_MEM_DEVICE) {
+      if (w) LV_CUDA(cudaMemcpyAsync(D.w, w, (size_t)E * 4, cudaMemcpyHostToDevice, st));
+      LV_CUDA(cudaMemcpyAsync(D.col, col, (size_t)E * 4, cudaMemcpyHostToDevice, st));
+      LV_CUDA(cudaMemcpyAsync(row64(), row_ptr, (size_t)(n + 1) * 8, cudaMemcpyHostToDevice, st));
+      in = uploaded(w != nullptr);
+    }
+    choose_weight_mode(in.wf);
     long long* doffs = nullptr;
     if (G > 1) {
       doffs = dalloc<long long>(ctx, owned, (size_t)G + 1, st);
       LV_CUDA(cudaMemcpyAsync(doffs, ho.data(), (G + 1) * 8, cudaMemcpyHostToDevice, st));
     }
-    prepare(ho, doffs, w != nullptr);
+    prepare(ho, doffs, in);
   }
 
   // A batch assembled from separate host graphs (local numbering each): every piece is
@@ -467,7 +472,9 @@ class Run {
     LV_CUDA(cudaMemcpyAsync(D.col, col, (size_t)E * 4, cudaMemcpyHostToDevice, st));
     LV_CUDA(cudaMemcpyAsync(row64(), row_ptr, (size_t)(n + 1) * 8, cudaMemcpyHostToDevice, st));
     const std::vector<int64_t> ho = {0, n_};
-    prepare(ho, nullptr, true, integer ? reinterpret_cast<const uint32_t*>(D.wB) : nullptr);
+    PrepIn in = uploaded(!integer);
+    if (integer) in.wu = reinterpret_cast<const uint32_t*>(D.wB);
+    prepare(ho, nullptr, in);
     // the checkpoint's vertex map and counters replace the fresh run's
     LV_CUDA(cudaMemcpyAsync(D.best, best, (size_t)n0 * 4, cudaMemcpyHostToDevice, st));
     const uint32_t lv_it[2] = {(uint32_t)level, (uint32_t)iterations};
@@ -501,11 +508,16 @@ class Run {
     LV_CUDA(cudaMemcpyAsync(doffs + G + 1, eo.data(), (G + 1) * 8, cudaMemcpyHostToDevice, st));
     k_rebase_pieces<<<ctx->sms * 4, 256, 0, st>>>(r64, D.col, doffs, doffs + G + 1, G, n, E);
     ++launches;
-    choose_weight_mode(weighted);
-    prepare(ho, doffs, weighted);
+    const PrepIn in = uploaded(weighted);
+    choose_weight_mode(in.wf);
+    prepare(ho, doffs, in);
   }
 
  private:
+  // k_prep's view of an input uploaded into the run's own buffers
+  PrepIn uploaded(bool weighted) {
+    return PrepIn{row64(), D.col, weighted ? reinterpret_cast<const float*>(D.w) : nullptr, nullptr, 0};
+  }
   long long* row64() { return reinterpret_cast<long long*>(D.cd); }  // (n+1) x 8 B, free until aggregation
 
   void allocate(uint32_t G_, int64_t n_, int64_t E64, int64_t n0_ = -1) {
@@ -575,14 +587,14 @@ class Run {
     bind();
   }
 
-  // Integer or float semantics (the weights, if any, are already in D.w), then the bin tables.
-  void choose_weight_mode(bool weighted) {
+  // Integer or float semantics (w: the weights in device memory, or nullptr), then the bin tables.
+  void choose_weight_mode(const float* w) {
     int wm = cfg.weight_mode;
-    if (!weighted) wm = LV_WEIGHTS_INTEGER;
+    if (!w) wm = LV_WEIGHTS_INTEGER;
     if (wm == LV_WEIGHTS_AUTO) {
       uint32_t* flag = reinterpret_cast<uint32_t*>(D.partials);
       LV_CUDA(cudaMemsetAsync(flag, 0, 4, st));
-      k_weights_integral<<<ctx->sms * 4, 256, 0, st>>>(reinterpret_cast<const float*>(D.w), E, flag);
+      k_weights_integral<<<ctx->sms * 4, 256, 0, st>>>(w, E, flag);
       ++launches;
       LV_CUDA(cudaMemcpyAsync(pinned, flag, 4, cudaMemcpyDeviceToHost, st));
       sync();
@@ -599,8 +611,7 @@ class Run {
   }
 
   // Control block, graph states, graph ids, degrees and totals, then the first level.
-  void prepare(const std::vector<int64_t>& ho, const long long* doffs, bool weighted,
-               const uint32_t* wu = nullptr) {
+  void prepare(const std::vector<int64_t>& ho, const long long* doffs, PrepIn in) {
     LV_CUDA(cudaMemsetAsync(D.ctrl, 0, sizeof(Ctrl), st));
     LV_CUDA(cudaMemsetAsync(D.gs, 0, sizeof(GraphState) * G, st));
     Ctrl hc{};
@@ -624,12 +635,18 @@ class Run {
       LV_CUDA(cudaMemcpyAsync(D.gid0, D.gid, (size_t)n * 4, cudaMemcpyDeviceToDevice, st));
       ++launches;
     }
-    const float* wf = weighted && !wu ? reinterpret_cast<const float*>(D.w) : nullptr;
     iota_best();
-    if (wint) k_prep<true><<<grid_n, 256, 0, st>>>(Dd, row64(), wf, wu, n, E);
-    else k_prep<false><<<grid_n, 256, 0, st>>>(Dd, row64(), wf, wu, n, E);
-    if (wint) k_prep_long<true><<<ctx->sms * 4, 512, 0, st>>>(Dd, wf, wu);
-    else k_prep_long<false><<<ctx->sms * 4, 512, 0, st>>>(Dd, wf, wu);
+    in.keep_w = cfg.refine ? 1 : 0;
+    if (!in.wf && !in.wu) {
+      k_prep_unit<<<grid_n, 256, 0, st>>>(Dd, in, n, E);
+      k_prep_unit_long<<<grid_n, 256, 0, st>>>(Dd, in, n);
+    } else if (wint) {
+      k_prep<true><<<grid_n, 256, 0, st>>>(Dd, in, n, E);
+      k_prep_long<true><<<ctx->sms * 4, 512, 0, st>>>(Dd, in);
+    } else {
+      k_prep<false><<<grid_n, 256, 0, st>>>(Dd, in, n, E);
+      k_prep_long<false><<<ctx->sms * 4, 512, 0, st>>>(Dd, in);
+    }
     if (wint) k_prep_total<true><<<1, 256, 0, st>>>(Dd);
     else k_prep_total<false><<<1, 256, 0, st>>>(Dd);
     launches += 4;
@@ -1510,7 +1527,10 @@ lv_status lv_community_get_graph(lv_community* c, int64_t* row_ptr, int32_t* col
     std::vector<double> hk(r.n);
     LV_CUDA(cudaMemcpyAsync(hr.data(), r.D.row, (size_t)(r.n + 1) * 4, cudaMemcpyDeviceToHost, r.st));
     LV_CUDA(cudaMemcpyAsync(hc.data(), r.D.col, (size_t)r.E * 4, cudaMemcpyDeviceToHost, r.st));
-    LV_CUDA(cudaMemcpyAsync(hw.data(), r.D.w, (size_t)r.E * 4, cudaMemcpyDeviceToHost, r.st));
+    // unit weights are not stored at level 0 (k_prep)
+    const bool unit = r.wint && r.ctrl_u32(offsetof(lv::Ctrl, unit_w)) != 0;
+    if (unit) std::fill(hw.begin(), hw.end(), 1u);
+    else LV_CUDA(cudaMemcpyAsync(hw.data(), r.D.w, (size_t)r.E * 4, cudaMemcpyDeviceToHost, r.st));
     LV_CUDA(cudaMemcpyAsync(hk.data(), r.D.k, (size_t)r.n * 8, cudaMemcpyDeviceToHost, r.st));
     r.sync();
     std::vector<std::pair<uint32_t, uint32_t>> rowbuf;

@@ -1474,103 +1474,144 @@ __global__ void k_chunk_bounds(int dslot, unsigned long long step) {
 
 // ---- level 0: input validation, weights, k, self-loop weight, total weight --------------------------
 // GraphDevice(GraphHost&) (graph.cuh:46-99) and the Community constructor (community.h:31-46):
-// k = sum of incident weights, m = total weight / 2 (graph.cu:81). One warp per vertex.
-constexpr uint32_t kPrepLongRow = 4096;
+// k = sum of incident weights, m = total weight / 2 (graph.cu:81).
+//
+// Both kinds of kernel give a warp 32 consecutive vertices, whose rows are one contiguous range of
+// entries (row r ends where row r + 1 starts).
+// Unit weights (k_prep_unit): bound by reading the columns once and writing the engine's copy. The
+// range is streamed with all lanes whatever the row lengths: k is the row length, no row sum is
+// needed, and only an entry naming one of the warp's own 32 vertices can be a self-loop. Ranges
+// over kPrepPiece entries are cut into pieces, a block each (k_prep_unit_long). One warp per row
+// measured 863 + 211 us at R-MAT scale 22 (128 M entries) and 4.43 ms on 768 Chung-Lu graphs with
+// 173 M entries (mean row 8: three lanes in four idle); now
+// 193 + 144 us and 0.60 ms.
+// Given weights (k_prep): teams of 8 lanes take the rows, four at a time, and sum their weights;
+// rows over kPrepLongRow entries go to k_prep_long, a block each.
+constexpr uint32_t kPrepLongRow = 512;
+constexpr uint32_t kPrepPiece = 8192;
+constexpr int kPrepBatch = 4;
 // k_prep's local marker (never stored in Ctrl::err): a weight other than 1 was seen.
 constexpr uint32_t kErrNotUnit = 1u << 31;
 
-// Validation and weight conversion of entries [e0, re) with stride `step` of row v (graph
-// vertex range [lo, hi)); sums of the row's weights and of its self-loop weights.
+// The level-0 input as k_prep and k_prep_long read it: the caller's device arrays, or the
+// engine's own buffers where the input was uploaded (col == D.col then). wf / wu: weights as
+// floats / u32 (a resumed level whose sums may exceed 2^24), both nullptr for unit weights.
+// keep_w: unit weights are stored all the same (the refinement kernels read D.w).
+struct PrepIn {
+  const long long* row64;
+  const uint32_t* col;
+  const float* wf;
+  const uint32_t* wu;
+  int keep_w;
+};
+
+// Validation and weight conversion of entry e of row v (graph vertex range [lo, hi)), adding its
+// weight to the row's sum and, if it is a self-loop, to the self sum.
 template <bool WINT>
-__device__ __forceinline__ void prep_entries(const Dev& D, uint32_t v, long long e0, long long re,
-                                             uint32_t step, uint32_t lo, uint32_t hi, const float* wf_in,
-                                             const uint32_t* wu_in, unsigned long long& ki,
-                                             unsigned long long& si, double& kf, double& sf,
-                                             uint32_t& err) {
-  for (long long e = e0; e < re; e += step) {
-    const uint32_t u = D.col[e];
-    if (u < lo || u >= hi) { err |= kErrInput; continue; }
-    const float x = wf_in ? wf_in[e] : 1.0f;
-    if (WINT) {
-      // integer weights come as floats (exact below 2^24) or, for a resumed level whose sums
-      // may exceed that, as u32 (wu_in)
-      if (!wu_in && (!(x >= 1.0f) || x != floorf(x) || x > 4294967040.0f)) { err |= kErrInput; continue; }
-      const uint32_t xi = wu_in ? wu_in[e] : (uint32_t)x;
-      if (xi == 0u) { err |= kErrInput; continue; }
-      if (xi != 1u) err |= kErrNotUnit;
-      reinterpret_cast<uint32_t*>(D.w)[e] = xi;
-      ki += xi;
-      if (u == v) si += xi;
-    } else {
-      if (!(x > 0.0f) || !(x < INFINITY)) { err |= kErrInput; continue; }
-      reinterpret_cast<float*>(D.w)[e] = x;
-      kf += (double)x;
-      if (u == v) sf += (double)x;
-    }
+__device__ __forceinline__ void prep_entry(const Dev& D, const PrepIn& in, uint32_t v, long long e,
+                                           uint32_t u, uint32_t lo, uint32_t hi, unsigned long long& ki,
+                                           unsigned long long& si, double& kf, double& sf, uint32_t& err) {
+  if (u < lo || u >= hi) { err |= kErrInput; return; }
+  if (in.col != D.col) D.col[e] = u;
+  const float x = in.wf ? in.wf[e] : 1.0f;
+  if (WINT) {
+    if (!in.wu && (!(x >= 1.0f) || x != floorf(x) || x > 4294967040.0f)) { err |= kErrInput; return; }
+    const uint32_t xi = in.wu ? in.wu[e] : (uint32_t)x;
+    if (xi == 0u) { err |= kErrInput; return; }
+    if (xi != 1u) err |= kErrNotUnit;
+    if (in.wf || in.wu || in.keep_w) reinterpret_cast<uint32_t*>(D.w)[e] = xi;
+    ki += xi;
+    if (u == v) si += xi;
+  } else {
+    if (!(x > 0.0f) || !(x < INFINITY)) { err |= kErrInput; return; }
+    reinterpret_cast<float*>(D.w)[e] = x;
+    kf += (double)x;
+    if (u == v) sf += (double)x;
   }
 }
 
 template <bool WINT>
-__global__ void __launch_bounds__(256) k_prep(int dslot, const long long* row64, const float* wf_in,
-                                              const uint32_t* wu_in,
-                                              uint32_t n, unsigned long long E) {
+__global__ void __launch_bounds__(256) k_prep(int dslot, PrepIn in, uint32_t n, unsigned long long E) {
   const Dev& D = c_dev[dslot];
   Ctrl* C = D.ctrl;
   const int lane = threadIdx.x & 31;
   const uint32_t warp = (blockIdx.x * blockDim.x + threadIdx.x) >> 5;
   const uint32_t nwarps = (gridDim.x * blockDim.x) >> 5;
   uint32_t err = 0;
-  // per-graph totals are kept in registers and flushed when the graph changes
+  // the running graph's totals, per lane; summed over the warp when the graph changes
   uint32_t cur_g = kEmpty;
   unsigned long long tk_i = 0, ts_i = 0;
   double tk_f = 0.0, ts_f = 0.0;
-  auto flush = [&]() {
-    if (cur_g == kEmpty || lane != 0) return;
+  // S holds sum k (= 2m) until k_prep_total
+  auto add_totals = [&](uint32_t g, unsigned long long k_i, unsigned long long s_i, double k_f, double s_f) {
     if (WINT) {
-      if (ts_i) atomicAdd(&D.gs[cur_g].I, ts_i);
-      if (tk_i) atomicAdd(&D.gs[cur_g].S, tk_i);  // S holds sum k (= 2m) until k_prep_total
+      if (s_i) atomicAdd(&D.gs[g].I, s_i);
+      if (k_i) atomicAdd(&D.gs[g].S, k_i);
     } else {
-      if (ts_f != 0.0) atomicAdd(reinterpret_cast<double*>(&D.gs[cur_g].I), ts_f);
-      if (tk_f != 0.0) atomicAdd(reinterpret_cast<double*>(&D.gs[cur_g].S), tk_f);
+      if (s_f != 0.0) atomicAdd(reinterpret_cast<double*>(&D.gs[g].I), s_f);
+      if (k_f != 0.0) atomicAdd(reinterpret_cast<double*>(&D.gs[g].S), k_f);
     }
   };
-  for (uint32_t v = warp; v < n; v += nwarps) {
-    const long long rs = row64[v], re = row64[v + 1];
-    const uint32_t g = D.gid ? D.gid[v] : 0u;
-    const uint32_t lo = D.gs[g].vb, hi = D.gs[g].ve;
-    if (rs < 0 || re <= rs || (unsigned long long)re > E) {
-      if (lane == 0) { err |= kErrInput; D.row[v] = 0; D.k[v] = 0.0; }
+  auto flush = [&]() {
+    if (WINT) { tk_i = warp_sum(tk_i); ts_i = warp_sum(ts_i); }
+    else { tk_f = warp_sum(tk_f); ts_f = warp_sum(ts_f); }
+    if (cur_g != kEmpty && lane == 0) add_totals(cur_g, tk_i, ts_i, tk_f, ts_f);
+    tk_i = ts_i = 0;
+    tk_f = ts_f = 0.0;
+  };
+  for (uint32_t vb = warp * 32u; vb < n; vb += nwarps * 32u) {
+    const uint32_t cnt = min(32u, n - vb);
+    const uint32_t v = vb + min((uint32_t)lane, cnt - 1u);
+    const bool live = lane < (int)cnt;
+    const long long rs = in.row64[v], re = in.row64[v + 1];
+    const bool bad = rs < 0 || re <= rs || (unsigned long long)re > E;
+    if (__any_sync(kFull, bad)) {  // (the run ends with this error: nothing reads the group's rows)
+      err |= kErrInput;
       continue;
     }
-    if (lane == 0) {
+    const uint32_t g = D.gid ? D.gid[v] : 0u;
+    const uint32_t lo = D.gs[g].vb, hi = D.gs[g].ve;
+    if (live) {
       D.row[v] = (uint32_t)rs;
       if (v == n - 1) D.row[n] = (uint32_t)re;
     }
-    if (re - rs > kPrepLongRow) {  // a block takes it (k_prep_long)
-      if (lane == 0) D.bins[kNumBins - 1][atomicAdd(&C->bin_count[kNumBins - 1], 1u)] = v;
-      continue;
+    uint32_t len = live ? (uint32_t)(re - rs) : 0u;
+    const bool is_long = len > kPrepLongRow;
+    if (is_long) {  // a block takes it (k_prep_long)
+      D.bins[kNumBins - 1][atomicAdd(&C->bin_count[kNumBins - 1], 1u)] = v;
+      len = 0;
     }
-    if (g != cur_g) {
+    const uint32_t g0 = __shfl_sync(kFull, g, 0);
+    const bool one_graph = __all_sync(kFull, g == g0);
+    if (one_graph && g0 != cur_g) {
       flush();
-      cur_g = g;
-      tk_i = ts_i = 0;
-      tk_f = ts_f = 0.0;
+      cur_g = g0;
     }
-    unsigned long long ki = 0, si = 0;
+    unsigned long long ki = 0, si = 0;  // this lane's vertex
     double kf = 0.0, sf = 0.0;
-    prep_entries<WINT>(D, v, rs + lane, re, 32, lo, hi, wf_in, wu_in, ki, si, kf, sf, err);
-    if (WINT) {
-      ki = warp_sum(ki);
-      si = warp_sum(si);
-      if (lane == 0) D.k[v] = (double)ki;
-      tk_i += ki;
-      ts_i += si;
+    // teams of 8 lanes take a row each, in row order (four rows at a time)
+    for (int r = 0; r < 32; r += 4) {
+      const int k = r + (lane >> 3);
+      const long long ers = __shfl_sync(kFull, rs, k);
+      const uint32_t el = __shfl_sync(kFull, len, k);
+      const uint32_t elo = __shfl_sync(kFull, lo, k), ehi = __shfl_sync(kFull, hi, k);
+      unsigned long long a = 0, b = 0;
+      double c = 0.0, d = 0.0;
+      for (uint32_t j = lane & 7; j < el; j += 8)
+        prep_entry<WINT>(D, in, vb + k, ers + j, in.col[ers + j], elo, ehi, a, b, c, d, err);
+      if (WINT) { a = team_sum<8>(a); b = team_sum<8>(b); }
+      else { c = team_sum<8>(c); d = team_sum<8>(d); }
+      // lane r + i gets the sums of row r + i
+      const int from = (lane & 3) * 8;
+      const unsigned long long a2 = __shfl_sync(kFull, a, from), b2 = __shfl_sync(kFull, b, from);
+      const double c2 = __shfl_sync(kFull, c, from), d2 = __shfl_sync(kFull, d, from);
+      if ((lane & ~3) == r) { ki = a2; si = b2; kf = c2; sf = d2; }
+    }
+    if (live && !is_long) D.k[v] = WINT ? (double)ki : kf;
+    if (one_graph) {
+      tk_i += ki; ts_i += si; tk_f += kf; ts_f += sf;
     } else {
-      kf = warp_sum(kf);
-      sf = warp_sum(sf);
-      if (lane == 0) D.k[v] = kf;
-      tk_f += kf;
-      ts_f += sf;
+      add_totals(g, ki, si, kf, sf);
     }
   }
   flush();
@@ -1579,9 +1620,9 @@ __global__ void __launch_bounds__(256) k_prep(int dslot, const long long* row64,
   if (err) report_err(C, err, 3);  // k_prep
 }
 
-// Rows longer than kPrepLongRow entries, one block each.
+// Rows longer than kPrepLongRow entries, one block each, kPrepBatch columns in flight per thread.
 template <bool WINT>
-__global__ void __launch_bounds__(512) k_prep_long(int dslot, const float* wf_in, const uint32_t* wu_in) {
+__global__ void __launch_bounds__(512) k_prep_long(int dslot, PrepIn in) {
   const Dev& D = c_dev[dslot];
   Ctrl* C = D.ctrl;
   __shared__ unsigned long long shu[33];
@@ -1590,11 +1631,20 @@ __global__ void __launch_bounds__(512) k_prep_long(int dslot, const float* wf_in
   uint32_t err = 0;
   for (uint32_t idx = blockIdx.x; idx < count; idx += gridDim.x) {
     const uint32_t v = D.bins[kNumBins - 1][idx];
-    const uint32_t rs = D.row[v], re = D.row[v + 1];
+    const uint32_t rs = D.row[v], re = (uint32_t)in.row64[v + 1];
     const uint32_t g = D.gid ? D.gid[v] : 0u;
+    const uint32_t lo = D.gs[g].vb, hi = D.gs[g].ve;
     unsigned long long ki = 0, si = 0;
     double kf = 0.0, sf = 0.0;
-    prep_entries<WINT>(D, v, rs + threadIdx.x, re, blockDim.x, D.gs[g].vb, D.gs[g].ve, wf_in, wu_in, ki, si, kf, sf, err);
+    for (uint32_t e = rs + threadIdx.x; e < re; e += kPrepBatch * 512u) {
+      uint32_t uu[kPrepBatch];
+#pragma unroll
+      for (int q = 0; q < kPrepBatch; ++q) uu[q] = e + q * 512u < re ? in.col[e + q * 512u] : 0u;
+#pragma unroll
+      for (int q = 0; q < kPrepBatch; ++q)
+        if (e + q * 512u < re)
+          prep_entry<WINT>(D, in, v, e + q * 512u, uu[q], lo, hi, ki, si, kf, sf, err);
+    }
     if (WINT) {
       ki = block_sum<512>(ki, shu);
       si = block_sum<512>(si, shu);
@@ -1616,6 +1666,150 @@ __global__ void __launch_bounds__(512) k_prep_long(int dslot, const float* wf_in
   if (err & kErrNotUnit) C->unit_w = 0;
   err &= ~kErrNotUnit;
   if (err) report_err(C, err, 4);  // k_prep_long
+}
+
+// Entries [j0, j1) of a 32-vertex range (entry 0 of the range is entry e0 of the graph), `step`
+// entries apart per round of the warp: bounds check, the engine's copy, and the number of
+// self-loops. `off`: where this lane's row starts in the range (kEmpty past the last vertex).
+// ONE: the range lies in one graph, whose bounds are lo / hi; otherwise every entry's row is found
+// for its graph's bounds, and self-loops are added to their graphs here.
+template <bool ONE>
+__device__ __forceinline__ uint32_t prep_stream(const Dev& D, const PrepIn& in, uint32_t vb, uint32_t cnt,
+                                                long long e0, uint32_t off, uint32_t lo, uint32_t hi,
+                                                uint32_t j0, uint32_t j1, uint32_t step, uint32_t& err) {
+  const int lane = threadIdx.x & 31;
+  uint32_t loops = 0;
+  for (uint32_t jb = j0; jb < j1; jb += step) {
+    uint32_t uu[kPrepBatch];
+#pragma unroll
+    for (int q = 0; q < kPrepBatch; ++q) {
+      const uint32_t j = jb + (uint32_t)q * 32u + lane;
+      uu[q] = j < j1 ? in.col[e0 + j] : kEmpty;
+    }
+#pragma unroll
+    for (int q = 0; q < kPrepBatch; ++q) {
+      const uint32_t j = jb + (uint32_t)q * 32u + lane;
+      const bool have = j < j1;
+      if (have && in.col != D.col) D.col[e0 + j] = uu[q];
+      if (have && in.keep_w) reinterpret_cast<uint32_t*>(D.w)[e0 + j] = 1u;
+      if (ONE && have && (uu[q] < lo || uu[q] >= hi)) err |= kErrInput;
+      const bool own = have && uu[q] - vb < cnt;  // names one of the 32 vertices
+      if (!ONE || __any_sync(kFull, own)) {
+        int k = 0;  // the entry's row: the last one starting at or before j
+#pragma unroll
+        for (int s = 16; s >= 1; s >>= 1)
+          if (__shfl_sync(kFull, off, k + s) <= j) k += s;
+        if (!ONE) {
+          const uint32_t rlo = __shfl_sync(kFull, lo, k), rhi = __shfl_sync(kFull, hi, k);
+          if (have && (uu[q] < rlo || uu[q] >= rhi)) err |= kErrInput;
+        }
+        if (own && uu[q] - vb == (uint32_t)k) {
+          if (ONE) ++loops;
+          else atomicAdd(&D.gs[D.gid[vb + k]].I, 1ull);
+        }
+      }
+    }
+  }
+  return loops;
+}
+
+__global__ void __launch_bounds__(256) k_prep_unit(int dslot, PrepIn in, uint32_t n, unsigned long long E) {
+  const Dev& D = c_dev[dslot];
+  Ctrl* C = D.ctrl;
+  const int lane = threadIdx.x & 31;
+  const uint32_t warp = (blockIdx.x * blockDim.x + threadIdx.x) >> 5;
+  const uint32_t nwarps = (gridDim.x * blockDim.x) >> 5;
+  uint32_t err = 0;
+  uint32_t cur_g = kEmpty;  // the running graph and its totals, per lane
+  unsigned long long tk = 0, ts = 0;
+  auto flush = [&]() {
+    tk = warp_sum(tk);
+    ts = warp_sum(ts);
+    if (cur_g != kEmpty && lane == 0) {
+      if (ts) atomicAdd(&D.gs[cur_g].I, ts);
+      atomicAdd(&D.gs[cur_g].S, tk);  // S holds sum k (= 2m) until k_prep_total
+    }
+    tk = ts = 0;
+  };
+  for (uint32_t vb = warp * 32u; vb < n; vb += nwarps * 32u) {
+    const uint32_t cnt = min(32u, n - vb);
+    const uint32_t v = vb + min((uint32_t)lane, cnt - 1u);
+    const bool live = lane < (int)cnt;
+    const long long rs = in.row64[v], re = in.row64[v + 1];
+    const bool bad = rs < 0 || re <= rs || (unsigned long long)re > E;
+    if (__any_sync(kFull, bad)) {  // (the run ends with this error: nothing reads the group's rows)
+      err |= kErrInput;
+      continue;
+    }
+    const uint32_t g = D.gid ? D.gid[v] : 0u;
+    const uint32_t lo = D.gs[g].vb, hi = D.gs[g].ve;
+    const uint32_t len = live ? (uint32_t)(re - rs) : 0u;
+    if (live) {
+      D.row[v] = (uint32_t)rs;
+      if (v == n - 1) D.row[n] = (uint32_t)re;
+      D.k[v] = (double)len;
+    }
+    const uint32_t g0 = __shfl_sync(kFull, g, 0);
+    const bool one = __all_sync(kFull, g == g0);
+    if (one) {
+      if (g0 != cur_g) {
+        flush();
+        cur_g = g0;
+      }
+      tk += len;
+    } else if (live) {
+      atomicAdd(&D.gs[g].S, (unsigned long long)len);
+    }
+    const long long e0 = __shfl_sync(kFull, rs, 0);
+    const uint32_t total = (uint32_t)(__shfl_sync(kFull, re, (int)cnt - 1) - e0);
+    const uint32_t off = live ? (uint32_t)(rs - e0) : kEmpty;
+    if (total > kPrepPiece) {
+      if (lane == 0) {
+        const uint32_t np = (total + kPrepPiece - 1) / kPrepPiece;
+        const uint32_t p0 = atomicAdd(&C->hub_items, np);
+        for (uint32_t q = 0; q < np; ++q) D.long_items[p0 + q] = ((unsigned long long)vb << 32) | q;
+      }
+    } else if (one) {
+      ts += prep_stream<true>(D, in, vb, cnt, e0, off, lo, hi, 0, total, 32u * kPrepBatch, err);
+    } else {
+      prep_stream<false>(D, in, vb, cnt, e0, off, lo, hi, 0, total, 32u * kPrepBatch, err);
+    }
+  }
+  flush();
+  if (err) report_err(C, err, 3);  // k_prep_unit
+}
+
+// The pieces queued by k_prep_unit, one block each, its warps in turn.
+__global__ void __launch_bounds__(256) k_prep_unit_long(int dslot, PrepIn in, uint32_t n) {
+  const Dev& D = c_dev[dslot];
+  Ctrl* C = D.ctrl;
+  const int lane = threadIdx.x & 31;
+  const uint32_t wid = threadIdx.x >> 5;
+  const uint32_t count = C->hub_items;
+  uint32_t err = 0;
+  for (uint32_t i = blockIdx.x; i < count; i += gridDim.x) {
+    const unsigned long long item = D.long_items[i];
+    const uint32_t vb = (uint32_t)(item >> 32), piece = (uint32_t)item;
+    const uint32_t cnt = min(32u, n - vb);
+    const uint32_t v = vb + min((uint32_t)lane, cnt - 1u);
+    const long long rs = in.row64[v], re = in.row64[v + 1];
+    const uint32_t g = D.gid ? D.gid[v] : 0u;
+    const uint32_t lo = D.gs[g].vb, hi = D.gs[g].ve;
+    const uint32_t g0 = __shfl_sync(kFull, g, 0);
+    const bool one = __all_sync(kFull, g == g0);
+    const long long e0 = __shfl_sync(kFull, rs, 0);
+    const uint32_t total = (uint32_t)(__shfl_sync(kFull, re, (int)cnt - 1) - e0);
+    const uint32_t off = lane < (int)cnt ? (uint32_t)(rs - e0) : kEmpty;
+    const uint32_t j0 = piece * kPrepPiece + wid * 32u * kPrepBatch;
+    const uint32_t j1 = min(total, (piece + 1u) * kPrepPiece);
+    if (one) {
+      const uint32_t s = warp_sum(prep_stream<true>(D, in, vb, cnt, e0, off, lo, hi, j0, j1, 256u * kPrepBatch, err));
+      if (lane == 0 && s) atomicAdd(&D.gs[g0].I, (unsigned long long)s);
+    } else {
+      prep_stream<false>(D, in, vb, cnt, e0, off, lo, hi, j0, j1, 256u * kPrepBatch, err);
+    }
+  }
+  if (err) report_err(C, err, 4);  // k_prep_unit_long
 }
 
 // m = (sum of k) / 2 per graph; integer mode requires 2m < 2^32 (the reference's u32 sums).
@@ -1920,6 +2114,7 @@ __global__ void __launch_bounds__(256) k_hub_insert(int dslot) {
   const uint32_t count = C->bin_count[kNumBins - 1], total = C->hub_members;
   const uint32_t* hubs = D.bins[kNumBins - 1];
   const Wt* __restrict__ w = reinterpret_cast<const Wt*>(D.w);
+  const bool unit = unit_weights<WINT>(C);
   const int lane = threadIdx.x & 31;
   uint32_t err = 0;
   // entries staying inside their community are summed in registers
@@ -1932,16 +2127,17 @@ __global__ void __launch_bounds__(256) k_hub_insert(int dslot) {
   };
   auto add = [&](uint32_t e, uint32_t s, uint32_t off, uint32_t cap) {
     const uint32_t d = D.new_comm[D.col[e]];
+    const Acc wv = unit ? Acc(1) : (Acc)w[e];
     if (d == s) {
       if (s != self_s) {
         flush_self();
         self_s = s;
         self_acc = Acc(0);
       }
-      self_acc += (Acc)w[e];
+      self_acc += wv;
       return;
     }
-    if (!hub_table_add<WINT>(D, off, cap, d, (Acc)w[e])) err |= kErrTableFull;
+    if (!hub_table_add<WINT>(D, off, cap, d, wv)) err |= kErrTableFull;
   };
   // warps take groups of 32 members from a shared counter (row lengths are heavy-tailed)
   for (;;) {
@@ -2444,7 +2640,7 @@ __global__ void __launch_bounds__(256) k_agg_compact(int dslot) {
 // Next level's row offsets, per-graph vertex ranges and the level switch. The per-graph part (two
 // dependent gathers of map per graph) is spread over the grid: walked by one thread it took
 // 1.0-1.9 ms per level of a 2,048-graph batch (10.4 of that run's 21.5 ms of kernel time), now
-// about 6 us.
+// 6-20 us.
 __global__ void k_agg_finish(int dslot) {
   const Dev& D = c_dev[dslot];
   Ctrl* C = D.ctrl;
