@@ -250,6 +250,8 @@ class Run {
   int grid_sq = 0;          // blocks of k_commit_sq (partials)
   int grid_team[6] = {0};
   int grid_block[2] = {0};
+  int grid_short = 0;
+  uint32_t short_mask = 0;     // bins whose rows k_opt_short takes
   uint32_t team_cap[6] = {0};
   uint32_t block_cap = 0;
   cudaStream_t st;
@@ -343,6 +345,10 @@ class Run {
       if (bins.maxdeg[b + 1] < bins.maxdeg[b]) throw Fail{LV_ERR_ARGUMENT, "bin_max_degree must be non-decreasing"};
     for (int b = 0; b < 6; ++b) team_cap[b] = next_pow2(2u * std::max(1u, bins.maxdeg[b]));
     block_cap = next_pow2(2u * std::max(1u, bins.maxdeg[6]));
+    // k_opt_short holds four entries per lane: a bin goes there when its rows fit
+    short_mask = 0;
+    for (int b = 0; b < kShortBins; ++b)
+      if (bins.maxdeg[b] <= (uint32_t)(kShortPerLane * kOptT[b])) short_mask |= 1u << b;
     const size_t slot = opt_slot_bytes();  // the gain kernels' tables are the larger ones
     int max_smem = 0;
     LV_CUDA(cudaDeviceGetAttribute(&max_smem, cudaDevAttrMaxSharedMemoryPerBlockOptin, ctx->device));
@@ -377,6 +383,7 @@ class Run {
     team_grid<32, 8>(3, (const void*)k_opt_team<8, WI>, (const void*)k_contract_team<32, WI>);
     team_grid<32, 16>(4, (const void*)k_opt_team<16, WI>, (const void*)k_contract_team<32, WI>);
     team_grid<32, 32>(5, (const void*)k_opt_team<32, WI>, (const void*)k_contract_team<32, WI>);
+    grid_short = ctx->sms * std::max(1, occupancy(ctx->device, (const void*)k_opt_short<WI>, 256, 0));
     const size_t bsmem = (size_t)block_cap * opt_slot_bytes();
     ensure_dyn_smem(ctx->device, (const void*)k_opt_block<WI>, bsmem);
     ensure_dyn_smem(ctx->device, (const void*)k_contract_block<WI>, (size_t)block_cap * con_slot_bytes());
@@ -727,10 +734,12 @@ class Run {
     if (!gc.on) LV_CUDA(cudaEventRecord(ev[4], st));  // no event nodes inside captured loops
     k_chunk_flags<<<grid_n, 256, 0, st>>>(Dd);
     k_bin_vertices<<<grid_n, 256, 0, st>>>(Dd, bins, WI ? 1 : 0);
-    k_opt_team<1, WI><<<grid_team[0], 256, (256 / 1) * team_cap[0] * slot, st>>>(Dd, 0, team_cap[0]);
-    k_opt_team<2, WI><<<grid_team[1], 256, (256 / 2) * team_cap[1] * slot, st>>>(Dd, 1, team_cap[1]);
-    k_opt_team<4, WI><<<grid_team[2], 256, (256 / 4) * team_cap[2] * slot, st>>>(Dd, 2, team_cap[2]);
-    k_opt_team<8, WI><<<grid_team[3], 256, (256 / 8) * team_cap[3] * slot, st>>>(Dd, 3, team_cap[3]);
+    if (short_mask) { k_opt_short<WI><<<grid_short, 256, 0, st>>>(Dd, short_mask); ++launches; }
+    // (short bins configured wider than k_opt_short holds)
+    if (!(short_mask & 1u)) { k_opt_team<1, WI><<<grid_team[0], 256, (256 / 1) * team_cap[0] * slot, st>>>(Dd, 0, team_cap[0]); ++launches; }
+    if (!(short_mask & 2u)) { k_opt_team<2, WI><<<grid_team[1], 256, (256 / 2) * team_cap[1] * slot, st>>>(Dd, 1, team_cap[1]); ++launches; }
+    if (!(short_mask & 4u)) { k_opt_team<4, WI><<<grid_team[2], 256, (256 / 4) * team_cap[2] * slot, st>>>(Dd, 2, team_cap[2]); ++launches; }
+    if (!(short_mask & 8u)) { k_opt_team<8, WI><<<grid_team[3], 256, (256 / 8) * team_cap[3] * slot, st>>>(Dd, 3, team_cap[3]); ++launches; }
     k_opt_team<16, WI><<<grid_team[4], 256, (256 / 16) * team_cap[4] * slot, st>>>(Dd, 4, team_cap[4]);
     k_opt_team<32, WI><<<grid_team[5], 256, (256 / 32) * team_cap[5] * slot, st>>>(Dd, 5, team_cap[5]);
     k_opt_block<WI><<<grid_block[0], 512, block_cap * slot, st>>>(Dd, 6, block_cap);
@@ -752,7 +761,7 @@ class Run {
     k_apply_hub<WI><<<ctx->sms * 8, 256, 0, st>>>(Dd);
     commit_sq();
     finalize(0, view);
-    launches += 20;
+    launches += 16;
   }
 
   // Runs one pass; returns the number of graphs still iterating.

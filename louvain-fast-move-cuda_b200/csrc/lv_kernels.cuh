@@ -308,21 +308,42 @@ __global__ void __launch_bounds__(kBinNT) k_bin_vertices(int dslot, BinCfg B, in
   }
 }
 
-// Warp-aggregated append of movers; every lane of the warp must call it.
-__device__ __forceinline__ void emit_move(const Dev& D, bool move, uint32_t v, uint32_t c,
-                                          uint32_t it) {
-  const unsigned mask = __ballot_sync(kFull, move);
-  if (!mask) return;
-  const int lane = threadIdx.x & 31;
-  const int leader = __ffs(mask) - 1;
-  uint32_t base = 0;
-  if (lane == leader) base = atomicAdd(&D.ctrl->mover_count, (uint32_t)__popc(mask));
-  base = __shfl_sync(kFull, base, leader);
-  if (move) {
-    D.new_comm[v] = c;
-    D.movers[base + __popc(mask & lanemask_lt())] = v;
+// Movers of the team kernels, staged per warp in shared memory and appended 32 at a time: one
+// atomic on the list's single counter per 32 movers (one per warp step -- four to 32 rows, often
+// a single mover -- queued up on that counter). Every lane of the warp calls every member.
+struct MoverStage {
+  uint32_t* v;   // this warp's 64 entries
+  uint32_t n;    // staged, below 32 between calls (warp-uniform)
+  __device__ __forceinline__ void flush(const Dev& D, uint32_t cnt) {
+    const uint32_t lane = threadIdx.x & 31;
+    uint32_t base = 0;
+    if (lane == 0) base = atomicAdd(&D.ctrl->mover_count, cnt);
+    base = __shfl_sync(kFull, base, 0);
+    if (lane < cnt) D.movers[base + lane] = v[lane];
   }
-}
+  __device__ __forceinline__ void add(const Dev& D, bool move, uint32_t vtx, uint32_t c) {
+    const unsigned mask = __ballot_sync(kFull, move);
+    if (!mask) return;
+    if (move) {
+      D.new_comm[vtx] = c;
+      v[n + __popc(mask & lanemask_lt())] = vtx;
+    }
+    n += __popc(mask);
+    __syncwarp();
+    if (n >= 32) {
+      flush(D, 32);
+      const uint32_t lane = threadIdx.x & 31;
+      n -= 32;
+      const uint32_t t = v[32 + lane];
+      __syncwarp();
+      v[lane] = t;
+      __syncwarp();
+    }
+  }
+  __device__ __forceinline__ void finish(const Dev& D) {
+    if (n) flush(D, n);
+  }
+};
 
 // A mover found by a block kernel: recorded in the hub part of the mover list, its row cut into
 // pieces of kHubPiece entries for k_apply_hub.
@@ -652,12 +673,13 @@ __global__ void __launch_bounds__(256, 4) k_opt_team(int dslot, int bin, uint32_
   const uint32_t count = C->bin_count[bin];
   if (blockIdx.x * TEAMS >= count) return;  // (block-uniform)
   const uint32_t* vlist = D.bins[bin];
-  const uint32_t it = C->it;
   const bool fast = C->fast != 0;
   const bool lowest = fast || C->rule_sort != 0;
   const bool unit = unit_weights<WINT>(C);
   const unsigned tmask = T == 32 ? kFull : (((1u << T) - 1u) << ((threadIdx.x & 31) & ~(uint32_t)(T - 1)));
   uint32_t err = 0;
+  __shared__ uint32_t s_mov[8][64];
+  MoverStage mv{s_mov[threadIdx.x >> 5], 0u};
   ScratchTable<WINT> tbl{keys, vals, slots, cap - 1u, 0u};
   if (!fast) {
     for (uint32_t s = lane; s < cap; s += T) tbl.clear(s);
@@ -706,9 +728,151 @@ __global__ void __launch_bounds__(256, 4) k_opt_team(int dslot, int bin, uint32_
       c = key_comm(best, lowest);
       move = c != x.cv && (!fast || v <= c);
     }
-    emit_move(D, move, v, c, it);
+    mv.add(D, move, v, c);
   }
+  mv.finish(D);
   if (err) report_err(C, err, 0);  // k_opt_team
+}
+
+// ---- pass: optimisation of short rows, sums by comparing all pairs in registers -------------------
+// Rows of up to 4 T entries, T lanes per row (T = 1, 2, 4, 8), four entries per lane. Every entry
+// adds up the weights of the row's entries in its own community by comparing itself with each of
+// them (broadcast within the team), so there is no table: no shared memory, no atomics, no
+// clearing, and with fp32 weights a sum in row order. That is d steps of four compare-and-adds per
+// lane, which the issue rate bounds; a hash insert costs about 16 warp-instructions per entry and
+// the evaluation comes on top, so the crossover lies above 32 entries (at 128 entries on 16 lanes
+// the pairs alone would cost what the table does). The four short bins of a full table pass, one
+// launch here against four table launches: planted partition of 1 M vertices (fp32 weights, mean row
+// 20) 630 -> 343 us, R-MAT scale 22 (unit weights) 411 -> 157 us, 768 Chung-Lu graphs 1767 -> 1345 us.
+constexpr int kShortBins = 4;       // bins 0..3, T = 1 << bin
+constexpr int kShortPerLane = 4;
+template <int T, bool WINT, bool UNIT>
+__device__ __forceinline__ void pair_sums(const uint32_t (&cc)[kShortPerLane],
+                                          const typename WTraits<WINT>::W (&ww)[kShortPerLane], uint32_t dmax,
+                                          typename WTraits<WINT>::Acc (&ss)[kShortPerLane]) {
+  using Acc = typename WTraits<WINT>::Acc;
+#pragma unroll
+  for (int p = 0; p < kShortPerLane; ++p) {
+    if ((uint32_t)(p * T) >= dmax) break;  // (warp-uniform) no row of this warp is that long
+#pragma unroll
+    for (int j = 0; j < T; ++j) {
+      const uint32_t c = T == 1 ? cc[p] : __shfl_sync(kFull, cc[p], j, T);
+      const Acc w = UNIT ? Acc(1) : (Acc)(T == 1 ? ww[p] : __shfl_sync(kFull, ww[p], j, T));
+#pragma unroll
+      for (int q = 0; q < kShortPerLane; ++q)
+        if (cc[q] == c) ss[q] += w;
+    }
+  }
+}
+
+template <int T, bool WINT>
+__device__ __forceinline__ void short_rows(const Dev& D, const uint32_t* vlist, uint32_t idx, uint32_t count,
+                                           bool fast, bool lowest, bool unit, MoverStage& mv) {
+  using Tr = WTraits<WINT>;
+  using Acc = typename Tr::Acc;
+  using Wt = typename Tr::W;
+  constexpr int NB = kShortPerLane;
+  const Wt* __restrict__ w = reinterpret_cast<const Wt*>(D.w);
+  const int lane = threadIdx.x % T;
+  const bool live = idx < count;
+  const uint32_t v = live ? vlist[idx] : 0u;
+  VtxCtx x{};
+  if (live) x = load_vtx(D, v, unit);
+  unsigned long long best = 0;
+  if (fast) {
+    if (live) best = fast_scan<WINT>(D, x, v, x.rs + lane, T);
+  } else {
+    const uint32_t d = x.re - x.rs;  // 0 when not live
+    uint32_t uu[NB], cc[NB], at[NB];
+    Wt ww[NB];
+    double ac[NB];
+    Acc ss[NB];
+#pragma unroll
+    for (int q = 0; q < NB; ++q) {
+      const bool in = (uint32_t)(lane + q * T) < d;
+      const uint32_t e = x.rs + lane + q * T;
+      uu[q] = in ? D.col[e] : v;
+      ww[q] = in ? (unit ? Wt(1) : w[e]) : Wt(0);
+      ss[q] = Acc(0);
+    }
+    Acc self_acc = Acc(0);
+#pragma unroll
+    for (int q = 0; q < NB; ++q) {
+      if constexpr (WINT) {
+        const unsigned long long y = uu[q] != v ? D.ca[uu[q]] : 0xFFFFFFFFFFFFFFFFull;
+        cc[q] = (uint32_t)y;
+        at[q] = (uint32_t)(y >> 32);
+      } else {
+        cc[q] = uu[q] != v ? D.comm[uu[q]] : kEmpty;
+        at[q] = 0;
+      }
+    }
+#pragma unroll
+    for (int q = 0; q < NB; ++q) {
+      if (cc[q] == x.cv) {  // the own community: only its sum is needed
+        self_acc += (Acc)ww[q];
+        cc[q] = kEmpty;
+      }
+      if constexpr (WINT) ac[q] = (double)at[q];
+      else ac[q] = cc[q] != kEmpty ? D.a[cc[q]] : 0.0;
+    }
+    const uint32_t dmax = __reduce_max_sync(kFull, d);
+    if (unit) pair_sums<T, WINT, true>(cc, ww, dmax, ss);
+    else pair_sums<T, WINT, false>(cc, ww, dmax, ss);
+    self_acc = team_sum<T>(self_acc);
+    const float self_v = Tr::to_float(self_acc);
+#pragma unroll
+    for (int q = 0; q < NB; ++q) {
+      if (cc[q] == kEmpty) continue;
+      const float diff = __fsub_rn(Tr::to_float(ss[q]), self_v);
+      const double p = gain_p(x.kv, x.own_minus_k, ac[q]);
+      const float g = gain_fast(diff, p, x.inv_m, x.inv_2m2, x.m, x.two_m2);
+      if (g > 0.0f) {
+        const unsigned long long key = argmax_key(g, cc[q], lowest);
+        if (key > best) best = key;
+      }
+    }
+  }
+  best = team_max<T>(best, kFull);
+  bool move = false;
+  uint32_t c = 0;
+  if (live && lane == 0 && best) {
+    c = key_comm(best, lowest);
+    move = c != x.cv && (!fast || v <= c);
+  }
+  mv.add(D, move, v, c);
+}
+
+// The short bins in one launch (`mask`: bit b = bin b is taken here; a bin whose configured limit
+// exceeds 4 T stays with k_opt_team). A block takes a contiguous share of each bin's list, so that
+// the movers it stages together are neighbours; the shares of different bins start at different
+// blocks, so that small lists spread over the GPU.
+template <bool WINT>
+__global__ void __launch_bounds__(256, WINT ? 4 : 3) k_opt_short(int dslot, uint32_t mask) {
+  const Dev& D = c_dev[dslot];
+  Ctrl* C = D.ctrl;
+  __shared__ uint32_t s_mov[8][64];
+  MoverStage mv{s_mov[threadIdx.x >> 5], 0u};
+  const bool fast = C->fast != 0;
+  const bool lowest = fast || C->rule_sort != 0;
+  const bool unit = unit_weights<WINT>(C);
+  for (int b = kShortBins - 1; b >= 0; --b) {
+    if (!(mask >> b & 1u)) continue;
+    const uint32_t count = C->bin_count[b];
+    const uint32_t per = 256u >> b;  // rows per block step
+    const uint32_t tiles = (count + per - 1) / per;
+    const uint32_t blk = (blockIdx.x + (uint32_t)b * (gridDim.x / kShortBins)) % gridDim.x;
+    const uint32_t t0 = (uint32_t)((unsigned long long)blk * tiles / gridDim.x);
+    const uint32_t t1 = (uint32_t)((unsigned long long)(blk + 1) * tiles / gridDim.x);
+    for (uint32_t t = t0; t < t1; ++t) {
+      const uint32_t idx = t * per + (threadIdx.x >> b);
+      if (b == 0) short_rows<1, WINT>(D, D.bins[0], idx, count, fast, lowest, unit, mv);
+      else if (b == 1) short_rows<2, WINT>(D, D.bins[1], idx, count, fast, lowest, unit, mv);
+      else if (b == 2) short_rows<4, WINT>(D, D.bins[2], idx, count, fast, lowest, unit, mv);
+      else short_rows<8, WINT>(D, D.bins[3], idx, count, fast, lowest, unit, mv);
+    }
+  }
+  mv.finish(D);
 }
 
 // Block-wide sum (all threads call; result valid in every thread; `sh` holds >= 33 values).
