@@ -130,6 +130,9 @@ struct Ctrl {
   unsigned long long abort_need;
   uint32_t seg_levels, seg_passes, seg_aggs, seg_contract, seg_contract_ok, seg_final;
   unsigned long long t_pass0, t_agg0, t_opt_ns, t_optk_ns, t_agg_ns;
+  uint32_t input_err;          // err as the input kernels left it: k_small does not start on a bad input
+  uint32_t small_levels;       // levels of the deepest graph that k_small ran
+  uint32_t small_work[2];      // next graph of each k_small class
   TraceRec trace[kTraceCap];
 };
 
@@ -163,6 +166,11 @@ __device__ __forceinline__ double gain_p(double k, double own_minus_k, double a_
 __device__ __forceinline__ float gain_exact(float diff, double p, double m, double two_m2) {
   return __double2float_rn(__dadd_rn(__ddiv_rn((double)diff, m), __ddiv_rn(p, two_m2)));
 }
+// The same as a call: the two divisions are some hundred instructions, a kernel evaluates gains in
+// many unrolled places, and the call is almost never made (gain_fast).
+__device__ __noinline__ float gain_exact_call(float diff, double p, double m, double two_m2) {
+  return gain_exact(diff, p, m, two_m2);
+}
 __device__ __forceinline__ float gain_ref(float w_vc, float self_v, double k, double a_own,
                                           double a_c, double m, double two_m2) {
   return gain_exact(__fsub_rn(w_vc, self_v), gain_p(k, __dsub_rn(a_own, k), a_c), m, two_m2);
@@ -188,7 +196,7 @@ __device__ __forceinline__ float gain_fast(float diff, double p, double inv_m, d
   const float lo = __double2float_rn(__dsub_rd(s, err));
   const float hi = __double2float_rn(__dadd_ru(s, err));
   if (__float_as_uint(lo) == __float_as_uint(hi)) return lo;
-  return gain_exact(diff, p, m, two_m2);
+  return gain_exact_call(diff, p, m, two_m2);
 }
 
 // Argmax key for a positive gain: the float bits order positive floats, the low word breaks

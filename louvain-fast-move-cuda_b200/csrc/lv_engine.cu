@@ -25,6 +25,7 @@
 #include "../../include/louvain_b200.h"
 #include "lv_kernels.cuh"
 #include "lv_refine.cuh"
+#include "lv_small.cuh"
 
 namespace lv {
 
@@ -258,9 +259,12 @@ class Run {
   uint32_t* pinned = nullptr;  // small readbacks (64 bytes of pinned host memory)
   bool own_pinned = false;
   bool finished = false;
+  bool small_ok = false;       // a whole run from its input: k_small may take its small graphs
   int32_t levels_run = 0;
   double t_opt_ms = 0, t_agg_ms = 0, t_opt0 = -1, t_agg0 = -1, t_optk_ms = 0;
   int64_t launches = 0;
+  bool graph_mode_used = false;  // the device clock times the phases
+  int64_t graph_launches = 0;
   bool debug = std::getenv("LV_DEBUG") != nullptr;  // per-level sizes and bin populations on stderr
   cudaEvent_t ev[6];
   std::vector<Block> arena_blocks;
@@ -433,11 +437,21 @@ class Run {
     }
     choose_weight_mode(in.wf);
     long long* doffs = nullptr;
+    std::vector<int64_t> eo = {0, E64};  // entry offsets of the graphs
     if (G > 1) {
-      doffs = dalloc<long long>(ctx, owned, (size_t)G + 1, st);
+      doffs = dalloc<long long>(ctx, owned, 2 * ((size_t)G + 1), st);
       LV_CUDA(cudaMemcpyAsync(doffs, ho.data(), (G + 1) * 8, cudaMemcpyHostToDevice, st));
+      eo.resize(G + 1);
+      if (in_mem == LV_MEM_DEVICE) {
+        k_gather64<<<ctx->sms, 256, 0, st>>>(doffs + G + 1, in.row64, doffs, G + 1);
+        ++launches;
+        LV_CUDA(cudaMemcpyAsync(eo.data(), doffs + G + 1, (G + 1) * 8, cudaMemcpyDeviceToHost, st));
+        sync();
+      } else {
+        for (uint32_t g = 0; g <= G; ++g) eo[g] = row_ptr[ho[g]];
+      }
     }
-    prepare(ho, doffs, in);
+    prepare(ho, eo, doffs, in);
   }
 
   // A batch assembled from separate host graphs (local numbering each): every piece is
@@ -481,7 +495,7 @@ class Run {
     const std::vector<int64_t> ho = {0, n_};
     PrepIn in = uploaded(!integer);
     if (integer) in.wu = reinterpret_cast<const uint32_t*>(D.wB);
-    prepare(ho, nullptr, in);
+    prepare(ho, {0, E64}, nullptr, in);
     // the checkpoint's vertex map and counters replace the fresh run's
     LV_CUDA(cudaMemcpyAsync(D.best, best, (size_t)n0 * 4, cudaMemcpyHostToDevice, st));
     const uint32_t lv_it[2] = {(uint32_t)level, (uint32_t)iterations};
@@ -517,7 +531,7 @@ class Run {
     ++launches;
     const PrepIn in = uploaded(weighted);
     choose_weight_mode(in.wf);
-    prepare(ho, doffs, in);
+    prepare(ho, eo, doffs, in);
   }
 
  private:
@@ -617,8 +631,77 @@ class Run {
     grid_sq = std::min(kMaxPartials, ctx->sms * 4);
   }
 
+  // The graphs k_small runs (lv_small.cuh), per class, largest first; eo: entry offsets. None when
+  // the caller asked for host-driven launches, refinement or its own degree bins, or steps through
+  // the phases; a single graph only when one edge chunk covers it (no early return to emulate).
+  std::vector<uint32_t> small_ids[kSmallClasses];
+  int64_t small_entries[kSmallClasses] = {};  // of each class's largest graph
+  size_t small_count() const {
+    size_t c = 0;
+    for (const auto& ids : small_ids) c += ids.size();
+    return c;
+  }
+  void plan_small(const std::vector<int64_t>& ho, const std::vector<int64_t>& eo) {
+    if (!small_ok || !cfg.use_graphs || cfg.refine || debug) return;
+    for (int b = 0; b < 7; ++b)
+      if (cfg.bin_max_degree[b] > 0 && (uint32_t)cfg.bin_max_degree[b] != kDefaultMaxDeg[b]) return;
+    for (uint32_t g = 0; g < G; ++g) {
+      const int64_t ng = ho[g + 1] - ho[g], eg = eo[g + 1] - eo[g];
+      if (single() && cfg.chunk_edges > 0 && eg > cfg.chunk_edges) continue;
+      if (ng > kSmallN || eg > kSmallE) continue;
+      small_ids[ng <= kPackN && eg <= kPackE ? 0 : 1].push_back(g);
+    }
+    if (small_ids[0].size() <= (size_t)ctx->sms) {  // few: for latency
+      small_ids[1].insert(small_ids[1].end(), small_ids[0].begin(), small_ids[0].end());
+      small_ids[0].clear();
+    }
+    for (auto& ids : small_ids)
+      std::sort(ids.begin(), ids.end(), [&](uint32_t a, uint32_t b) {
+        const int64_t x = eo[a + 1] - eo[a], y = eo[b + 1] - eo[b];
+        return x != y ? x > y : a < b;
+      });
+    for (int c = 0; c < kSmallClasses; ++c)
+      if (!small_ids[c].empty()) small_entries[c] = eo[small_ids[c][0] + 1] - eo[small_ids[c][0]];
+  }
+  template <bool WI, int C>
+  void launch_small_class() {
+    const std::vector<uint32_t>& ids = small_ids[C];
+    if (ids.empty()) return;
+    uint32_t* dids = dalloc<uint32_t>(ctx, owned, ids.size(), st);
+    LV_CUDA(cudaMemcpyAsync(dids, ids.data(), ids.size() * 4, cudaMemcpyHostToDevice, st));
+    auto* fn = k_small<WI, kSmallNT[C], kSmallMinB[C]>;
+    const SmallCfg sc{cfg.mode, cfg.fast_first, single() ? 1 : 0, (uint32_t)std::max(0, cfg.max_levels),
+                      2u * (C == 0 ? kPackN : kSmallN)};
+    const size_t smem = (size_t)sc.cap * opt_slot_bytes();
+    ensure_dyn_smem(ctx->device, (const void*)fn, smem);
+    // CTAs per graph (class 1): as long as each has kSmallShare entries of the largest graph and the
+    // graphs do not fill the GPU on their own
+    uint32_t ncta = C == 1 ? kSmallMaxCtas : 1;
+    while (ncta > 1 && (small_entries[C] < (int64_t)ncta * kSmallShare || ids.size() * ncta > 2u * ctx->sms)) ncta /= 2;
+    const int occ = std::max(1, occupancy(ctx->device, (const void*)fn, kSmallNT[C], smem));
+    const uint32_t clusters = std::max(1u, std::min<uint32_t>((uint32_t)(ctx->sms * occ) / ncta, (uint32_t)ids.size()));
+    cudaLaunchConfig_t lc{};
+    lc.gridDim = dim3(clusters * ncta);
+    lc.blockDim = dim3(kSmallNT[C]);
+    lc.dynamicSmemBytes = smem;
+    lc.stream = st;
+    cudaLaunchAttribute at{};
+    at.id = cudaLaunchAttributeClusterDimension;
+    at.val.clusterDim.x = ncta;
+    at.val.clusterDim.y = at.val.clusterDim.z = 1;
+    lc.attrs = &at;
+    lc.numAttrs = 1;
+    LV_CUDA(cudaLaunchKernelEx(&lc, fn, Dd, (const uint32_t*)dids, (uint32_t)ids.size(), &D.ctrl->small_work[C], sc));
+    ++launches;
+  }
+  template <bool WI>
+  void launch_small() {
+    launch_small_class<WI, 1>();
+    launch_small_class<WI, 0>();
+  }
+
   // Control block, graph states, graph ids, degrees and totals, then the first level.
-  void prepare(const std::vector<int64_t>& ho, const long long* doffs, PrepIn in) {
+  void prepare(const std::vector<int64_t>& ho, const std::vector<int64_t>& eo, const long long* doffs, PrepIn in) {
     LV_CUDA(cudaMemsetAsync(D.ctrl, 0, sizeof(Ctrl), st));
     LV_CUDA(cudaMemsetAsync(D.gs, 0, sizeof(GraphState) * G, st));
     Ctrl hc{};
@@ -657,6 +740,8 @@ class Run {
     if (wint) k_prep_total<true><<<1, 256, 0, st>>>(Dd);
     else k_prep_total<false><<<1, 256, 0, st>>>(Dd);
     launches += 4;
+    plan_small(ho, eo);
+    if (small_count()) return;  // louvain() starts with them
     check_device_errors();
     level_start();
   }
@@ -1198,8 +1283,6 @@ class Run {
     finished = true;
     graph_mode_used = true;
   }
-  bool graph_mode_used = false;
-  int64_t graph_launches = 0;
 
   // OptimizationPhase::run: passes until every graph of the batch has stopped its level.
   int32_t optimization_run() {
@@ -1216,6 +1299,17 @@ class Run {
 
   // modularity_routine's level loop: captured and device-driven (use_graphs), or host-driven.
   void louvain() {
+    if (small_count()) {
+      if (wint) launch_small<true>(); else launch_small<false>();
+      graph_mode_used = true;
+      check_device_errors();  // the input's errors too: k_small does not start on a bad input
+      if (small_count() == G) {  // nothing is left for the level loop
+        graph_launches = 1;
+        finished = true;
+        return;
+      }
+      level_start();
+    }
     if (cfg.use_graphs && !cfg.refine && !debug && !finished) {
       if (wint) louvain_graph<true>(); else louvain_graph<false>();
       return;
@@ -1227,41 +1321,38 @@ class Run {
   }
 
   void stats(lv_stats* s) {
-    std::vector<GraphState> hs(G);
-    LV_CUDA(cudaMemcpyAsync(hs.data(), D.gs, sizeof(GraphState) * G, cudaMemcpyDeviceToHost, st));
-    sync();
-    unsigned long long act[2];
-    LV_CUDA(cudaMemcpyAsync(act, reinterpret_cast<char*>(D.ctrl) + offsetof(Ctrl, act_vertices_total),
-                            16, cudaMemcpyDeviceToHost, st));
+    // one readback: the first graph's state and the control block from the totals to the clocks
+    constexpr size_t c0 = offsetof(Ctrl, act_vertices_total), c1 = offsetof(Ctrl, trace);
+    GraphState g0;
+    Ctrl* hc = nullptr;
+    std::vector<char> buf(c1);
+    hc = reinterpret_cast<Ctrl*>(buf.data());
+    LV_CUDA(cudaMemcpyAsync(&g0, D.gs, sizeof(g0), cudaMemcpyDeviceToHost, st));
+    LV_CUDA(cudaMemcpyAsync(buf.data() + c0, reinterpret_cast<char*>(D.ctrl) + c0, c1 - c0, cudaMemcpyDeviceToHost, st));
     sync();
     std::memset(s, 0, sizeof(*s));
-    s->active_vertices = (int64_t)act[0];
-    s->active_entries = (int64_t)act[1];
+    s->active_vertices = (int64_t)hc->act_vertices_total;
+    s->active_entries = (int64_t)hc->act_entries_total;
     // 12 B per active entry (destination, weight, destination's community) and 24 B per
     // active vertex (row offsets, community, k, own total, decision)
-    s->bytes_optimization = 12.0 * (double)act[1] + 24.0 * (double)act[0];
-    s->ms_optimization_kernels = (float)t_optk_ms;
+    s->bytes_optimization = 12.0 * (double)s->active_entries + 24.0 * (double)s->active_vertices;
     s->kernel_launches = launches;
-    s->modularity = hs[0].Q;
+    s->modularity = g0.Q;
     s->n = n0;
     s->m = m_edges;
     s->levels = levels_run;
     if (graph_mode_used) {
       // a captured run has no host events between its kernels: the device clock times them
-      unsigned long long t[3];
-      LV_CUDA(cudaMemcpyAsync(t, reinterpret_cast<char*>(D.ctrl) + offsetof(Ctrl, t_opt_ns), sizeof(t),
-                              cudaMemcpyDeviceToHost, st));
-      sync();
-      t_opt_ms = t[0] * 1e-6;
-      t_optk_ms = t[1] * 1e-6;
-      t_agg_ms = t[2] * 1e-6;
-      s->ms_optimization_kernels = (float)t_optk_ms;
-      s->levels = (int32_t)seg_counts().levels;
+      t_opt_ms = hc->t_opt_ns * 1e-6;
+      t_optk_ms = hc->t_optk_ns * 1e-6;
+      t_agg_ms = hc->t_agg_ns * 1e-6;
+      s->levels = (int32_t)std::max(hc->seg_levels, hc->small_levels);
     }
+    s->ms_optimization_kernels = (float)t_optk_ms;
     s->graph_launches = graph_launches;
     s->refine_passes = refine_passes_run;
-    s->iterations = (int32_t)hs[0].total_iters;
-    s->n_communities = (int32_t)hs[0].n_best;
+    s->iterations = (int32_t)g0.total_iters;
+    s->n_communities = (int32_t)g0.n_best;
     s->ms_optimization = (float)t_opt_ms;
     s->ms_aggregation = (float)t_agg_ms;
     s->ms_first_optimization = (float)std::max(0.0, t_opt0);
@@ -1590,6 +1681,7 @@ static lv_status run_common(lv_context* ctx, uint32_t G, const int64_t* offs, in
     cudaEvent_t t0 = ctx->ev[0], t1 = ctx->ev[1], t2 = ctx->ev[2];
     LV_CUDA(cudaEventRecord(t0, ctx->stream));
     lv::Run r(ctx);
+    r.small_ok = true;
     r.init(G, offs, n, row_ptr, col, w, in_mem);
     LV_CUDA(cudaEventRecord(t1, ctx->stream));
     r.louvain();

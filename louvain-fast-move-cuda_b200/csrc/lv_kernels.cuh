@@ -312,26 +312,30 @@ __global__ void __launch_bounds__(kBinNT) k_bin_vertices(int dslot, BinCfg B, in
 // atomic on the list's single counter per 32 movers (one per warp step -- four to 32 rows, often
 // a single mover -- queued up on that counter). Every lane of the warp calls every member.
 struct MoverStage {
-  uint32_t* v;   // this warp's 64 entries
-  uint32_t n;    // staged, below 32 between calls (warp-uniform)
-  __device__ __forceinline__ void flush(const Dev& D, uint32_t cnt) {
+  uint32_t* v;      // this warp's 64 entries
+  uint32_t n;       // staged, below 32 between calls (warp-uniform)
+  uint32_t* list;   // the mover list and its counter
+  uint32_t* count;
+  __device__ __forceinline__ void flush(uint32_t cnt) {
     const uint32_t lane = threadIdx.x & 31;
     uint32_t base = 0;
-    if (lane == 0) base = atomicAdd(&D.ctrl->mover_count, cnt);
+    if (lane == 0) base = atomicAdd(count, cnt);
     base = __shfl_sync(kFull, base, 0);
-    if (lane < cnt) D.movers[base + lane] = v[lane];
+    if (lane < cnt) list[base + lane] = v[lane];
   }
-  __device__ __forceinline__ void add(const Dev& D, bool move, uint32_t vtx, uint32_t c) {
+  // vtx moves from community `pre` to c
+  __device__ __forceinline__ void add(const Dev& D, bool move, uint32_t vtx, uint32_t pre, uint32_t c) {
     const unsigned mask = __ballot_sync(kFull, move);
     if (!mask) return;
     if (move) {
       D.new_comm[vtx] = c;
+      D.cn[vtx] = ((unsigned long long)c << 32) | pre;
       v[n + __popc(mask & lanemask_lt())] = vtx;
     }
     n += __popc(mask);
     __syncwarp();
     if (n >= 32) {
-      flush(D, 32);
+      flush(32);
       const uint32_t lane = threadIdx.x & 31;
       n -= 32;
       const uint32_t t = v[32 + lane];
@@ -340,8 +344,15 @@ struct MoverStage {
       __syncwarp();
     }
   }
-  __device__ __forceinline__ void finish(const Dev& D) {
-    if (n) flush(D, n);
+  __device__ __forceinline__ void finish() {
+    if (n) flush(n);
+    n = 0;
+  }
+  __device__ __forceinline__ void switch_to(uint32_t* l, uint32_t* c) {
+    finish();
+    __syncwarp();
+    list = l;
+    count = c;
   }
 };
 
@@ -399,28 +410,28 @@ constexpr int kBatch = 4;
 constexpr int kApplyBatch = 8;
 
 // Fast pass: best key over positive per-entry gains (self = 0, destination's own total).
-template <bool WINT>
+template <bool WINT, int NB = kBatch>
 __device__ __forceinline__ unsigned long long fast_scan(const Dev& D, const VtxCtx& x, uint32_t v,
                                                         uint32_t e0, uint32_t step) {
   using Tr = WTraits<WINT>;
   using Wt = typename Tr::W;
-  const Wt* __restrict__ w = reinterpret_cast<const Wt*>(D.w);
+  const Wt* w = reinterpret_cast<const Wt*>(D.w);
   unsigned long long best = 0;
-  for (uint32_t e = e0; e < x.re; e += kBatch * step) {
-    uint32_t uu[kBatch];
-    float wf[kBatch];
-    double au[kBatch];
+  for (uint32_t e = e0; e < x.re; e += NB * step) {
+    uint32_t uu[NB];
+    float wf[NB];
+    double au[NB];
 #pragma unroll
-    for (int k = 0; k < kBatch; ++k) {
+    for (int k = 0; k < NB; ++k) {
       const uint32_t ek = e + k * step;
       const bool in = ek < x.re;
       uu[k] = in ? D.col[ek] : v;
       wf[k] = in ? (x.unit ? 1.0f : Tr::w_float(w[ek])) : 0.0f;
     }
 #pragma unroll
-    for (int k = 0; k < kBatch; ++k) au[k] = uu[k] != v ? D.a[uu[k]] : 0.0;
+    for (int k = 0; k < NB; ++k) au[k] = uu[k] != v ? D.a[uu[k]] : 0.0;
 #pragma unroll
-    for (int k = 0; k < kBatch; ++k) {
+    for (int k = 0; k < NB; ++k) {
       if (uu[k] == v) continue;
       // self = 0: diff = w - 0 = w exactly
       const double p = gain_p(x.kv, x.own_minus_k, au[k]);
@@ -526,7 +537,7 @@ __device__ __forceinline__ uint32_t insert_list(const Dev& D, const VtxCtx& x, u
   using Tr = WTraits<WINT>;
   using Acc = typename Tr::Acc;
   using Wt = typename Tr::W;
-  const Wt* __restrict__ w = reinterpret_cast<const Wt*>(D.w);
+  const Wt* w = reinterpret_cast<const Wt*>(D.w);
   const uint32_t lt = lanemask_lt();
   uint32_t nl = 0;
   for (uint32_t b = x.rs; b < x.re; b += NB * step) {
@@ -679,7 +690,7 @@ __global__ void __launch_bounds__(256, 4) k_opt_team(int dslot, int bin, uint32_
   const unsigned tmask = T == 32 ? kFull : (((1u << T) - 1u) << ((threadIdx.x & 31) & ~(uint32_t)(T - 1)));
   uint32_t err = 0;
   __shared__ uint32_t s_mov[8][64];
-  MoverStage mv{s_mov[threadIdx.x >> 5], 0u};
+  MoverStage mv{s_mov[threadIdx.x >> 5], 0u, D.movers, &C->mover_count};
   ScratchTable<WINT> tbl{keys, vals, slots, cap - 1u, 0u};
   if (!fast) {
     for (uint32_t s = lane; s < cap; s += T) tbl.clear(s);
@@ -728,9 +739,9 @@ __global__ void __launch_bounds__(256, 4) k_opt_team(int dslot, int bin, uint32_
       c = key_comm(best, lowest);
       move = c != x.cv && (!fast || v <= c);
     }
-    mv.add(D, move, v, c);
+    mv.add(D, move, v, x.cv, c);
   }
-  mv.finish(D);
+  mv.finish();
   if (err) report_err(C, err, 0);  // k_opt_team
 }
 
@@ -746,7 +757,8 @@ __global__ void __launch_bounds__(256, 4) k_opt_team(int dslot, int bin, uint32_
 // 20) 630 -> 343 us, R-MAT scale 22 (unit weights) 411 -> 157 us, 768 Chung-Lu graphs 1767 -> 1345 us.
 constexpr int kShortBins = 4;       // bins 0..3, T = 1 << bin
 constexpr int kShortPerLane = 4;
-template <int T, bool WINT, bool UNIT>
+// COMPACT (here and below): loops rolled for a kernel short of instruction cache (lv_small.cuh).
+template <int T, bool WINT, bool UNIT, bool COMPACT = false>
 __device__ __forceinline__ void pair_sums(const uint32_t (&cc)[kShortPerLane],
                                           const typename WTraits<WINT>::W (&ww)[kShortPerLane], uint32_t dmax,
                                           typename WTraits<WINT>::Acc (&ss)[kShortPerLane]) {
@@ -754,7 +766,7 @@ __device__ __forceinline__ void pair_sums(const uint32_t (&cc)[kShortPerLane],
 #pragma unroll
   for (int p = 0; p < kShortPerLane; ++p) {
     if ((uint32_t)(p * T) >= dmax) break;  // (warp-uniform) no row of this warp is that long
-#pragma unroll
+#pragma unroll (COMPACT ? 1 : T)
     for (int j = 0; j < T; ++j) {
       const uint32_t c = T == 1 ? cc[p] : __shfl_sync(kFull, cc[p], j, T);
       const Acc w = UNIT ? Acc(1) : (Acc)(T == 1 ? ww[p] : __shfl_sync(kFull, ww[p], j, T));
@@ -765,82 +777,108 @@ __device__ __forceinline__ void pair_sums(const uint32_t (&cc)[kShortPerLane],
   }
 }
 
-template <int T, bool WINT>
+// `load(v)`: the vertex's state (VtxCtx)
+template <int T, bool WINT, bool COMPACT = false, class Load>
 __device__ __forceinline__ void short_rows(const Dev& D, const uint32_t* vlist, uint32_t idx, uint32_t count,
-                                           bool fast, bool lowest, bool unit, MoverStage& mv) {
+                                           bool lowest, bool unit, MoverStage& mv, Load&& load) {
   using Tr = WTraits<WINT>;
   using Acc = typename Tr::Acc;
   using Wt = typename Tr::W;
   constexpr int NB = kShortPerLane;
-  const Wt* __restrict__ w = reinterpret_cast<const Wt*>(D.w);
+  const Wt* w = reinterpret_cast<const Wt*>(D.w);
   const int lane = threadIdx.x % T;
   const bool live = idx < count;
   const uint32_t v = live ? vlist[idx] : 0u;
   VtxCtx x{};
-  if (live) x = load_vtx(D, v, unit);
+  if (live) x = load(v);
   unsigned long long best = 0;
-  if (fast) {
-    if (live) best = fast_scan<WINT>(D, x, v, x.rs + lane, T);
+  const uint32_t d = x.re - x.rs;  // 0 when not live
+  uint32_t uu[NB], cc[NB], at[NB];
+  Wt ww[NB];
+  double ac[NB];
+  Acc ss[NB];
+#pragma unroll
+  for (int q = 0; q < NB; ++q) {
+    const bool in = (uint32_t)(lane + q * T) < d;
+    const uint32_t e = x.rs + lane + q * T;
+    uu[q] = in ? D.col[e] : v;
+    ww[q] = in ? (unit ? Wt(1) : w[e]) : Wt(0);
+    ss[q] = Acc(0);
+  }
+  Acc self_acc = Acc(0);
+#pragma unroll
+  for (int q = 0; q < NB; ++q) {
+    if constexpr (WINT) {
+      const unsigned long long y = uu[q] != v ? D.ca[uu[q]] : 0xFFFFFFFFFFFFFFFFull;
+      cc[q] = (uint32_t)y;
+      at[q] = (uint32_t)(y >> 32);
+    } else {
+      cc[q] = uu[q] != v ? D.comm[uu[q]] : kEmpty;
+      at[q] = 0;
+    }
+  }
+#pragma unroll
+  for (int q = 0; q < NB; ++q) {
+    if (cc[q] == x.cv) {  // the own community: only its sum is needed
+      self_acc += (Acc)ww[q];
+      cc[q] = kEmpty;
+    }
+    if constexpr (WINT) ac[q] = (double)at[q];
+    else ac[q] = cc[q] != kEmpty ? D.a[cc[q]] : 0.0;
+  }
+  const uint32_t dmax = __reduce_max_sync(kFull, d);
+  if (!COMPACT && unit) pair_sums<T, WINT, true>(cc, ww, dmax, ss);
+  else pair_sums<T, WINT, false, COMPACT>(cc, ww, dmax, ss);
+  self_acc = team_sum<T>(self_acc);
+  const float self_v = Tr::to_float(self_acc);
+  auto gain = [&](uint32_t c, Acc sum, double a_c) {
+    if (c == kEmpty) return;
+    const float diff = __fsub_rn(Tr::to_float(sum), self_v);
+    const double p = gain_p(x.kv, x.own_minus_k, a_c);
+    const float g = gain_fast(diff, p, x.inv_m, x.inv_2m2, x.m, x.two_m2);
+    if (g > 0.0f) {
+      const unsigned long long key = argmax_key(g, c, lowest);
+      if (key > best) best = key;
+    }
+  };
+  if constexpr (COMPACT) {
+#pragma unroll 1
+    for (int i = 0; i < NB; ++i) {
+      gain(cc[0], ss[0], ac[0]);
+#pragma unroll
+      for (int q = 0; q + 1 < NB; ++q) { cc[q] = cc[q + 1]; ss[q] = ss[q + 1]; ac[q] = ac[q + 1]; }
+    }
   } else {
-    const uint32_t d = x.re - x.rs;  // 0 when not live
-    uint32_t uu[NB], cc[NB], at[NB];
-    Wt ww[NB];
-    double ac[NB];
-    Acc ss[NB];
 #pragma unroll
-    for (int q = 0; q < NB; ++q) {
-      const bool in = (uint32_t)(lane + q * T) < d;
-      const uint32_t e = x.rs + lane + q * T;
-      uu[q] = in ? D.col[e] : v;
-      ww[q] = in ? (unit ? Wt(1) : w[e]) : Wt(0);
-      ss[q] = Acc(0);
-    }
-    Acc self_acc = Acc(0);
-#pragma unroll
-    for (int q = 0; q < NB; ++q) {
-      if constexpr (WINT) {
-        const unsigned long long y = uu[q] != v ? D.ca[uu[q]] : 0xFFFFFFFFFFFFFFFFull;
-        cc[q] = (uint32_t)y;
-        at[q] = (uint32_t)(y >> 32);
-      } else {
-        cc[q] = uu[q] != v ? D.comm[uu[q]] : kEmpty;
-        at[q] = 0;
-      }
-    }
-#pragma unroll
-    for (int q = 0; q < NB; ++q) {
-      if (cc[q] == x.cv) {  // the own community: only its sum is needed
-        self_acc += (Acc)ww[q];
-        cc[q] = kEmpty;
-      }
-      if constexpr (WINT) ac[q] = (double)at[q];
-      else ac[q] = cc[q] != kEmpty ? D.a[cc[q]] : 0.0;
-    }
-    const uint32_t dmax = __reduce_max_sync(kFull, d);
-    if (unit) pair_sums<T, WINT, true>(cc, ww, dmax, ss);
-    else pair_sums<T, WINT, false>(cc, ww, dmax, ss);
-    self_acc = team_sum<T>(self_acc);
-    const float self_v = Tr::to_float(self_acc);
-#pragma unroll
-    for (int q = 0; q < NB; ++q) {
-      if (cc[q] == kEmpty) continue;
-      const float diff = __fsub_rn(Tr::to_float(ss[q]), self_v);
-      const double p = gain_p(x.kv, x.own_minus_k, ac[q]);
-      const float g = gain_fast(diff, p, x.inv_m, x.inv_2m2, x.m, x.two_m2);
-      if (g > 0.0f) {
-        const unsigned long long key = argmax_key(g, cc[q], lowest);
-        if (key > best) best = key;
-      }
-    }
+    for (int q = 0; q < NB; ++q) gain(cc[q], ss[q], ac[q]);
   }
   best = team_max<T>(best, kFull);
   bool move = false;
   uint32_t c = 0;
   if (live && lane == 0 && best) {
     c = key_comm(best, lowest);
-    move = c != x.cv && (!fast || v <= c);
+    move = c != x.cv;
   }
-  mv.add(D, move, v, c);
+  mv.add(D, move, v, x.cv, c);
+}
+
+// Rows of the fast pass, T lanes each (T a power of two up to 32, the same for the whole warp).
+template <bool WINT, int NB = kBatch, class Load>
+__device__ __forceinline__ void fast_rows(const Dev& D, const uint32_t* vlist, uint32_t idx, uint32_t count,
+                                          uint32_t T, MoverStage& mv, Load&& load) {
+  const uint32_t lane = threadIdx.x & (T - 1u);
+  const bool live = idx < count;
+  const uint32_t v = live ? vlist[idx] : 0u;
+  VtxCtx x{};
+  if (live) x = load(v);
+  unsigned long long best = 0;
+  if (live) best = fast_scan<WINT, NB>(D, x, v, x.rs + lane, T);
+  for (uint32_t o = T / 2; o > 0; o >>= 1) {
+    const unsigned long long y = __shfl_xor_sync(kFull, best, o);
+    best = y > best ? y : best;
+  }
+  const uint32_t c = key_comm(best, true);
+  mv.add(D, live && lane == 0 && best && c != x.cv && v <= c, v, x.cv, c);
 }
 
 // The short bins in one launch (`mask`: bit b = bin b is taken here; a bin whose configured limit
@@ -852,10 +890,11 @@ __global__ void __launch_bounds__(256, WINT ? 4 : 3) k_opt_short(int dslot, uint
   const Dev& D = c_dev[dslot];
   Ctrl* C = D.ctrl;
   __shared__ uint32_t s_mov[8][64];
-  MoverStage mv{s_mov[threadIdx.x >> 5], 0u};
+  MoverStage mv{s_mov[threadIdx.x >> 5], 0u, D.movers, &C->mover_count};
   const bool fast = C->fast != 0;
-  const bool lowest = fast || C->rule_sort != 0;
+  const bool lowest = C->rule_sort != 0;
   const bool unit = unit_weights<WINT>(C);
+  auto load = [&](uint32_t v) { return load_vtx(D, v, unit); };
   for (int b = kShortBins - 1; b >= 0; --b) {
     if (!(mask >> b & 1u)) continue;
     const uint32_t count = C->bin_count[b];
@@ -866,13 +905,14 @@ __global__ void __launch_bounds__(256, WINT ? 4 : 3) k_opt_short(int dslot, uint
     const uint32_t t1 = (uint32_t)((unsigned long long)(blk + 1) * tiles / gridDim.x);
     for (uint32_t t = t0; t < t1; ++t) {
       const uint32_t idx = t * per + (threadIdx.x >> b);
-      if (b == 0) short_rows<1, WINT>(D, D.bins[0], idx, count, fast, lowest, unit, mv);
-      else if (b == 1) short_rows<2, WINT>(D, D.bins[1], idx, count, fast, lowest, unit, mv);
-      else if (b == 2) short_rows<4, WINT>(D, D.bins[2], idx, count, fast, lowest, unit, mv);
-      else short_rows<8, WINT>(D, D.bins[3], idx, count, fast, lowest, unit, mv);
+      if (fast) fast_rows<WINT>(D, D.bins[b], idx, count, 1u << b, mv, load);
+      else if (b == 0) short_rows<1, WINT>(D, D.bins[0], idx, count, lowest, unit, mv, load);
+      else if (b == 1) short_rows<2, WINT>(D, D.bins[1], idx, count, lowest, unit, mv, load);
+      else if (b == 2) short_rows<4, WINT>(D, D.bins[2], idx, count, lowest, unit, mv, load);
+      else short_rows<8, WINT>(D, D.bins[3], idx, count, lowest, unit, mv, load);
     }
   }
-  mv.finish(D);
+  mv.finish();
 }
 
 // Block-wide sum (all threads call; result valid in every thread; `sh` holds >= 33 values).
@@ -1206,12 +1246,66 @@ __global__ void k_pack_cn(int dslot) {
 
 constexpr uint32_t kApplyShort = 32;
 
+// The walk over the rows of up to 32 movers held one per lane (row start rs, length len, 0 for none,
+// pre-pass community old, target nw), all lanes busy whatever the row lengths: activity push, and
+// add(u, f, w as double, w as u32) for every entry (to u) that changes the internal weight by f w.
+template <bool WINT, int NB = kApplyBatch, class F>
+__device__ __forceinline__ void apply_rows(const Dev& D, uint32_t rs, uint32_t len, uint32_t old, uint32_t nw,
+                                           uint32_t it, bool unit, F&& add) {
+  using Tr = WTraits<WINT>;
+  using Wt = typename Tr::W;
+  const Wt* w = reinterpret_cast<const Wt*>(D.w);
+  const int lane = threadIdx.x & 31;
+  uint32_t incl = len;
+#pragma unroll
+  for (int o = 1; o < 32; o <<= 1) {
+    const uint32_t y = __shfl_up_sync(kFull, incl, o);
+    if (lane >= o) incl += y;
+  }
+  const uint32_t total = __shfl_sync(kFull, incl, 31);
+  const uint32_t excl = incl - len;
+  for (uint32_t jb = 0; jb < total; jb += 32u * NB) {
+    uint32_t ee[NB], oo[NB], nn[NB], uu[NB], pre[NB], nc[NB];
+#pragma unroll
+    for (int q = 0; q < NB; ++q) {
+      const uint32_t j = jb + (uint32_t)q * 32u + lane;
+      int k = 0;  // owner: the last lane whose row starts at or before j
+#pragma unroll
+      for (int step = 16; step >= 1; step >>= 1) {
+        const uint32_t ex = __shfl_sync(kFull, excl, k + step);
+        if (ex <= j) k += step;
+      }
+      ee[q] = __shfl_sync(kFull, rs, k) + (j - __shfl_sync(kFull, excl, k));
+      oo[q] = __shfl_sync(kFull, old, k);
+      nn[q] = __shfl_sync(kFull, nw, k);
+      uu[q] = j < total ? D.col[ee[q]] : kEmpty;
+    }
+#pragma unroll
+    for (int q = 0; q < NB; ++q) {
+      const unsigned long long x = uu[q] != kEmpty ? D.cn[uu[q]] : 0ull;
+      pre[q] = (uint32_t)x;
+      nc[q] = (uint32_t)(x >> 32);
+    }
+#pragma unroll
+    for (int q = 0; q < NB; ++q) {
+      if (uu[q] == kEmpty) continue;
+      const uint32_t u = uu[q];
+      const bool mu = nc[q] != pre[q];  // new_comm equals comm unless u moved this pass
+      const uint32_t post = nc[q];
+      if (post != nn[q]) D.active_it[u] = it + 1;
+      const int dd = (int)(nn[q] == post) - (int)(oo[q] == pre[q]);
+      if (dd) {
+        const int f = mu ? dd : 2 * dd;
+        if (WINT) add(u, f, 0.0, unit ? 1u : (uint32_t)w[ee[q]]);
+        else add(u, f, Tr::w_double(w[ee[q]]), 0u);
+      }
+    }
+  }
+}
+
 template <bool WINT>
 __global__ void __launch_bounds__(256) k_apply(int dslot) {
   const Dev& D = c_dev[dslot];
-  using Tr = WTraits<WINT>;
-  using Wt = typename Tr::W;
-  const Wt* __restrict__ w = reinterpret_cast<const Wt*>(D.w);
   Ctrl* C = D.ctrl;
   // the optimisation kernels of this pass ended when the first apply block starts
   if (blockIdx.x == 0 && threadIdx.x == 0) C->t_optk_ns += global_ns() - C->t_pass0;
@@ -1258,58 +1352,17 @@ __global__ void __launch_bounds__(256) k_apply(int dslot) {
       if (defer) D.members[b0 + __popc(dm & lanemask_lt())] = v;
     }
     if (defer) len = 0;
-    uint32_t incl = len;
-#pragma unroll
-    for (int o = 1; o < 32; o <<= 1) {
-      const uint32_t y = __shfl_up_sync(kFull, incl, o);
-      if (lane >= o) incl += y;
-    }
-    const uint32_t total = __shfl_sync(kFull, incl, 31);
-    const uint32_t excl = incl - len;
-    for (uint32_t jb = 0; jb < total; jb += 32u * kApplyBatch) {
-      uint32_t ee[kApplyBatch], oo[kApplyBatch], nn[kApplyBatch], uu[kApplyBatch], pre[kApplyBatch], nc[kApplyBatch];
-#pragma unroll
-      for (int q = 0; q < kApplyBatch; ++q) {
-        const uint32_t j = jb + (uint32_t)q * 32u + lane;
-        int k = 0;  // owner: the last lane whose row starts at or before j
-#pragma unroll
-        for (int step = 16; step >= 1; step >>= 1) {
-          const uint32_t ex = __shfl_sync(kFull, excl, k + step);
-          if (ex <= j) k += step;
-        }
-        ee[q] = __shfl_sync(kFull, rs, k) + (j - __shfl_sync(kFull, excl, k));
-        oo[q] = __shfl_sync(kFull, old, k);
-        nn[q] = __shfl_sync(kFull, nw, k);
-        uu[q] = j < total ? D.col[ee[q]] : kEmpty;
-      }
-#pragma unroll
-      for (int q = 0; q < kApplyBatch; ++q) {
-        const unsigned long long x = uu[q] != kEmpty ? D.cn[uu[q]] : 0ull;
-        pre[q] = (uint32_t)x;
-        nc[q] = (uint32_t)(x >> 32);
-      }
-#pragma unroll
-      for (int q = 0; q < kApplyBatch; ++q) {
-        if (uu[q] == kEmpty) continue;
-        const uint32_t u = uu[q];
-        const bool mu = nc[q] != pre[q];  // new_comm equals comm unless u moved this pass
-        const uint32_t post = nc[q];
-        if (post != nn[q]) D.active_it[u] = it + 1;
-        const int dd = (int)(nn[q] == post) - (int)(oo[q] == pre[q]);
-        if (dd) {
-          const int f = mu ? dd : 2 * dd;
-          if (D.gid) {
-            const uint32_t g = D.gid[u];
-            if (g != gcur) {
-              flush();
-              gcur = g;
-            }
-          }
-          if (WINT) di += (long long)f * (unit ? 1ll : (long long)w[ee[q]]);
-          else df += (double)f * Tr::w_double(w[ee[q]]);
+    apply_rows<WINT>(D, rs, len, old, nw, it, unit, [&](uint32_t u, int f, double wt, uint32_t wi) {
+      if (D.gid) {
+        const uint32_t g = D.gid[u];
+        if (g != gcur) {
+          flush();
+          gcur = g;
         }
       }
-    }
+      if (WINT) di += (long long)f * (long long)wi;
+      else df += (double)f * wt;
+    });
   }
   if (!D.gid) {
     // one graph: a single sum per warp
@@ -1996,6 +2049,8 @@ __global__ void k_prep_total(int dslot) {
     st->inv_2m2 = __drcp_rn(st->two_m2);
     st->S = 0;
   }
+  __syncthreads();  // (one block)
+  if (threadIdx.x == 0) C->input_err = C->err;
 }
 
 // Integer-weight detection for LV_WEIGHTS_AUTO: any weight that is not a non-negative integer
@@ -2014,6 +2069,11 @@ __global__ void k_fill_gid(uint32_t* gid, const long long* offs, uint32_t G) {
     const long long b = offs[g], e = offs[g + 1];
     for (long long v = b + threadIdx.x; v < e; v += blockDim.x) gid[v] = g;
   }
+}
+
+// out[i] = a[at[i]] (the graphs' entry offsets of a batch whose input lies on the device).
+__global__ void k_gather64(long long* out, const long long* a, const long long* at, uint32_t count) {
+  for (uint32_t i = blockIdx.x * blockDim.x + threadIdx.x; i < count; i += gridDim.x * blockDim.x) out[i] = a[at[i]];
 }
 
 // Graphs uploaded one by one into a packed batch keep their local numbering; this rebases

@@ -138,6 +138,7 @@ struct lv_server {
   void run_batch(const std::vector<lv::Request*>& batch, int slot) {
     try {
       lv::Run run(ctx, streams[slot], pinned[slot], dslots[slot].get());
+      run.small_ok = true;
       std::vector<lv::Run::Piece> ps;
       ps.reserve(batch.size());
       for (lv::Request* r : batch) {
