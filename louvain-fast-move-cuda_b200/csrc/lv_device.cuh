@@ -133,6 +133,8 @@ struct Ctrl {
   uint32_t input_err;          // err as the input kernels left it: k_small does not start on a bad input
   uint32_t small_levels;       // levels of the deepest graph that k_small ran
   uint32_t small_work[2];      // next graph of each k_small class
+  uint32_t commit_ticket, scan_ticket, bin_ticket;  // blocks done: the last one does the kernel's tail
+  uint32_t pad_ticket;
   TraceRec trace[kTraceCap];
 };
 
@@ -428,6 +430,22 @@ struct ScratchTable {
     }
   }
 };
+
+// ---- last block of a grid ----------------------------------------------------------------------
+// True in every thread of the block that gets here last (all blocks call it once, after their
+// global writes, which that block then sees; it reads them with __ldcg). The ticket is left at 0.
+__device__ __forceinline__ bool last_block(uint32_t* ticket) {
+  __shared__ uint32_t s_last;
+  __threadfence();
+  __syncthreads();
+  if (threadIdx.x == 0) {
+    s_last = atomicAdd(ticket, 1u) == gridDim.x - 1u;
+    if (s_last) *ticket = 0u;
+  }
+  __syncthreads();
+  if (s_last) __threadfence();
+  return s_last != 0;
+}
 
 // ---- warp / block reductions -------------------------------------------------------------------
 template <int T>

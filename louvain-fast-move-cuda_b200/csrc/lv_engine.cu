@@ -55,6 +55,8 @@ struct DevSlot {
   GraphCtl gc{};
   int64_t k_pass = 0, k_level = 0, k_contract = 0, k_ok = 0, k_final = 0;  // kernels per segment
   cudaStream_t cs[3] = {nullptr, nullptr, nullptr};  // capture streams of nested bodies
+  cudaStream_t bs[5] = {};                           // and of the branches inside a body
+  cudaEvent_t be[6] = {};                            // fork, and the end of each branch
 
   cudaError_t create() {
     std::lock_guard<std::mutex> lk(g_slot_mu);
@@ -76,6 +78,10 @@ struct DevSlot {
     release_graph();
     for (auto& x : cs)
       if (x) cudaStreamDestroy(x);
+    for (auto& x : bs)
+      if (x) cudaStreamDestroy(x);
+    for (auto& x : be)
+      if (x) cudaEventDestroy(x);
     if (id >= 0) {
       std::lock_guard<std::mutex> lk(g_slot_mu);
       g_slot_used[id] = false;
@@ -259,6 +265,7 @@ class Run {
   uint32_t* pinned = nullptr;  // small readbacks (64 bytes of pinned host memory)
   bool own_pinned = false;
   bool finished = false;
+  bool chunked = false;        // level 0 spans several edge chunks (later levels have fewer entries)
   bool small_ok = false;       // a whole run from its input: k_small may take its small graphs
   int32_t levels_run = 0;
   double t_opt_ms = 0, t_agg_ms = 0, t_opt0 = -1, t_agg0 = -1, t_optk_ms = 0;
@@ -740,6 +747,7 @@ class Run {
     if (wint) k_prep_total<true><<<1, 256, 0, st>>>(Dd);
     else k_prep_total<false><<<1, 256, 0, st>>>(Dd);
     launches += 4;
+    chunked = single() && cfg.chunk_edges > 0 && (int64_t)E > cfg.chunk_edges;
     plan_small(ho, eo);
     if (small_count()) return;  // louvain() starts with them
     check_device_errors();
@@ -755,21 +763,41 @@ class Run {
   void scan() {
     const int grid = ctx->sms * 4;
     k_scan_tiles<T, SRC><<<grid, kScanNT, 0, st>>>(Dd);
-    k_scan_sums<T, SRC><<<1, 1024, 0, st>>>(Dd);
     k_scan_apply<T, SRC, INCL><<<grid, kScanNT, 0, st>>>(Dd);
-    launches += 3;
+    launches += 2;
+  }
+
+  // ---- branches ---------------------------------------------------------------------------------
+  // Independent launches of a captured body go to branches of the graph, so that they run side by
+  // side: fork() after the work they depend on, on(i) to launch on branch i (0: the body's own
+  // stream), join() before the work that depends on all. A host-driven run launches them in
+  // order on its one stream.
+  int n_branch = 0;
+  cudaStream_t body_st = nullptr;
+  void fork(int n) {
+    n_branch = gc.on ? n : 0;
+    body_st = st;
+    if (!n_branch) return;
+    LV_CUDA(cudaEventRecord(slot->be[0], body_st));
+    for (int i = 1; i <= n; ++i) LV_CUDA(cudaStreamWaitEvent(slot->bs[i - 1], slot->be[0], 0));
+  }
+  void on(int i) { st = i > 0 && n_branch ? slot->bs[i - 1] : body_st; }
+  void join() {
+    st = body_st;
+    for (int i = 1; i <= n_branch; ++i) {
+      LV_CUDA(cudaEventRecord(slot->be[i], slot->bs[i - 1]));
+      LV_CUDA(cudaStreamWaitEvent(body_st, slot->be[i], 0));
+    }
+    n_branch = 0;
   }
 
   // ---- level start ------------------------------------------------------------------------------
-  void commit_sq() {
-    if (wint) k_commit_sq<true><<<grid_sq, 256, 0, st>>>(Dd, single() ? 1 : 0);
-    else k_commit_sq<false><<<grid_sq, 256, 0, st>>>(Dd, single() ? 1 : 0);
-  }
   // view: a refinement pass (regular passes only: no fast pass, no trace record)
-  void finalize(int level_start_flag, bool view = false) {
-    const int ff = view ? 0 : cfg.fast_first, vw = view ? 1 : 0;
-    if (wint) k_finalize<true><<<1, 1024, 0, st>>>(Dd, single() ? 1 : 0, grid_sq, level_start_flag, cfg.mode, ff, gc, vw);
-    else k_finalize<false><<<1, 1024, 0, st>>>(Dd, single() ? 1 : 0, grid_sq, level_start_flag, cfg.mode, ff, gc, vw);
+  void commit(int level_start_flag, bool view = false) {
+    const PassEnd pe{single() ? 1 : 0, level_start_flag, cfg.mode, view ? 0 : cfg.fast_first, view ? 1 : 0};
+    if (wint) k_commit<true><<<grid_sq, 256, 0, st>>>(Dd, pe, gc);
+    else k_commit<false><<<grid_sq, 256, 0, st>>>(Dd, pe, gc);
+    ++launches;
   }
 
   void ensure_arena(uint64_t need_slots) {
@@ -795,16 +823,14 @@ class Run {
 
   // Community::update at a new level, then the arena the level's global tables need.
   void level_start_kernels() {
-    if (single() && cfg.chunk_edges > 0) {
+    if (chunked) {
       k_chunk_bounds<<<1, 1, 0, st>>>(Dd, (unsigned long long)cfg.chunk_edges);
       ++launches;
     }
-    k_level_init<<<grid_n, 256, 0, st>>>(Dd);
-    commit_sq();
+    k_level_init<<<grid_n, 256, 0, st>>>(Dd, bins.maxdeg[6], bins.block_cap);
+    ++launches;
     // a refined run measures a level's gain from the previous level's end (k_ref_decide)
-    finalize(cfg.refine && levels_run > 0 ? 2 : 1);
-    k_arena_need<<<grid_n, 256, 0, st>>>(Dd, bins.maxdeg[6], bins.block_cap);
-    launches += 4;
+    commit(cfg.refine && levels_run > 0 ? 2 : 1);
   }
   void level_start() {
     level_start_kernels();
@@ -817,36 +843,47 @@ class Run {
   void launch_pass(bool view = false) {
     const size_t slot = opt_slot_bytes();
     if (!gc.on) LV_CUDA(cudaEventRecord(ev[4], st));  // no event nodes inside captured loops
-    k_chunk_flags<<<grid_n, 256, 0, st>>>(Dd);
+    if (chunked) { k_chunk_flags<<<grid_n, 256, 0, st>>>(Dd); ++launches; }
     k_bin_vertices<<<grid_n, 256, 0, st>>>(Dd, bins, WI ? 1 : 0);
+    // the bins' rows are independent: bin 7 (a chain of four kernels) on the body's stream
+    fork(5);
+    on(1);
     if (short_mask) { k_opt_short<WI><<<grid_short, 256, 0, st>>>(Dd, short_mask); ++launches; }
     // (short bins configured wider than k_opt_short holds)
     if (!(short_mask & 1u)) { k_opt_team<1, WI><<<grid_team[0], 256, (256 / 1) * team_cap[0] * slot, st>>>(Dd, 0, team_cap[0]); ++launches; }
     if (!(short_mask & 2u)) { k_opt_team<2, WI><<<grid_team[1], 256, (256 / 2) * team_cap[1] * slot, st>>>(Dd, 1, team_cap[1]); ++launches; }
     if (!(short_mask & 4u)) { k_opt_team<4, WI><<<grid_team[2], 256, (256 / 4) * team_cap[2] * slot, st>>>(Dd, 2, team_cap[2]); ++launches; }
     if (!(short_mask & 8u)) { k_opt_team<8, WI><<<grid_team[3], 256, (256 / 8) * team_cap[3] * slot, st>>>(Dd, 3, team_cap[3]); ++launches; }
+    on(2);
     k_opt_team<16, WI><<<grid_team[4], 256, (256 / 16) * team_cap[4] * slot, st>>>(Dd, 4, team_cap[4]);
+    on(3);
     k_opt_team<32, WI><<<grid_team[5], 256, (256 / 32) * team_cap[5] * slot, st>>>(Dd, 5, team_cap[5]);
+    on(4);
     k_opt_block<WI><<<grid_block[0], 512, block_cap * slot, st>>>(Dd, 6, block_cap);
+    on(5);
     k_opt_block<WI, 256><<<grid_block[1], 256, (block_cap / 2) * slot, st>>>(Dd, kHalfBin, block_cap / 2);
     // bin 7: rows cut into pieces over many blocks, global tables, argmax merged per vertex
+    on(0);
     k_opt_hub_prep<WI><<<ctx->sms * 4, 256, 0, st>>>(Dd);
     k_opt_hub_scan<WI><<<ctx->sms * 8, 256, 0, st>>>(Dd);
     k_opt_hub_eval<WI><<<ctx->sms * 8, 256, 0, st>>>(Dd);
     k_opt_hub_decide<<<ctx->sms, 256, 0, st>>>(Dd);
+    join();
     if (view) {
       k_ref_resolve<<<grid_n, 256, 0, st>>>(Dd);
       k_ref_reject<<<grid_n, 256, 0, st>>>(Dd);
       launches += 2;
     }
     if (!gc.on) LV_CUDA(cudaEventRecord(ev[5], st));
-    k_pack_cn<<<grid_n, 256, 0, st>>>(Dd);
+    fork(1);
+    on(1);
+    k_apply_hub<WI><<<ctx->sms * 8, 256, 0, st>>>(Dd);
+    on(0);
     k_apply<WI><<<grid_n, 256, 0, st>>>(Dd);
     k_apply_long<WI><<<grid_n, 256, 0, st>>>(Dd);
-    k_apply_hub<WI><<<ctx->sms * 8, 256, 0, st>>>(Dd);
-    commit_sq();
-    finalize(0, view);
-    launches += 16;
+    join();
+    launches += 12;
+    commit(0, view);
   }
 
   // Runs one pass; returns the number of graphs still iterating.
@@ -886,23 +923,20 @@ class Run {
   // the arena check and let the host redo the aggregation with a larger arena.
   template <bool WI>
   void agg_prefix(int force) {
-    agg_decide(force, 0);
+    agg_begin(force, 0);
     agg_renumber<WI>();
   }
-  void agg_decide(int force, int defer_i) {
-    const uint32_t gb = 32;  // grid-stride over graphs; fixed so that captured graphs are reusable
-    k_agg_decide<<<gb, 256, 0, st>>>(Dd, force, (uint32_t)std::max(0, cfg.max_levels), defer_i);
+  void agg_begin(int force, int defer_i) {
+    k_agg_begin<<<grid_n, 256, 0, st>>>(Dd, force, (uint32_t)std::max(0, cfg.max_levels), defer_i);
     ++launches;
   }
   template <bool WI>
   void agg_renumber() {
-    const uint32_t gb = 32;
-    k_agg_clear_map<<<grid_n, 256, 0, st>>>(Dd);
+    if (cfg.refine) { k_agg_clear<<<grid_n, 256, 0, st>>>(Dd); ++launches; }
     k_agg_mark<<<grid_n, 256, 0, st>>>(Dd);
-    k_agg_flags<<<grid_n, 256, 0, st>>>(Dd);
     scan<unsigned long long, true, kScanMap>();
-    k_agg_meta<<<gb, 256, 0, st>>>(Dd);
-    launches += 4;
+    k_agg_meta<<<1, 1024, 0, st>>>(Dd, gc);
+    launches += 2;
   }
 
   // ---- refinement (lv_refine.cuh) -------------------------------------------------------------
@@ -942,9 +976,7 @@ class Run {
     const int main = Dd;
     Dd = Dr;
     try {
-      commit_sq();
-      finalize(1, true);
-      launches += 2;
+      commit(1, true);
       for (int64_t p = 0;; ++p) {
         const uint32_t left = ctrl_u32(offsetof(Ctrl, n_iterating));
         if (left == 0 || (cfg.refine_passes > 0 && p >= cfg.refine_passes)) break;
@@ -967,46 +999,57 @@ class Run {
   }
   template <bool WI>
   void agg_contract_a() {
-    k_agg_clear_next<<<grid_n, 256, 0, st>>>(Dd);
     k_agg_count<<<grid_n, 256, 0, st>>>(Dd);
     scan<unsigned long long, false, kScanCd>();
-    k_agg_scatter<<<grid_n, 256, 0, st>>>(Dd);
-    k_agg_bin<<<grid_n, 256, 0, st>>>(Dd, bins);
-    launches += 4;
+    k_agg_scatter_bin<<<grid_n, 256, 0, st>>>(Dd, bins, gc);
+    launches += 2;
   }
   template <bool WI>
   void agg_contract_b() {
     const size_t slot = con_slot_bytes();
-    // the largest new communities: many blocks insert into their global tables
-    k_arena_clear<WI><<<ctx->sms * 8, 256, 0, st>>>(Dd);
-    k_hub_owner<<<ctx->sms * 2, 256, 0, st>>>(Dd, kNumBins - 1);
-    k_hub_member_prefix<<<1, 1024, 0, st>>>(Dd);
+    // independent: the largest new communities (many blocks insert into their global tables), the
+    // others by team or block, and the input vertices' new communities
+    fork(5);
+    k_hub_setup<WI><<<ctx->sms * 8, 256, 0, st>>>(Dd);
     k_hub_insert<WI><<<grid_n, 256, 0, st>>>(Dd);
     k_hub_insert_long<WI><<<ctx->sms * 8, 256, 0, st>>>(Dd);
     k_hub_emit<WI><<<ctx->sms * 8, 512, 0, st>>>(Dd);
-    k_contract_team<4, WI><<<grid_team[0], 256, (256 / 4) * team_cap[0] * slot, st>>>(Dd, 0, team_cap[0]);
-    k_contract_team<8, WI><<<grid_team[1], 256, (256 / 8) * team_cap[1] * slot, st>>>(Dd, 1, team_cap[1]);
-    k_contract_team<16, WI><<<grid_team[2], 256, (256 / 16) * team_cap[2] * slot, st>>>(Dd, 2, team_cap[2]);
-    k_contract_team<32, WI><<<grid_team[3], 256, (256 / 32) * team_cap[3] * slot, st>>>(Dd, 3, team_cap[3]);
-    k_contract_team<32, WI><<<grid_team[4], 256, (256 / 32) * team_cap[4] * slot, st>>>(Dd, 4, team_cap[4]);
+    on(1);
     k_contract_team<32, WI><<<grid_team[5], 256, (256 / 32) * team_cap[5] * slot, st>>>(Dd, 5, team_cap[5]);
+    k_contract_team<4, WI><<<grid_team[0], 256, (256 / 4) * team_cap[0] * slot, st>>>(Dd, 0, team_cap[0]);
+    on(2);
+    k_contract_team<32, WI><<<grid_team[4], 256, (256 / 32) * team_cap[4] * slot, st>>>(Dd, 4, team_cap[4]);
+    k_contract_team<8, WI><<<grid_team[1], 256, (256 / 8) * team_cap[1] * slot, st>>>(Dd, 1, team_cap[1]);
+    on(3);
+    k_contract_team<32, WI><<<grid_team[3], 256, (256 / 32) * team_cap[3] * slot, st>>>(Dd, 3, team_cap[3]);
+    k_contract_team<16, WI><<<grid_team[2], 256, (256 / 16) * team_cap[2] * slot, st>>>(Dd, 2, team_cap[2]);
+    on(4);
     k_contract_block<WI><<<grid_block[0], 512, block_cap * slot, st>>>(Dd, 6, block_cap);
+    on(5);
     k_contract_block<WI, 256><<<grid_block[1], 256, (block_cap / 2) * slot, st>>>(Dd, kHalfBin, block_cap / 2);
+    k_agg_best<<<grid_n, 256, 0, st>>>(Dd);
+    join();
     scan<uint32_t, false, kScanDeg>();
     k_agg_compact<WI><<<grid_n, 256, 0, st>>>(Dd);
-    launches += 15;
+    agg_finish();
+    launches += 14;
   }
-  void agg_tail() {
-    k_agg_best<<<grid_n, 256, 0, st>>>(Dd);
+  void agg_finish() {
     k_agg_finish<<<grid_n, 256, 0, st>>>(Dd);
-    launches += 2;
+    ++launches;
+  }
+  // The end of a run: no contraction.
+  void agg_final() {
+    k_agg_best<<<grid_n, 256, 0, st>>>(Dd);
+    ++launches;
+    agg_finish();
   }
 
   // Returns true if any graph continues to a new level.
   template <bool WI>
   bool aggregate_impl(int force) {
     if (cfg.refine) {
-      agg_decide(force, 1);
+      agg_begin(force, 1);
       // every iterating graph is at level levels_run: none refines at the level cap
       const bool at_cap = cfg.max_levels > 0 && levels_run + 1 >= cfg.max_levels;
       if (force != 0 && !at_cap) refine<WI>(force);
@@ -1037,8 +1080,9 @@ class Run {
       }
       ensure_arena(need);
       agg_contract_b<WI>();
+    } else {
+      agg_final();
     }
-    agg_tail();
     check_device_errors();
     n = ctrl_u32(offsetof(Ctrl, n));
     E = ctrl_u32(offsetof(Ctrl, E));
@@ -1063,11 +1107,11 @@ class Run {
   // ---- the captured run ------------------------------------------------------------------------------
   // The whole level loop as one CUDA graph with device-side control:
   //   while (level) {
-  //     k_gate_pass; while (pass) { <one pass, k_finalize sets `pass`> }
-  //     <aggregation prefix>; k_gate_contract
-  //     if (contract) { <binning>; k_gate_arena_agg
-  //                     if (ok) { <contraction>; <tail>; <level start>; k_gate_level } }
-  //     else          { <tail> }            (k_gate_contract cleared `level`)
+  //     while (pass) { <one pass; k_commit sets `pass`> }
+  //     <aggregation prefix; k_agg_meta sets `contract`>
+  //     if (contract) { <binning; k_agg_scatter_bin sets `ok`>
+  //                     if (ok) { <contraction>; <level start; its k_commit sets `level`, `pass`> } }
+  //     else          { <end> }            (k_agg_meta cleared `level`)
   //   }
   // A launch runs every remaining level of every graph without a host round trip. It stops
   // early only when a level needs a larger hash-table arena (Ctrl::abort says which); the host
@@ -1086,7 +1130,7 @@ class Run {
     k.grid_n = grid_n;
     k.grid_sq = grid_sq;
     k.grid_block = grid_block[0];
-    k.chunk_edges = single() ? cfg.chunk_edges : 0;
+    k.chunk_edges = chunked ? cfg.chunk_edges : 0;
     for (int b = 0; b < kNumBins; ++b) k.maxdeg[b] = bins.maxdeg[b];
     k.block_cap = bins.block_cap;
     for (int b = 0; b < 6; ++b) {
@@ -1141,12 +1185,17 @@ class Run {
     slot->release_graph();
     for (auto& x : slot->cs)
       if (!x) LV_CUDA(cudaStreamCreateWithFlags(&x, cudaStreamNonBlocking));
+    for (auto& x : slot->bs)
+      if (!x) LV_CUDA(cudaStreamCreateWithFlags(&x, cudaStreamNonBlocking));
+    for (auto& x : slot->be)
+      if (!x) LV_CUDA(cudaEventCreateWithFlags(&x, cudaEventDisableTiming));
     cudaStream_t* cs = slot->cs;
     cudaGraph_t graph = nullptr;
     LV_CUDA(cudaGraphCreate(&graph, 0));
     slot->graph = graph;
-    // each handle belongs to the graph that holds its conditional node; only the level loop's
-    // handle has a launch default (1), the others are set by a gate kernel before their node
+    // each handle belongs to the graph that holds its conditional node; the level and pass loops'
+    // handles have a launch default (a launch begins at a level start), later values are set by the
+    // kernel before the node (pass: also by the level start that ends the level's body)
     cudaGraphConditionalHandle hL, hP, hC, hO;
     LV_CUDA(cudaGraphConditionalHandleCreate(&hL, graph, 1, cudaGraphCondAssignDefault));
     gc = GraphCtl{};
@@ -1161,46 +1210,37 @@ class Run {
     try {
       LV_CUDA(cudaGraphAddNode(&top, graph, nullptr, 0, &p));
       cudaGraph_t level_body = p.conditional.phGraph_out[0];
-      LV_CUDA(cudaGraphConditionalHandleCreate(&hP, level_body, 0, 0));
+      LV_CUDA(cudaGraphConditionalHandleCreate(&hP, level_body, 1, cudaGraphCondAssignDefault));
       LV_CUDA(cudaGraphConditionalHandleCreate(&hC, level_body, 0, 0));
       gc.pass = hP;
       gc.contract = hC;
       gc.on = 1;
       int64_t a = 0, b = 0, c = 0, d = 0, e = 0;
       capture_into(level_body, cs[0], [&] {
-        k_gate_pass<<<1, 1, 0, st>>>(Dd, gc);
-        ++launches;
         cudaGraph_t* pb = add_cond(st, hP, cudaGraphCondTypeWhile, 1);
         a = launches;
         capture_into(pb[0], cs[1], [&] { launch_pass<WI>(); });
         slot->k_pass = launches - a;
         b = launches;
         agg_prefix<WI>(-1);
-        k_gate_contract<<<1, 1, 0, st>>>(Dd, gc);
-        ++launches;
         cudaGraph_t* cb = add_cond(st, hC, cudaGraphCondTypeIf, 2);
-        slot->k_level = launches - b + 1;  // + k_gate_pass
+        slot->k_level = launches - b;
         LV_CUDA(cudaGraphConditionalHandleCreate(&hO, cb[0], 0, 0));
         gc.ok = hO;
         c = launches;
         capture_into(cb[0], cs[1], [&] {
           agg_contract_a<WI>();
-          k_gate_arena_agg<<<1, 1, 0, st>>>(Dd, gc);
-          ++launches;
           cudaGraph_t* ob = add_cond(st, hO, cudaGraphCondTypeIf, 1);
           slot->k_contract = launches - c;
           d = launches;
           capture_into(ob[0], cs[2], [&] {
             agg_contract_b<WI>();
-            agg_tail();
             level_start_kernels();
-            k_gate_level<<<1, 1, 0, st>>>(Dd, gc);
-            ++launches;
           });
           slot->k_ok = launches - d;
         });
         e = launches;
-        capture_into(cb[1], cs[1], [&] { agg_tail(); });
+        capture_into(cb[1], cs[1], [&] { agg_final(); });
         slot->k_final = launches - e;
       });
       LV_CUDA(cudaGraphInstantiate(&slot->exec, graph, 0));

@@ -2,11 +2,17 @@
 //
 // One pass of the optimisation phase (the reference's optimize() + fast_move_update() +
 // compute_modularity(), phaseOptimization.cuh:116-181) is, here:
-//   k_chunk_flags -> k_bin_vertices -> k_opt_team<T> x6 / k_opt_block x2 -> k_apply ->
-//   k_commit_sq -> k_finalize
-// and aggregation (phaseAggregation.cuh:19-190) is:
-//   k_agg_flags -> scan -> k_agg_meta -> k_agg_best -> k_agg_count -> scan -> k_agg_scatter
-//   -> k_agg_bin -> k_contract_team<T> x6 / k_contract_block x2 -> scan -> k_agg_compact
+//   [k_chunk_flags ->] k_bin_vertices -> { k_opt_short | k_opt_team<T> x2 | k_opt_block x2 |
+//   k_opt_hub_* x4 } -> { k_apply -> k_apply_long | k_apply_hub } -> k_commit
+// and aggregation (phaseAggregation.cuh:19-190) with the next level's start is:
+//   k_agg_begin -> k_agg_mark -> scan x2 -> k_agg_meta -> k_agg_count -> scan x2 ->
+//   k_agg_scatter_bin -> { k_hub_* x4 | k_contract_team<T> x6 | k_contract_block x2 |
+//   k_agg_best } -> scan x2 -> k_agg_compact -> k_agg_finish -> k_level_init -> k_commit
+// ({ a | b }: independent, side by side in a captured run.) A launch in the captured loop costs
+// about 4 us beyond its work, so steps that need only "all blocks done" before a few words of
+// work (scan sums, modularity and the stop rule, the loop conditions) are done by the last block
+// of the kernel before them. R-MAT with 300,000 vertices 4.86 -> 3.87 ms, Chung-Lu with 150,000
+// 3.55 -> 2.56 ms, against 17 launches in a row per pass and about 45 per level.
 // All loops are grid-stride over sizes read from the device control block, so the grids do
 // not depend on the level and the sequence can be captured once and replayed.
 #pragma once
@@ -150,7 +156,6 @@ __device__ __forceinline__ bool has_nonloop(const Dev& D, uint32_t v, uint32_t d
 __global__ void k_chunk_flags(int dslot) {
   const Dev& D = c_dev[dslot];
   Ctrl* C = D.ctrl;
-  if (blockIdx.x == 0 && threadIdx.x == 0) C->t_pass0 = global_ns();  // first kernel of a pass
   if (!C->chunk_on || !(C->fast || C->rule_sort)) return;
   const uint32_t n = C->n, it = C->it, nch = C->n_chunks;
   // chunks seen by this thread (the first 32 as bits; later ones, rare, flagged at once),
@@ -184,6 +189,7 @@ constexpr int kBinNT = 256, kBinPer = 4, kBinTile = kBinNT * kBinPer;
 __global__ void __launch_bounds__(kBinNT) k_bin_vertices(int dslot, BinCfg B, int pack_ca) {
   const Dev& D = c_dev[dslot];
   Ctrl* C = D.ctrl;
+  if (blockIdx.x == 0 && threadIdx.x == 0) C->t_pass0 = global_ns();
   const uint32_t n = C->n, it = C->it;
   // table passes with integer weights: every vertex's (total, community) word for the gathers
   // of the gain kernels (the totals do not change before this pass's apply kernels)
@@ -358,10 +364,10 @@ struct MoverStage {
 
 // A mover found by a block kernel: recorded in the hub part of the mover list, its row cut into
 // pieces of kHubPiece entries for k_apply_hub.
-__device__ __forceinline__ void emit_hub_move(const Dev& D, uint32_t v, uint32_t c, uint32_t it,
-                                              uint32_t d) {
+__device__ __forceinline__ void emit_hub_move(const Dev& D, uint32_t v, uint32_t pre, uint32_t c, uint32_t d) {
   Ctrl* C = D.ctrl;
   D.new_comm[v] = c;
+  D.cn[v] = ((unsigned long long)c << 32) | pre;
   D.movers[C->n - 1u - atomicAdd(&C->hub_mover_count, 1u)] = v;
   const uint32_t np = (d + kHubPiece - 1) / kHubPiece;
   const uint32_t p0 = atomicAdd(&C->apply_items, np);
@@ -982,7 +988,6 @@ __global__ void __launch_bounds__(NT, 1024 / NT) k_opt_block(int dslot, int bin,
   const uint32_t count = C->bin_count[bin];
   if (blockIdx.x >= count) return;  // (block-uniform)
   const uint32_t* vlist = D.bins[bin];
-  const uint32_t it = C->it;
   const bool fast = C->fast != 0;
   const bool lowest = fast || C->rule_sort != 0;
   const bool unit = unit_weights<WINT>(C);
@@ -1038,7 +1043,7 @@ __global__ void __launch_bounds__(NT, 1024 / NT) k_opt_block(int dslot, int bin,
       y = team_max<32>(y, kFull);
       if (lane == 0 && y) {
         const uint32_t c = key_comm(y, lowest);
-        if (c != x.cv && (!fast || v <= c)) emit_hub_move(D, v, c, it, d);
+        if (c != x.cv && (!fast || v <= c)) emit_hub_move(D, v, x.cv, c, d);
       }
     }
   }
@@ -1165,7 +1170,7 @@ __global__ void __launch_bounds__(256) k_opt_hub_eval(int dslot) {
 __global__ void k_opt_hub_decide(int dslot) {
   const Dev& D = c_dev[dslot];
   Ctrl* C = D.ctrl;
-  const uint32_t count = C->bin_count[kNumBins - 1], it = C->it;
+  const uint32_t count = C->bin_count[kNumBins - 1];
   const bool fast = C->fast != 0;
   const bool lowest = fast || C->rule_sort != 0;
   for (uint32_t pos = blockIdx.x * blockDim.x + threadIdx.x; pos < count; pos += gridDim.x * blockDim.x) {
@@ -1173,7 +1178,8 @@ __global__ void k_opt_hub_decide(int dslot) {
     if (!best) continue;
     const uint32_t v = D.bins[kNumBins - 1][pos];
     const uint32_t c = key_comm(best, lowest);
-    if (c != D.comm[v] && (!fast || v <= c)) emit_hub_move(D, v, c, it, D.row[v + 1] - D.row[v]);
+    const uint32_t pre = D.comm[v];
+    if (c != pre && (!fast || v <= c)) emit_hub_move(D, v, pre, c, D.row[v + 1] - D.row[v]);
   }
 }
 
@@ -1235,15 +1241,8 @@ __device__ __forceinline__ void apply_entries(const Dev& D, uint32_t v, uint32_t
 // to k_apply_long (a warp each; movers sit in the list grouped by degree, so a warp taking 32
 // long rows would hold up the whole kernel). An entry's change of the internal weight goes to
 // its own graph, which is the mover's (edges never cross graphs).
-// Before the apply kernels: each vertex's pre-pass community and this pass's target packed
-// in one word, so that an entry costs one 8-byte gather instead of two 4-byte ones.
-__global__ void k_pack_cn(int dslot) {
-  const Dev& D = c_dev[dslot];
-  const uint32_t n = D.ctrl->n;
-  for (uint32_t v = blockIdx.x * blockDim.x + threadIdx.x; v < n; v += gridDim.x * blockDim.x)
-    D.cn[v] = ((unsigned long long)D.new_comm[v] << 32) | D.comm[v];
-}
-
+// (Dev::cn holds each vertex's pre-pass community and this pass's target in one word, so that an entry
+// costs one 8-byte gather: kept up by the level start, the kernels that emit moves and the commit.)
 constexpr uint32_t kApplyShort = 32;
 
 // The walk over the rows of up to 32 movers held one per lane (row start rs, length len, 0 for none,
@@ -1444,64 +1443,6 @@ __global__ void __launch_bounds__(512) k_apply_hub(int dslot) {
   }
 }
 
-// ---- pass: commit moves and recompute sum_c a_c^2 -----------------------------------------------
-// Integer mode squares exactly in u64 (a_c <= 2m < 2^32). One graph: per-block partials,
-// summed in a fixed order by k_finalize. Several graphs: one block per graph.
-template <bool WINT>
-__global__ void __launch_bounds__(256) k_commit_sq(int dslot, int single) {
-  const Dev& D = c_dev[dslot];
-  Ctrl* C = D.ctrl;
-  const uint32_t count = C->mover_count, hubs = C->hub_mover_count, nn = C->n;
-  for (uint32_t i = blockIdx.x * blockDim.x + threadIdx.x; i < count + hubs; i += gridDim.x * blockDim.x) {
-    const uint32_t v = D.movers[i < count ? i : nn - 1u - (i - count)];
-    D.comm[v] = D.new_comm[v];
-  }
-  __shared__ double shd[33];
-  __shared__ unsigned long long shu[33];
-  if (single) {
-    const uint32_t n = C->n;
-    unsigned long long su = 0;
-    double sf = 0.0;
-    if (D.gs[0].phase == kIterating) {
-      for (uint32_t c = blockIdx.x * blockDim.x + threadIdx.x; c < n; c += gridDim.x * blockDim.x) {
-        const double x = D.a[c];
-        if (WINT) { const unsigned long long xi = (unsigned long long)x; su += xi * xi; }
-        else sf = __dadd_rn(sf, __dmul_rn(x, x));
-      }
-    }
-    if (WINT) {
-      unsigned long long tot;
-      block_excl_scan<unsigned long long, 256>(su, shu, &tot);
-      if (threadIdx.x == 0) reinterpret_cast<unsigned long long*>(D.partials)[blockIdx.x] = tot;
-    } else {
-      double tot;
-      block_excl_scan<double, 256>(sf, shd, &tot);
-      if (threadIdx.x == 0) D.partials[blockIdx.x] = tot;
-    }
-  } else {
-    for (uint32_t g = blockIdx.x; g < C->G; g += gridDim.x) {
-      GraphState* st = &D.gs[g];
-      if (st->phase != kIterating) continue;
-      unsigned long long su = 0;
-      double sf = 0.0;
-      for (uint32_t c = st->vb + threadIdx.x; c < st->ve; c += blockDim.x) {
-        const double x = D.a[c];
-        if (WINT) { const unsigned long long xi = (unsigned long long)x; su += xi * xi; }
-        else sf = __dadd_rn(sf, __dmul_rn(x, x));
-      }
-      if (WINT) {
-        unsigned long long tot;
-        block_excl_scan<unsigned long long, 256>(su, shu, &tot);
-        if (threadIdx.x == 0) st->S = tot;
-      } else {
-        double tot;
-        block_excl_scan<double, 256>(sf, shd, &tot);
-        if (threadIdx.x == 0) st->S = __double_as_longlong(tot);
-      }
-    }
-  }
-}
-
 __device__ __forceinline__ double modularity_of(double I, double S, double m) {
   // community.h:104: in / (2m) - sum_a2 / (4 m m)
   return __dsub_rn(__ddiv_rn(I, __dmul_rn(2.0, m)), __ddiv_rn(S, __dmul_rn(__dmul_rn(4.0, m), m)));
@@ -1523,34 +1464,37 @@ __global__ void k_set_pass(Ctrl* C, uint32_t p, int mode, int fast_first) {
   if (threadIdx.x == 0 && blockIdx.x == 0) set_pass_rule(C, p, mode, fast_first);
 }
 
-// ---- pass end: modularity, stop rule, counters ----------------------------------------------------
+// ---- pass end: commit moves, sum_c a_c^2, modularity, stop rule, counters -------------------------
 // phaseOptimization.cuh:167-179: dQ = Q_after - Q_before; the level's passes stop when
 // dQ <= threshold (or after EARLY_STOP_LIMIT passes). `level_start` = 1 evaluates the level's
 // starting modularity instead (Community::update -> compute_modularity, community.h:57-65).
 // level_start = 2 keeps Q_level (a refined run's next level measures its gain from the
 // previous level's end). view = 1: a refinement pass (no trace record, no pass statistics).
+struct PassEnd {
+  int single, level_start, mode, fast_first, view;
+};
+
+// The part after every block's commit, by the last block of k_commit (256 threads).
 template <bool WINT>
-__global__ void __launch_bounds__(1024) k_finalize(int dslot, int single, int nparts, int level_start,
-                                                   int mode, int fast_first, GraphCtl gc, int view) {
-  const Dev& D = c_dev[dslot];
+__device__ __forceinline__ void finalize(const Dev& D, const PassEnd& pe, const GraphCtl& gc) {
   Ctrl* C = D.ctrl;
   __shared__ double shd[33];
   __shared__ unsigned long long shu[33];
   __shared__ uint32_t shc[33];
-  if (single) {
+  if (pe.single) {
     unsigned long long su = 0;
     double sf = 0.0;
-    for (int i = threadIdx.x; i < nparts; i += blockDim.x) {
-      if (WINT) su += reinterpret_cast<const unsigned long long*>(D.partials)[i];
-      else sf = __dadd_rn(sf, D.partials[i]);
+    for (uint32_t i = threadIdx.x; i < gridDim.x; i += 256) {
+      if (WINT) su += __ldcg(reinterpret_cast<const unsigned long long*>(D.partials) + i);
+      else sf = __dadd_rn(sf, __ldcg(D.partials + i));
     }
     if (WINT) {
       unsigned long long tot;
-      block_excl_scan<unsigned long long, 1024>(su, shu, &tot);
+      block_excl_scan<unsigned long long, 256>(su, shu, &tot);
       if (threadIdx.x == 0 && D.gs[0].phase == kIterating) D.gs[0].S = tot;
     } else {
       double tot;
-      block_excl_scan<double, 1024>(sf, shd, &tot);
+      block_excl_scan<double, 256>(sf, shd, &tot);
       if (threadIdx.x == 0 && D.gs[0].phase == kIterating) D.gs[0].S = __double_as_longlong(tot);
     }
     __syncthreads();
@@ -1559,12 +1503,14 @@ __global__ void __launch_bounds__(1024) k_finalize(int dslot, int single, int np
   for (uint32_t g = threadIdx.x; g < C->G; g += blockDim.x) {
     GraphState* st = &D.gs[g];
     if (st->phase != kIterating) continue;
-    const double I = WINT ? (double)st->I : __longlong_as_double((long long)st->I);
-    const double S = WINT ? (double)st->S : __longlong_as_double((long long)st->S);
+    const unsigned long long ib = __ldcg(&st->I), sb = __ldcg(&st->S);
+    const double I = WINT ? (double)ib : __longlong_as_double((long long)ib);
+    const double S = WINT ? (double)sb : __longlong_as_double((long long)sb);
+    if (WINT && !pe.single) st->S = 0;  // k_commit adds the next pass's squares to it
     const double Q = modularity_of(I, S, st->m);
-    if (level_start) {
+    if (pe.level_start) {
       st->Q = Q;
-      if (level_start == 1) st->Q_level = Q;
+      if (pe.level_start == 1) st->Q_level = Q;
       st->iters = 0;
       ++iterating;
       continue;
@@ -1573,7 +1519,7 @@ __global__ void __launch_bounds__(1024) k_finalize(int dslot, int single, int np
     st->Q = Q;
     st->iters += 1;
     st->total_iters += 1;
-    if (single && !view) {
+    if (pe.single && !pe.view) {
       st->moved = C->mover_count + C->hub_mover_count;
       const uint32_t t = C->trace_len;
       if (t < kTraceCap) {
@@ -1589,7 +1535,8 @@ __global__ void __launch_bounds__(1024) k_finalize(int dslot, int single, int np
   }
   // count graphs still iterating
   uint32_t tot;
-  block_excl_scan<uint32_t, 1024>(iterating, shc, &tot);
+  block_excl_scan<uint32_t, 256>(iterating, shc, &tot);
+  for (uint32_t i = threadIdx.x; i < C->n_chunks && i < kMaxChunks; i += 256) C->chunk_any[i] = 0;
   if (threadIdx.x == 0) {
     C->n_iterating = tot;
     C->loop_continue = tot > 0;
@@ -1600,19 +1547,31 @@ __global__ void __launch_bounds__(1024) k_finalize(int dslot, int single, int np
     C->hub_items = 0;
     C->apply_items = 0;
     C->hub_cursor = 0;
-    for (uint32_t i = 0; i < C->n_chunks && i < kMaxChunks; ++i) C->chunk_any[i] = 0;
-    if (!view) {
+    if (!pe.view) {
       C->act_entries_total += C->act_entries;
       C->act_vertices_total += C->act_vertices;
     }
     C->act_entries = 0;
     C->act_vertices = 0;
-    if (level_start) {
+    if (pe.level_start) {
       C->pass = 0;
+      // captured run: the level's optimisation tables must fit the arena; if not, the run stops with
+      // the level started and the host grows the arena and resumes
+      if (gc.on) {
+        const bool ok = C->arena_need <= C->arena_slots;
+        if (!ok) {
+          C->abort = kAbortOptArena;
+          C->abort_need = C->arena_need;
+        }
+        if (C->seg_aggs > kGuardLevels) atomicOr(&C->err, kErrLoop);
+        const bool go = ok && !(C->err & kErrLoop);
+        set_cond(gc, gc.level, go);
+        set_cond(gc, gc.pass, go && tot > 0);
+      }
     } else {
       C->it += 1;
       C->pass += 1;
-      if (!view) {
+      if (!pe.view) {
         C->seg_passes += 1;
         C->t_opt_ns += global_ns() - C->t_pass0;
       }
@@ -1620,28 +1579,126 @@ __global__ void __launch_bounds__(1024) k_finalize(int dslot, int single, int np
       // the captured pass loop runs while a graph iterates (and no guard has tripped)
       set_cond(gc, gc.pass, tot > 0 && !(C->err & kErrLoop));
     }
-    set_pass_rule(C, C->pass, mode, fast_first);
+    set_pass_rule(C, C->pass, pe.mode, pe.fast_first);
   }
 }
 
+// Integer mode squares exactly in u64 (a_c <= 2m < 2^32). One graph: per-block partials, summed in a
+// fixed order by the last block. Several graphs: warps take spans of kSqSpan vertices and add a
+// graph's part with one atomic where a span ends or the graph changes (a block per graph waited for
+// its largest graphs: up to 0.71 ms a pass on 768 graphs of up to 200,000 vertices, now 0.41); with fp32
+// weights a block per graph, so that the double sum has one order.
+constexpr uint32_t kSqSpan = 512;
+template <bool WINT>
+__global__ void __launch_bounds__(256) k_commit(int dslot, PassEnd pe, GraphCtl gc) {
+  const Dev& D = c_dev[dslot];
+  Ctrl* C = D.ctrl;
+  const uint32_t count = C->mover_count, hubs = C->hub_mover_count, n = C->n;
+  for (uint32_t i = blockIdx.x * blockDim.x + threadIdx.x; i < count + hubs; i += gridDim.x * blockDim.x) {
+    const uint32_t v = D.movers[i < count ? i : n - 1u - (i - count)];
+    const uint32_t c = D.new_comm[v];
+    D.comm[v] = c;
+    D.cn[v] = ((unsigned long long)c << 32) | c;
+  }
+  __shared__ double shd[33];
+  __shared__ unsigned long long shu[33];
+  if (pe.single) {
+    unsigned long long su = 0;
+    double sf = 0.0;
+    if (D.gs[0].phase == kIterating) {
+      for (uint32_t c = blockIdx.x * blockDim.x + threadIdx.x; c < n; c += gridDim.x * blockDim.x) {
+        const double x = D.a[c];
+        if (WINT) { const unsigned long long xi = (unsigned long long)x; su += xi * xi; }
+        else sf = __dadd_rn(sf, __dmul_rn(x, x));
+      }
+    }
+    if (WINT) {
+      unsigned long long tot;
+      block_excl_scan<unsigned long long, 256>(su, shu, &tot);
+      if (threadIdx.x == 0) reinterpret_cast<unsigned long long*>(D.partials)[blockIdx.x] = tot;
+    } else {
+      double tot;
+      block_excl_scan<double, 256>(sf, shd, &tot);
+      if (threadIdx.x == 0) D.partials[blockIdx.x] = tot;
+    }
+  } else if (WINT) {
+    const int lane = threadIdx.x & 31;
+    const uint32_t nwarps = (gridDim.x * blockDim.x) >> 5;
+    for (uint32_t sp = (blockIdx.x * blockDim.x + threadIdx.x) >> 5; (unsigned long long)sp * kSqSpan < n; sp += nwarps) {
+      uint32_t cur = kEmpty;  // the running graph
+      bool on = false;
+      unsigned long long su = 0;
+      auto flush = [&]() {
+        su = warp_sum(su);
+        if (lane == 0 && su) atomicAdd(&D.gs[cur].S, su);
+        su = 0;
+      };
+      const uint32_t end = min(n, (sp + 1u) * kSqSpan);
+      for (uint32_t b = sp * kSqSpan; b < end; b += 32) {
+        const bool live = b + lane < end;
+        const uint32_t c = live ? b + lane : b;
+        const uint32_t g = D.gid[c], g0 = __shfl_sync(kFull, g, 0);
+        const unsigned long long x = (unsigned long long)D.a[c];
+        if (__all_sync(kFull, g == g0)) {
+          if (g0 != cur) {
+            flush();
+            cur = g0;
+            on = D.gs[g0].phase == kIterating;
+          }
+          if (on && live) su += x * x;
+        } else if (live && D.gs[g].phase == kIterating) {
+          atomicAdd(&D.gs[g].S, x * x);
+        }
+      }
+      flush();
+    }
+  } else {
+    for (uint32_t g = blockIdx.x; g < C->G; g += gridDim.x) {
+      GraphState* st = &D.gs[g];
+      if (st->phase != kIterating) continue;
+      double sf = 0.0;
+      for (uint32_t c = st->vb + threadIdx.x; c < st->ve; c += blockDim.x) {
+        const double x = D.a[c];
+        sf = __dadd_rn(sf, __dmul_rn(x, x));
+      }
+      double tot;
+      block_excl_scan<double, 256>(sf, shd, &tot);
+      if (threadIdx.x == 0) st->S = __double_as_longlong(tot);
+    }
+  }
+  if (last_block(&C->commit_ticket)) finalize<WINT>(D, pe, gc);
+}
 
 // ---- level start ------------------------------------------------------------------------------------
 // Community::update (community.h:57-65): identity partition, totals = k, every vertex active
 // (phaseOptimization.cuh:52).
-__global__ void k_level_init(int dslot) {
+// The same walk sums the hash-table arena that the global-table bin (rows over min_deg entries whose
+// table exceeds block_cap slots) needs at this level.
+__global__ void k_level_init(int dslot, uint32_t min_deg, uint32_t block_cap) {
   const Dev& D = c_dev[dslot];
   Ctrl* C = D.ctrl;
   const uint32_t n = C->n, it = C->it;
+  unsigned long long need = 0;
   for (uint32_t v = blockIdx.x * blockDim.x + threadIdx.x; v < n; v += gridDim.x * blockDim.x) {
     const uint32_t g = D.gid ? D.gid[v] : 0u;
     if (D.gs[g].phase != kIterating) continue;
+    const uint32_t d = D.row[v + 1] - D.row[v];
+    if (d > min_deg) {
+      const uint32_t ng = D.gid ? D.gs[g].ve - D.gs[g].vb : n;
+      if (table_cap(d, ng) > block_cap) need += hub_table_cap(d, ng);
+    }
     // new_comm == comm marks "did not move" for the apply kernels (movers get new_comm != comm
-    // and k_commit_sq copies it back), so it starts equal too
+    // and k_commit copies it back), so it starts equal too
     D.comm[v] = v;
     D.new_comm[v] = v;
+    D.cn[v] = ((unsigned long long)v << 32) | v;
     D.a[v] = D.k[v];
     D.active_it[v] = it;
   }
+  need = warp_sum(need);
+  if ((threadIdx.x & 31) == 0 && need) atomicAdd(&C->arena_need, need);
+  if (blockIdx.x == 0)
+    for (int i = threadIdx.x; i < kMaxChunks; i += blockDim.x) C->chunk_any[i] = 0;
   if (blockIdx.x == 0 && threadIdx.x == 0) {
     C->mover_count = 0;
     C->long_movers = 0;
@@ -1650,8 +1707,6 @@ __global__ void k_level_init(int dslot) {
     C->apply_items = 0;
     for (int b = 0; b < kListBins; ++b) C->bin_count[b] = 0;
     C->hub_cursor = 0;
-    C->arena_need = 0;
-    for (int i = 0; i < kMaxChunks; ++i) C->chunk_any[i] = 0;
   }
 }
 
@@ -2101,24 +2156,6 @@ __global__ void k_rebase_pieces(long long* row64, uint32_t* col, const long long
   if (tid == 0) row64[n] = E;
 }
 
-// Hash-table arena needed by the global-table bin at this level: sum over vertices with
-// degree above the shared-memory bound of next_pow2(2 d).
-__global__ void k_arena_need(int dslot, uint32_t min_deg, uint32_t block_cap) {
-  const Dev& D = c_dev[dslot];
-  unsigned long long* need = &D.ctrl->arena_need;
-  const uint32_t n = D.ctrl->n;
-  unsigned long long s = 0;
-  for (uint32_t v = blockIdx.x * blockDim.x + threadIdx.x; v < n; v += gridDim.x * blockDim.x) {
-    const uint32_t d = D.row[v + 1] - D.row[v];
-    if (d <= min_deg) continue;
-    const uint32_t g = D.gid ? D.gid[v] : 0u;
-    const uint32_t ng = D.gid ? D.gs[g].ve - D.gs[g].vb : n;
-    if (table_cap(d, ng) > block_cap) s += hub_table_cap(d, ng);
-  }
-  s = warp_sum(s);
-  if ((threadIdx.x & 31) == 0 && s) atomicAdd(need, s);
-}
-
 // ---- aggregation -------------------------------------------------------------------------------------
 // phaseAggregation.cuh:27-43: new id = inclusive count of nonempty communities minus one. The
 // reference tests a_c > 0 (CountNotZero); with every weight positive that is exactly "has a
@@ -2131,22 +2168,13 @@ __global__ void k_agg_mark(int dslot) {
     D.map[D.comm[v]] = 1ull;
 }
 
-__global__ void k_agg_flags(int dslot) {
-  const Dev& D = c_dev[dslot];
-  const uint32_t n = D.ctrl->n;
-  for (uint32_t c = blockIdx.x * blockDim.x + threadIdx.x; c < n; c += gridDim.x * blockDim.x) {
-    const uint32_t g = D.gid ? D.gid[c] : 0u;
-    const unsigned long long ne = D.map[c] != 0ull ? 1ull : 0ull;
-    D.map[c] = (ne << 32) | (ne & (unsigned long long)D.gs[g].cont);
-  }
-}
-
-// Per graph: n_of_best_communities, base of its final ids, next-level vertex range.
-__global__ void k_agg_meta(int dslot) {
+// Per graph: n_of_best_communities, base of its final ids, next-level vertex range; then (captured
+// run) whether the contraction runs at all or the run ends. One block.
+__global__ void __launch_bounds__(1024) k_agg_meta(int dslot, GraphCtl gc) {
   const Dev& D = c_dev[dslot];
   Ctrl* C = D.ctrl;
   const uint32_t n = C->n;
-  for (uint32_t g = blockIdx.x * blockDim.x + threadIdx.x; g < C->G; g += gridDim.x * blockDim.x) {
+  for (uint32_t g = threadIdx.x; g < C->G; g += blockDim.x) {
     GraphState* st = &D.gs[g];
     if (!st->agg) continue;
     const unsigned long long before = st->vb > 0 ? D.map[st->vb - 1] : 0ull;
@@ -2155,7 +2183,17 @@ __global__ void k_agg_meta(int dslot) {
     st->n_best = (uint32_t)(end >> 32) - st->map_base;
     st->n_next = (uint32_t)end - (uint32_t)before;
   }
-  if (blockIdx.x == 0 && threadIdx.x == 0) C->n_next = n ? (uint32_t)D.map[n - 1] : 0u;
+  if (threadIdx.x == 0) {
+    const uint32_t n2 = n ? (uint32_t)D.map[n - 1] : 0u;
+    C->n_next = n2;
+    D.newdeg[n2] = 0;  // (the row-offset scan reads n2 + 1 entries)
+    if (gc.on) {
+      if (n2 > 0) C->seg_contract += 1; else C->seg_final += 1;
+      const bool go = n2 > 0 && !(C->err & kErrLoop);
+      set_cond(gc, gc.contract, go);
+      if (!go) set_cond(gc, gc.level, false);
+    }
+  }
 }
 
 // community.h:48-55 update_best: best[v0] = new(comm[best[v0]]). Graphs that stop here get
@@ -2192,18 +2230,8 @@ __global__ void k_agg_count(int dslot) {
     const uint32_t d = D.row[v + 1] - D.row[v];
     const unsigned long long old = atomicAdd(&D.cd[s], (1ull << 32) | d);
     D.rank[v] = (uint32_t)(old >> 32);
+    if (D.gidB) D.gidB[s] = g;
     D.new_comm[v] = s;  // next-level id of v's community, read by the contraction
-  }
-}
-
-__global__ void k_agg_scatter(int dslot) {
-  const Dev& D = c_dev[dslot];
-  const uint32_t n = D.ctrl->n;
-  for (uint32_t v = blockIdx.x * blockDim.x + threadIdx.x; v < n; v += gridDim.x * blockDim.x) {
-    const uint32_t g = D.gid ? D.gid[v] : 0u;
-    if (!D.gs[g].cont) continue;
-    const uint32_t s = D.new_comm[v];
-    D.members[(uint32_t)(D.cd[s] >> 32) + D.rank[v]] = v;
   }
 }
 
@@ -2218,10 +2246,19 @@ __device__ __forceinline__ uint32_t contract_cap(uint32_t dsum, uint32_t ng, boo
 // Bin the new communities by their summed member degree (the contraction's work). Bin 7
 // communities (the largest) are contracted by many blocks at once into a global table whose
 // arena offset is recorded per community in hubtab (kEmpty for every other community).
-__global__ void k_agg_bin(int dslot, BinCfg B) {
+// The same kernel places the members (independent work), and its last block checks (captured run)
+// that the global tables fit the arena; if not, the run stops here (nothing of this aggregation is
+// final yet) and the host grows the arena and redoes it.
+__global__ void __launch_bounds__(256) k_agg_scatter_bin(int dslot, BinCfg B, GraphCtl gc) {
   const Dev& D = c_dev[dslot];
   Ctrl* C = D.ctrl;
-  const uint32_t n2 = C->n_next;
+  const uint32_t n = C->n, n2 = C->n_next;
+  for (uint32_t v = blockIdx.x * blockDim.x + threadIdx.x; v < n; v += gridDim.x * blockDim.x) {
+    const uint32_t g = D.gid ? D.gid[v] : 0u;
+    if (!D.gs[g].cont) continue;
+    const uint32_t s = D.new_comm[v];
+    D.members[(uint32_t)(D.cd[s] >> 32) + D.rank[v]] = v;
+  }
   for (uint32_t base = blockIdx.x * blockDim.x; base < n2; base += gridDim.x * blockDim.x) {
     const uint32_t s = base + threadIdx.x;
     int bin = -1;
@@ -2230,37 +2267,75 @@ __global__ void k_agg_bin(int dslot, BinCfg B) {
       dsum = (uint32_t)D.cd[s + 1] - (uint32_t)D.cd[s];
       bin = bin_of(B, dsum);
       if (bin >= kNumBins - 2) {
-        const uint32_t g = D.gid ? D.gid[D.members[(uint32_t)(D.cd[s] >> 32)]] : 0u;
+        const uint32_t g = D.gid ? D.gidB[s] : 0u;
         cap = contract_cap(dsum, D.gs[g].n_next, bin == kNumBins - 1);
         // a bin-6 community whose table fits half the block table: the half-block list
         if (bin == kNumBins - 2 && 2u * cap <= B.block_cap) bin = kHalfBin;
       }
     }
+    // lane b claims bin b's space: one atomic latency for all bins
+    uint32_t want = 0, before = 0, mine = 0;
+    const uint32_t lane = threadIdx.x & 31;
 #pragma unroll
     for (int b = 0; b < kListBins; ++b) {
-      const uint32_t pos = warp_append(bin, b, &C->bin_count[b]);
-      if (pos != kEmpty) {
-        D.bins[b][pos] = s;
-        if (b == kNumBins - 1) {
-          const uint32_t off = atomicAdd(&C->hub_cursor, cap);
-          D.hub_off[pos] = off;
-          D.hubtab[s] = off;
-        }
+      const unsigned mk = __ballot_sync(kFull, bin == b);
+      if (lane == b) want = __popc(mk);
+      if (bin == b) before = __popc(mk & lanemask_lt());
+    }
+    if (want) mine = atomicAdd(&C->bin_count[lane], want);
+    const uint32_t pos = __shfl_sync(kFull, mine, bin < 0 ? 0 : bin) + before;
+    if (bin >= 0) {
+      D.bins[bin][pos] = s;
+      if (bin == kNumBins - 1) {
+        const uint32_t off = atomicAdd(&C->hub_cursor, cap);
+        D.hub_off[pos] = off;
+        D.hubtab[s] = off;
       }
     }
   }
+  if (gc.on && last_block(&C->bin_ticket) && threadIdx.x == 0) {
+    const uint32_t used = __ldcg(&C->hub_cursor);
+    const bool ok = used <= C->arena_slots;
+    if (ok) {
+      C->seg_contract_ok += 1;
+    } else {
+      C->abort = kAbortAggArena;
+      C->abort_need = used;
+      set_cond(gc, gc.level, false);
+    }
+    set_cond(gc, gc.ok, ok);
+  }
 }
 
-// Bin-7 set-up once the arena is large enough: owner of every table chunk, and zeroed
-// accumulators (row length, k') of each such community.
-__global__ void k_hub_owner(int dslot, int bin) {
+// Bin-7 set-up once the arena is large enough: empty tables, the owner of every table chunk, zeroed
+// accumulators (row length, k') of each such community, and where its members start among all
+// bin-7 members (exclusive prefix of their member counts, in `rank`, which is free after the
+// scatter; by the last block) and how many those are.
+template <bool WINT>
+__global__ void __launch_bounds__(256) k_hub_setup(int dslot) {
   const Dev& D = c_dev[dslot];
   Ctrl* C = D.ctrl;
-  const uint32_t count = C->bin_count[bin];
+  __shared__ uint32_t sh[33];
+  const uint32_t count = C->bin_count[kNumBins - 1];
+  if (blockIdx.x == gridDim.x - 1) {
+    uint32_t run = 0;
+    for (uint32_t base = 0; base < count; base += 256) {
+      const uint32_t idx = base + threadIdx.x;
+      uint32_t m = 0;
+      if (idx < count) {
+        const uint32_t s = D.bins[kNumBins - 1][idx];
+        m = (uint32_t)(D.cd[s + 1] >> 32) - (uint32_t)(D.cd[s] >> 32);
+      }
+      uint32_t tot;
+      const uint32_t ex = block_excl_scan<uint32_t, 256>(m, sh, &tot);
+      if (idx < count) D.rank[idx] = run + ex;
+      run += tot;
+    }
+    if (threadIdx.x == 0) C->hub_members = run;
+  }
   for (uint32_t idx = blockIdx.x; idx < count; idx += gridDim.x) {
-    const uint32_t s = D.bins[bin][idx];
-    const uint32_t v0 = D.members[(uint32_t)(D.cd[s] >> 32)];
-    const uint32_t g = D.gid ? D.gid[v0] : 0u;
+    const uint32_t s = D.bins[kNumBins - 1][idx];
+    const uint32_t g = D.gid ? D.gidB[s] : 0u;
     const uint32_t dsum = (uint32_t)D.cd[s + 1] - (uint32_t)D.cd[s];
     const uint32_t cap = contract_cap(dsum, D.gs[g].n_next, true);
     const uint32_t c0 = D.hub_off[idx] / kHubChunk;
@@ -2269,9 +2344,11 @@ __global__ void k_hub_owner(int dslot, int bin) {
       D.newdeg[s] = 0;
       D.kB[s] = 0.0;
       D.hubself[s] = 0ull;
-      if (D.gidB) D.gidB[s] = g;
     }
   }
+  const uint32_t used = min(C->hub_cursor, C->arena_slots);
+  for (uint32_t s = blockIdx.x * blockDim.x + threadIdx.x; s < used; s += gridDim.x * blockDim.x)
+    arena_clear_slot<WINT>(D, s);
 }
 
 // Insert into a community's global contraction table at arena offset `off` (capacity `cap`).
@@ -2299,29 +2376,6 @@ __device__ __forceinline__ void hub_table_load(const Dev& D, uint32_t i, uint32_
     key = D.arena_keys[i];
     sum = key != kEmpty ? reinterpret_cast<const Acc*>(D.arena_vals)[i] : Acc(0);
   }
-}
-
-// Where the members of each bin-7 community start among all bin-7 members (exclusive prefix of
-// their member counts, in `rank`, which is free after the scatter) and how many there are.
-__global__ void __launch_bounds__(1024) k_hub_member_prefix(int dslot) {
-  const Dev& D = c_dev[dslot];
-  __shared__ uint32_t sh[33];
-  Ctrl* C = D.ctrl;
-  const uint32_t count = C->bin_count[kNumBins - 1];
-  uint32_t run = 0;
-  for (uint32_t base = 0; base < count; base += 1024) {
-    const uint32_t idx = base + threadIdx.x;
-    uint32_t m = 0;
-    if (idx < count) {
-      const uint32_t s = D.bins[kNumBins - 1][idx];
-      m = (uint32_t)(D.cd[s + 1] >> 32) - (uint32_t)(D.cd[s] >> 32);
-    }
-    uint32_t tot;
-    const uint32_t ex = block_excl_scan<uint32_t, 1024>(m, sh, &tot);
-    if (idx < count) D.rank[idx] = run + ex;
-    run += tot;
-  }
-  if (threadIdx.x == 0) C->hub_members = run;
 }
 
 // Bin-7 insert: the members of all large communities at once (and no other vertex), 32 per
@@ -2889,6 +2943,7 @@ __global__ void k_agg_finish(int dslot) {
     st->agg = 0;
   }
   if (tid == 0) {
+    C->arena_need = 0;  // summed by the next level's start
     C->E_next = D.rowB[n2];
     C->n = n2;
     C->E = C->E_next;
@@ -2898,17 +2953,26 @@ __global__ void k_agg_finish(int dslot) {
   }
 }
 
-// Which graphs aggregate now and whether they continue: modularityAlgorithms.h:52
-// cont = Q_end - Q_level_start > threshold. force >= 0 overrides (phase-level API).
-// defer_i: a refined run resets I in k_ref_decide, once refinement has decided.
-__global__ void k_agg_decide(int dslot, int force, uint32_t max_levels, int defer_i) {
+// Start of an aggregation: which graphs aggregate now and whether they continue
+// (modularityAlgorithms.h:52, cont = Q_end - Q_level_start > threshold; force >= 0 overrides, for
+// the phase-level API; defer_i: a refined run resets I in k_ref_decide, once refinement has
+// decided), and the cleared scratch: community marks, per-new-community counters and hub offsets
+// (their number is not known yet, but at most n), the counters the binning appends with. An
+// aggregation can be run again from here.
+__global__ void k_agg_begin(int dslot, int force, uint32_t max_levels, int defer_i) {
   const Dev& D = c_dev[dslot];
   Ctrl* C = D.ctrl;
-  if (blockIdx.x == 0 && threadIdx.x == 0) {
+  const uint32_t n = C->n;
+  const uint32_t tid = blockIdx.x * blockDim.x + threadIdx.x, nth = gridDim.x * blockDim.x;
+  if (tid == 0) {
     C->t_agg0 = global_ns();
     C->seg_aggs += 1;
+    for (int b = 0; b < kListBins; ++b) C->bin_count[b] = 0;
+    C->hub_cursor = 0;
+    C->long_count = 0;  // k_hub_insert queues this aggregation's long rows from zero
+    C->hub_work = 0;    // and takes its member groups from zero
   }
-  for (uint32_t g = blockIdx.x * blockDim.x + threadIdx.x; g < C->G; g += gridDim.x * blockDim.x) {
+  for (uint32_t g = tid; g < C->G; g += nth) {
     GraphState* st = &D.gs[g];
     if (st->phase == kFinished) { st->agg = 0; continue; }
     st->agg = 1;
@@ -2919,93 +2983,33 @@ __global__ void k_agg_decide(int dslot, int force, uint32_t max_levels, int defe
     st->cont = cont;
     if (cont && !defer_i) st->I = 0;  // the contraction adds the next level's self-loop weight
   }
+  for (uint32_t i = tid; i <= n; i += nth) {
+    D.cd[i] = 0ull;
+    if (i < n) {
+      D.map[i] = 0ull;
+      D.hubtab[i] = kEmpty;
+    }
+  }
 }
-
-// ---- device-sized clears and the gates of a captured run ----------------------------------------
-// Aggregation scratch cleared to the level's own sizes (read on the device).
-__global__ void k_agg_clear_map(int dslot) {
-  const Dev& D = c_dev[dslot];
-  const uint32_t n = D.ctrl->n;
-  for (uint32_t i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x) D.map[i] = 0ull;
-}
-// Before the contraction: per-new-community counters and hub offsets, and the counters the
-// binning appends with (so that an aggregation can be run again from its start).
-__global__ void k_agg_clear_next(int dslot) {
+// The same scratch and counters again, after the refinement passes have used them.
+__global__ void k_agg_clear(int dslot) {
   const Dev& D = c_dev[dslot];
   Ctrl* C = D.ctrl;
-  const uint32_t n2 = C->n_next;
-  for (uint32_t i = blockIdx.x * blockDim.x + threadIdx.x; i <= n2; i += gridDim.x * blockDim.x) {
-    D.cd[i] = 0ull;
-    if (i < n2) D.hubtab[i] = kEmpty;
-  }
+  const uint32_t n = C->n;
+  for (uint32_t i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x) D.map[i] = 0ull;
   if (blockIdx.x == 0 && threadIdx.x == 0) {
-    D.newdeg[n2] = 0;
     for (int b = 0; b < kListBins; ++b) C->bin_count[b] = 0;
     C->hub_cursor = 0;
-    C->long_count = 0;  // k_hub_insert queues this aggregation's long rows from zero
-    C->hub_work = 0;    // and takes its member groups from zero
+    C->long_count = 0;
+    C->hub_work = 0;
   }
-}
-// The global contraction tables of this aggregation: empty keys, zero values.
-template <bool WINT>
-__global__ void k_arena_clear(int dslot) {
-  const Dev& D = c_dev[dslot];
-  Ctrl* C = D.ctrl;
-  const uint32_t used = min(C->hub_cursor, C->arena_slots);
-  for (uint32_t s = blockIdx.x * blockDim.x + threadIdx.x; s < used; s += gridDim.x * blockDim.x)
-    arena_clear_slot<WINT>(D, s);
-}
-// Level body entry: the pass loop runs while some graph iterates.
-__global__ void k_gate_pass(int dslot, GraphCtl gc) {
-  const Dev& D = c_dev[dslot];
-  Ctrl* C = D.ctrl;
-  if (C->seg_aggs > kGuardLevels) atomicOr(&C->err, kErrLoop);
-  const bool stop = (C->err & kErrLoop) != 0;
-  set_cond(gc, gc.pass, C->n_iterating > 0 && !stop);
-  if (stop) set_cond(gc, gc.level, false);
-}
-// After the renumbering: contract (then-branch) when some graph continues, else the run ends.
-__global__ void k_gate_contract(int dslot, GraphCtl gc) {
-  const Dev& D = c_dev[dslot];
-  Ctrl* C = D.ctrl;
-  const bool more = C->n_next > 0;
-  if (more) C->seg_contract += 1; else C->seg_final += 1;
-  const bool stop = (C->err & kErrLoop) != 0;
-  set_cond(gc, gc.contract, more && !stop);
-  if (!more || stop) set_cond(gc, gc.level, false);
-}
-// After the contraction binning: its global tables must fit the arena; if not, the run stops
-// here (nothing of this aggregation is final yet) and the host grows the arena and redoes it.
-__global__ void k_gate_arena_agg(int dslot, GraphCtl gc) {
-  const Dev& D = c_dev[dslot];
-  Ctrl* C = D.ctrl;
-  const bool ok = C->hub_cursor <= C->arena_slots;
-  if (ok) {
-    C->seg_contract_ok += 1;
-  } else {
-    C->abort = kAbortAggArena;
-    C->abort_need = C->hub_cursor;
-    set_cond(gc, gc.level, false);
-  }
-  set_cond(gc, gc.ok, ok);
-}
-// End of a level start: the next level's optimisation tables must fit the arena; if not, the
-// run stops with the level started and the host grows the arena and resumes.
-__global__ void k_gate_level(int dslot, GraphCtl gc) {
-  const Dev& D = c_dev[dslot];
-  Ctrl* C = D.ctrl;
-  const bool ok = C->arena_need <= C->arena_slots;
-  if (!ok) {
-    C->abort = kAbortOptArena;
-    C->abort_need = C->arena_need;
-  }
-  set_cond(gc, gc.level, ok && !(C->err & kErrLoop));
 }
 
-// ---- scans (3-phase: tile sums, scan of tile sums, tile scan + offset) ---------------------------
+// ---- scans (tile sums, scanned by the last block; tile scan + offset) ------------------------------
 // The three scans of an aggregation, each named by what it scans so that its arrays and length
 // come from the device state (a captured run replays them at every level with every size):
-//   kScanMap: map -> map, inclusive, n entries (community renumbering)
+//   kScanMap: map -> map, inclusive, n entries (community renumbering: nonempty communities in the
+//             high word, those of graphs that continue to a new level in the low one)
 //   kScanCd:  cd -> cd, exclusive, n_next + 1 entries (members and degree sums per community)
 //   kScanDeg: newdeg -> rowB, exclusive, n_next + 1 entries (next-level row offsets)
 // The blocks stride over tiles, so the grid does not depend on the size either.
@@ -3032,6 +3036,13 @@ __device__ __forceinline__ T* scan_out(const Dev& D) {
 }
 
 template <class T, int SRC>
+__device__ __forceinline__ T scan_value(const Dev& D, const T* in, uint64_t j) {
+  const T x = in[j];
+  if constexpr (SRC == kScanMap) return x ? ((T)1 << 32) | (T)D.gs[D.gid ? D.gid[j] : 0u].cont : (T)0;
+  else return x;
+}
+
+template <class T, int SRC>
 __global__ void __launch_bounds__(kScanNT) k_scan_tiles(int dslot) {
   const Dev& D = c_dev[dslot];
   __shared__ T sh[33];
@@ -3045,29 +3056,22 @@ __global__ void __launch_bounds__(kScanNT) k_scan_tiles(int dslot) {
 #pragma unroll
     for (int i = 0; i < kScanIPT; ++i) {
       const uint64_t j = base + (uint64_t)i * kScanNT + threadIdx.x;
-      if (j < n) s += in[j];
+      if (j < n) s += scan_value<T, SRC>(D, in, j);
     }
     T tot;
     block_excl_scan<T, kScanNT>(s, sh, &tot);
     if (threadIdx.x == 0) tile_sums[t] = tot;
   }
-}
-
-template <class T, int SRC>
-__global__ void __launch_bounds__(1024) k_scan_sums(int dslot) {
-  const Dev& D = c_dev[dslot];
-  __shared__ T sh[33];
-  const uint32_t ntiles = (scan_len<SRC>(D) + kScanTile - 1) / kScanTile;
-  T* tile_sums = reinterpret_cast<T*>(D.scan_tmp);
-  // each thread scans a contiguous run, then the block scans the run totals
-  const uint32_t per = (ntiles + 1023) / 1024;
+  if (!last_block(&D.ctrl->scan_ticket)) return;
+  // each thread scans a contiguous run of the tile sums, then the block scans the run totals
+  const uint32_t per = (ntiles + kScanNT - 1) / kScanNT;
   const uint32_t b = threadIdx.x * per, e = min(b + per, ntiles);
   T s = T(0);
-  for (uint32_t i = b; i < e; ++i) s += tile_sums[i];
+  for (uint32_t i = b; i < e; ++i) s += __ldcg(tile_sums + i);
   T tot;
-  T off = block_excl_scan<T, 1024>(s, sh, &tot);
+  T off = block_excl_scan<T, kScanNT>(s, sh, &tot);
   for (uint32_t i = b; i < e; ++i) {
-    const T x = tile_sums[i];
+    const T x = __ldcg(tile_sums + i);
     tile_sums[i] = off;
     off += x;
   }
@@ -3091,7 +3095,7 @@ __global__ void __launch_bounds__(kScanNT) k_scan_apply(int dslot) {
 #pragma unroll
     for (int i = 0; i < kScanIPT; ++i) {
       const uint64_t j = base + i;
-      vals[i] = j < n ? in[j] : T(0);
+      vals[i] = j < n ? scan_value<T, SRC>(D, in, j) : T(0);
       s += vals[i];
     }
     T tot;

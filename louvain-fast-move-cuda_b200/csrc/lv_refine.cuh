@@ -65,6 +65,7 @@ __global__ void k_ref_init(int dslot, uint32_t max_levels) {
   for (uint32_t v = tid; v < n; v += nth) {
     D.ref[v] = v;
     D.ref_new[v] = v;
+    D.cn[v] = ((unsigned long long)v << 32) | v;  // (the refine view's: shared, the level has ended)
     D.aref[v] = D.k[v];
     D.rsz[v] = 1u;
     D.rflag[v] = 0u;
@@ -361,7 +362,9 @@ __global__ void k_ref_reject(int dslot) {
     if (v >= n) continue;
     if (D.rflag[v] & kRefReject) {
       D.rflag[v] &= ~kRefReject;
-      D.new_comm[v] = D.comm[v];
+      const uint32_t c = D.comm[v];
+      D.new_comm[v] = c;
+      D.cn[v] = ((unsigned long long)c << 32) | c;
     } else {
       const uint32_t t = D.new_comm[v];
       if (t >= n) continue;
