@@ -58,6 +58,7 @@ struct GraphState {
   uint32_t total_iters;
   uint32_t moved;     // moves of the last pass
   uint32_t n_next;    // aggregation: vertices of this graph at the next level
+  unsigned long long I_full;  // internal weight summed by k_apply_full (u64 or double bits)
   double inv_m;       // rn(1/m) and rn(1/two_m2), for the gain upper bound only
   double inv_2m2;
 };
@@ -135,6 +136,7 @@ struct Ctrl {
   uint32_t small_work[2];      // next graph of each k_small class
   uint32_t commit_ticket, scan_ticket, bin_ticket;  // blocks done: the last one does the kernel's tail
   uint32_t pad_ticket;
+  unsigned long long mover_entries;  // entries of this pass's movers
   TraceRec trace[kTraceCap];
 };
 

@@ -32,7 +32,7 @@ namespace lv {
 // Everything that fixes the kernel sequence of a captured run apart from the data: when two
 // runs agree on it, the second reuses the first one's instantiated graph.
 struct GraphKey {
-  int32_t wint, single, mode, fast_first, max_levels, sms, grid_n, grid_sq, grid_block;
+  int32_t wint, single, full_walk, mode, fast_first, max_levels, sms, grid_n, grid_sq, grid_block;
   int64_t chunk_edges;
   uint32_t maxdeg[kNumBins], block_cap, team_cap[6];
   int32_t grid_team[6];
@@ -266,6 +266,7 @@ class Run {
   bool own_pinned = false;
   bool finished = false;
   bool chunked = false;        // level 0 spans several edge chunks (later levels have fewer entries)
+  bool full_walk = false;      // some level can have a heavy pass (later levels have fewer entries)
   bool small_ok = false;       // a whole run from its input: k_small may take its small graphs
   int32_t levels_run = 0;
   double t_opt_ms = 0, t_agg_ms = 0, t_opt0 = -1, t_agg0 = -1, t_optk_ms = 0;
@@ -748,6 +749,7 @@ class Run {
     else k_prep_total<false><<<1, 256, 0, st>>>(Dd);
     launches += 4;
     chunked = single() && cfg.chunk_edges > 0 && (int64_t)E > cfg.chunk_edges;
+    full_walk = E >= kFullMinE;
     plan_small(ho, eo);
     if (small_count()) return;  // louvain() starts with them
     check_device_errors();
@@ -875,9 +877,14 @@ class Run {
       launches += 2;
     }
     if (!gc.on) LV_CUDA(cudaEventRecord(ev[5], st));
-    fork(1);
+    fork(full_walk ? 2 : 1);
     on(1);
     k_apply_hub<WI><<<ctx->sms * 8, 256, 0, st>>>(Dd);
+    if (full_walk) {
+      on(2);
+      k_apply_full<WI><<<ctx->sms * 8, 256, 0, st>>>(Dd);
+      ++launches;
+    }
     on(0);
     k_apply<WI><<<grid_n, 256, 0, st>>>(Dd);
     k_apply_long<WI><<<grid_n, 256, 0, st>>>(Dd);
@@ -1123,6 +1130,7 @@ class Run {
     std::memset(&k, 0, sizeof(k));
     k.wint = wint;
     k.single = single();
+    k.full_walk = full_walk;
     k.mode = cfg.mode;
     k.fast_first = cfg.fast_first;
     k.max_levels = cfg.max_levels;

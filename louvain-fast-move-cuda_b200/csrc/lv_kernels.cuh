@@ -322,20 +322,28 @@ struct MoverStage {
   uint32_t n;       // staged, below 32 between calls (warp-uniform)
   uint32_t* list;   // the mover list and its counter
   uint32_t* count;
+  unsigned long long* entries;  // entries of all movers (nullptr: not counted)
+  uint32_t acc;     // this lane's, since the last flush
   __device__ __forceinline__ void flush(uint32_t cnt) {
     const uint32_t lane = threadIdx.x & 31;
     uint32_t base = 0;
     if (lane == 0) base = atomicAdd(count, cnt);
+    if (entries) {
+      const uint32_t e = __reduce_add_sync(kFull, acc);
+      if (lane == 0) atomicAdd(entries, (unsigned long long)e);
+      acc = 0;
+    }
     base = __shfl_sync(kFull, base, 0);
     if (lane < cnt) list[base + lane] = v[lane];
   }
-  // vtx moves from community `pre` to c
-  __device__ __forceinline__ void add(const Dev& D, bool move, uint32_t vtx, uint32_t pre, uint32_t c) {
+  // vtx (row length d) moves from community `pre` to c
+  __device__ __forceinline__ void add(const Dev& D, bool move, uint32_t vtx, uint32_t pre, uint32_t c, uint32_t d) {
     const unsigned mask = __ballot_sync(kFull, move);
     if (!mask) return;
     if (move) {
       D.new_comm[vtx] = c;
       D.cn[vtx] = ((unsigned long long)c << 32) | pre;
+      acc += d;
       v[n + __popc(mask & lanemask_lt())] = vtx;
     }
     n += __popc(mask);
@@ -369,6 +377,7 @@ __device__ __forceinline__ void emit_hub_move(const Dev& D, uint32_t v, uint32_t
   D.new_comm[v] = c;
   D.cn[v] = ((unsigned long long)c << 32) | pre;
   D.movers[C->n - 1u - atomicAdd(&C->hub_mover_count, 1u)] = v;
+  atomicAdd(&C->mover_entries, (unsigned long long)d);
   const uint32_t np = (d + kHubPiece - 1) / kHubPiece;
   const uint32_t p0 = atomicAdd(&C->apply_items, np);
   for (uint32_t k = 0; k < np; ++k) D.apply_items[p0 + k] = ((unsigned long long)v << 32) | k;
@@ -696,7 +705,7 @@ __global__ void __launch_bounds__(256, 4) k_opt_team(int dslot, int bin, uint32_
   const unsigned tmask = T == 32 ? kFull : (((1u << T) - 1u) << ((threadIdx.x & 31) & ~(uint32_t)(T - 1)));
   uint32_t err = 0;
   __shared__ uint32_t s_mov[8][64];
-  MoverStage mv{s_mov[threadIdx.x >> 5], 0u, D.movers, &C->mover_count};
+  MoverStage mv{s_mov[threadIdx.x >> 5], 0u, D.movers, &C->mover_count, &C->mover_entries, 0u};
   ScratchTable<WINT> tbl{keys, vals, slots, cap - 1u, 0u};
   if (!fast) {
     for (uint32_t s = lane; s < cap; s += T) tbl.clear(s);
@@ -745,7 +754,7 @@ __global__ void __launch_bounds__(256, 4) k_opt_team(int dslot, int bin, uint32_
       c = key_comm(best, lowest);
       move = c != x.cv && (!fast || v <= c);
     }
-    mv.add(D, move, v, x.cv, c);
+    mv.add(D, move, v, x.cv, c, x.re - x.rs);
   }
   mv.finish();
   if (err) report_err(C, err, 0);  // k_opt_team
@@ -865,7 +874,7 @@ __device__ __forceinline__ void short_rows(const Dev& D, const uint32_t* vlist, 
     c = key_comm(best, lowest);
     move = c != x.cv;
   }
-  mv.add(D, move, v, x.cv, c);
+  mv.add(D, move, v, x.cv, c, x.re - x.rs);
 }
 
 // Rows of the fast pass, T lanes each (T a power of two up to 32, the same for the whole warp).
@@ -884,19 +893,23 @@ __device__ __forceinline__ void fast_rows(const Dev& D, const uint32_t* vlist, u
     best = y > best ? y : best;
   }
   const uint32_t c = key_comm(best, true);
-  mv.add(D, live && lane == 0 && best && c != x.cv && v <= c, v, x.cv, c);
+  mv.add(D, live && lane == 0 && best && c != x.cv && v <= c, v, x.cv, c, x.re - x.rs);
 }
 
 // The short bins in one launch (`mask`: bit b = bin b is taken here; a bin whose configured limit
-// exceeds 4 T stays with k_opt_team). A block takes a contiguous share of each bin's list, so that
-// the movers it stages together are neighbours; the shares of different bins start at different
-// blocks, so that small lists spread over the GPU.
+// exceeds 4 T stays with k_opt_team). A block takes runs of kShortRun consecutive tiles of a list: long
+// enough that the movers a warp stages together are neighbours (of one graph, in a batch), short
+// enough that the grid moves through the list together, so that a batch's gathers stay within the
+// few graphs in flight and in L2 (a contiguous share per block instead: 1.61
+// against 1.22 ms for the first pass over 768 graphs with 20 M vertices). The runs of different bins
+// start at different blocks, so that small lists spread over the GPU.
+constexpr uint32_t kShortRun = 8;
 template <bool WINT>
 __global__ void __launch_bounds__(256, WINT ? 4 : 3) k_opt_short(int dslot, uint32_t mask) {
   const Dev& D = c_dev[dslot];
   Ctrl* C = D.ctrl;
   __shared__ uint32_t s_mov[8][64];
-  MoverStage mv{s_mov[threadIdx.x >> 5], 0u, D.movers, &C->mover_count};
+  MoverStage mv{s_mov[threadIdx.x >> 5], 0u, D.movers, &C->mover_count, &C->mover_entries, 0u};
   const bool fast = C->fast != 0;
   const bool lowest = C->rule_sort != 0;
   const bool unit = unit_weights<WINT>(C);
@@ -907,9 +920,10 @@ __global__ void __launch_bounds__(256, WINT ? 4 : 3) k_opt_short(int dslot, uint
     const uint32_t per = 256u >> b;  // rows per block step
     const uint32_t tiles = (count + per - 1) / per;
     const uint32_t blk = (blockIdx.x + (uint32_t)b * (gridDim.x / kShortBins)) % gridDim.x;
-    const uint32_t t0 = (uint32_t)((unsigned long long)blk * tiles / gridDim.x);
-    const uint32_t t1 = (uint32_t)((unsigned long long)(blk + 1) * tiles / gridDim.x);
-    for (uint32_t t = t0; t < t1; ++t) {
+    // tiles a block takes in a row: up to kShortRun, fewer while the list does not fill the grid
+    const uint32_t run = min(kShortRun, max(1u, tiles / gridDim.x));
+    for (uint32_t t0 = blk * run; t0 < tiles; t0 += gridDim.x * run)
+    for (uint32_t t = t0, t1 = min(tiles, t0 + run); t < t1; ++t) {
       const uint32_t idx = t * per + (threadIdx.x >> b);
       if (fast) fast_rows<WINT>(D, D.bins[b], idx, count, 1u << b, mv, load);
       else if (b == 0) short_rows<1, WINT>(D, D.bins[0], idx, count, lowest, unit, mv, load);
@@ -1245,9 +1259,24 @@ __device__ __forceinline__ void apply_entries(const Dev& D, uint32_t v, uint32_t
 // costs one 8-byte gather: kept up by the level start, the kernels that emit moves and the commit.)
 constexpr uint32_t kApplyShort = 32;
 
+// A heavy pass -- its movers own at least half of the level's entries, as in most first passes of a
+// level -- is applied by k_apply_full, which walks every row instead of the movers'. A pushed entry
+// costs 9-16 ps while the per-vertex state stays in L2 and about 33 ps beyond (kL2Vertices: 20 bytes
+// of it per vertex against 126 MB), a walked one 4-8 ps. Pushed -> walked, us: R-MAT scale 22 at 55 %
+// of the entries 1145 -> 590, at 24 % 482 -> 580; planted partition at 50 % 125 -> 180; 768 graphs
+// with 20 M vertices at 35 % 2500 -> 1540, at 19 % 1560 -> 1370, at 13 % 1100 -> 1240. Below kFullMinE
+// entries the walk's own latency (about 40 us) is not worth it.
+constexpr uint32_t kFullMinE = 1u << 22;
+constexpr uint32_t kL2Vertices = 6000000;
+__device__ __forceinline__ bool heavy_pass(const Ctrl* C) {
+  const unsigned long long e = C->mover_entries, all = C->E;
+  return all >= kFullMinE && (C->n >= kL2Vertices ? e * 6ull > all : e * 2ull > all);
+}
+
 // The walk over the rows of up to 32 movers held one per lane (row start rs, length len, 0 for none,
 // pre-pass community old, target nw), all lanes busy whatever the row lengths: activity push, and
-// add(u, f, w as double, w as u32) for every entry (to u) that changes the internal weight by f w.
+// add(k, f, w as double, w as u32) for every entry (of lane k's row) that changes the internal weight
+// by f w.
 template <bool WINT, int NB = kApplyBatch, class F>
 __device__ __forceinline__ void apply_rows(const Dev& D, uint32_t rs, uint32_t len, uint32_t old, uint32_t nw,
                                            uint32_t it, bool unit, F&& add) {
@@ -1265,6 +1294,7 @@ __device__ __forceinline__ void apply_rows(const Dev& D, uint32_t rs, uint32_t l
   const uint32_t excl = incl - len;
   for (uint32_t jb = 0; jb < total; jb += 32u * NB) {
     uint32_t ee[NB], oo[NB], nn[NB], uu[NB], pre[NB], nc[NB];
+    int kk[NB];
 #pragma unroll
     for (int q = 0; q < NB; ++q) {
       const uint32_t j = jb + (uint32_t)q * 32u + lane;
@@ -1274,6 +1304,7 @@ __device__ __forceinline__ void apply_rows(const Dev& D, uint32_t rs, uint32_t l
         const uint32_t ex = __shfl_sync(kFull, excl, k + step);
         if (ex <= j) k += step;
       }
+      kk[q] = k;
       ee[q] = __shfl_sync(kFull, rs, k) + (j - __shfl_sync(kFull, excl, k));
       oo[q] = __shfl_sync(kFull, old, k);
       nn[q] = __shfl_sync(kFull, nw, k);
@@ -1295,9 +1326,29 @@ __device__ __forceinline__ void apply_rows(const Dev& D, uint32_t rs, uint32_t l
       const int dd = (int)(nn[q] == post) - (int)(oo[q] == pre[q]);
       if (dd) {
         const int f = mu ? dd : 2 * dd;
-        if (WINT) add(u, f, 0.0, unit ? 1u : (uint32_t)w[ee[q]]);
-        else add(u, f, Tr::w_double(w[ee[q]]), 0u);
+        if (WINT) add(kk[q], f, 0.0, unit ? 1u : (uint32_t)w[ee[q]]);
+        else add(kk[q], f, Tr::w_double(w[ee[q]]), 0u);
       }
+    }
+  }
+}
+
+// Adds each lane's internal-weight change (vi or vf) to its graph's sum (field `at` of the graph
+// states): one atomic per distinct graph among the lanes. Every lane of the warp calls it.
+template <bool WINT>
+__device__ __forceinline__ void add_by_graph(const Dev& D, unsigned long long GraphState::*at, uint32_t g,
+                                             long long vi, double vf) {
+  unsigned todo = __ballot_sync(kFull, WINT ? vi != 0 : vf != 0.0);
+  while (todo) {
+    const uint32_t gl = __shfl_sync(kFull, g, __ffs(todo) - 1);
+    const bool mine = g == gl;
+    todo &= ~__ballot_sync(kFull, mine);
+    if (WINT) {
+      const long long t = warp_sum(mine ? vi : 0ll);
+      if ((threadIdx.x & 31) == 0) atomicAdd(&(D.gs[gl].*at), (unsigned long long)t);
+    } else {
+      const double t = warp_sum(mine ? vf : 0.0);
+      if ((threadIdx.x & 31) == 0) atomicAdd(reinterpret_cast<double*>(&(D.gs[gl].*at)), t);
     }
   }
 }
@@ -1310,18 +1361,20 @@ __global__ void __launch_bounds__(256) k_apply(int dslot) {
   if (blockIdx.x == 0 && threadIdx.x == 0) C->t_optk_ns += global_ns() - C->t_pass0;
   const uint32_t count = C->mover_count, it = C->it;
   const bool unit = unit_weights<WINT>(C);
+  const bool heavy = heavy_pass(C);  // then only the totals here
   const int lane = threadIdx.x & 31;
   const uint32_t warp = (blockIdx.x * blockDim.x + threadIdx.x) >> 5;
   const uint32_t nwarps = (gridDim.x * blockDim.x) >> 5;
-  uint32_t gcur = 0;  // graph of the running internal-weight change
+  // The internal weight's change: per lane while a step's 32 movers are of one graph (summed over the
+  // warp when the graph changes), else per mover in shared memory. (Added per lane at every change
+  // of graph it was one atomic per lane and step on the graphs' few words.)
+  __shared__ unsigned long long s_row[8][32];
+  unsigned long long* row = s_row[threadIdx.x >> 5];
+  uint32_t gcur = 0;
   long long di = 0;
   double df = 0.0;
   auto flush = [&]() {
-    if (WINT) {
-      if (di) atomicAdd(&D.gs[gcur].I, (unsigned long long)di);
-    } else if (df != 0.0) {
-      atomicAdd(reinterpret_cast<double*>(&D.gs[gcur].I), df);
-    }
+    add_by_graph<WINT>(D, &GraphState::I, gcur, di, df);
     di = 0;
     df = 0.0;
   };
@@ -1341,6 +1394,7 @@ __global__ void __launch_bounds__(256) k_apply(int dslot) {
         atomicAdd(&D.a[old], -kv);
       }
     }
+    if (heavy) continue;
     // long rows: queued for k_apply_long (the list lives in `members`, unused during passes)
     const bool defer = len > kApplyShort;
     const unsigned dm = __ballot_sync(kFull, defer);
@@ -1351,26 +1405,34 @@ __global__ void __launch_bounds__(256) k_apply(int dslot) {
       if (defer) D.members[b0 + __popc(dm & lanemask_lt())] = v;
     }
     if (defer) len = 0;
-    apply_rows<WINT>(D, rs, len, old, nw, it, unit, [&](uint32_t u, int f, double wt, uint32_t wi) {
-      if (D.gid) {
-        const uint32_t g = D.gid[u];
-        if (g != gcur) {
-          flush();
-          gcur = g;
-        }
+    uint32_t g = 0;
+    bool one = true;
+    if (D.gid) {
+      g = D.gid[idx < count ? v : D.movers[base]];
+      one = __all_sync(kFull, g == __shfl_sync(kFull, g, 0));
+      if (one && g != gcur) {
+        flush();
+        gcur = g;
       }
-      if (WINT) di += (long long)f * (long long)wi;
-      else df += (double)f * wt;
-    });
+    }
+    if (one) {
+      apply_rows<WINT>(D, rs, len, old, nw, it, unit, [&](int, int f, double wt, uint32_t wi) {
+        if (WINT) di += (long long)f * (long long)wi;
+        else df += (double)f * wt;
+      });
+    } else {
+      row[lane] = 0ull;
+      __syncwarp();
+      apply_rows<WINT>(D, rs, len, old, nw, it, unit, [&](int k, int f, double wt, uint32_t wi) {
+        if (WINT) atomicAdd(&row[k], (unsigned long long)((long long)f * (long long)wi));
+        else atomicAdd(reinterpret_cast<double*>(&row[k]), (double)f * wt);
+      });
+      __syncwarp();
+      add_by_graph<WINT>(D, &GraphState::I, g, (long long)row[lane], __longlong_as_double((long long)row[lane]));
+      __syncwarp();
+    }
   }
-  if (!D.gid) {
-    // one graph: a single sum per warp
-    di = warp_sum(di);
-    df = warp_sum(df);
-    if (lane == 0) flush();
-  } else {
-    flush();
-  }
+  flush();
 }
 
 // The team kernels' movers with rows longer than kApplyShort (queued by k_apply, which also
@@ -1408,6 +1470,7 @@ __global__ void __launch_bounds__(512) k_apply_hub(int dslot) {
   const Dev& D = c_dev[dslot];
   Ctrl* C = D.ctrl;
   const uint32_t count = C->apply_items, it = C->it;
+  const bool heavy = heavy_pass(C);
   const bool unit = unit_weights<WINT>(C);
   __shared__ long long shi[32];
   __shared__ double shf[32];
@@ -1423,6 +1486,7 @@ __global__ void __launch_bounds__(512) k_apply_hub(int dslot) {
       atomicAdd(&D.a[nw], kv);
       atomicAdd(&D.a[old], -kv);
     }
+    if (heavy) continue;
     long long di = 0;
     double df = 0.0;
     const uint32_t ps = D.row[v] + piece * kHubPiece;
@@ -1441,6 +1505,132 @@ __global__ void __launch_bounds__(512) k_apply_hub(int dslot) {
     }
     __syncthreads();
   }
+}
+
+// A heavy pass: the internal weight summed afresh and the activity pulled, instead of pushed from
+// the movers. Pushing stores an activity stamp and gathers a (target, community) word for every
+// entry of every mover; here an undirected edge is gathered from one side only (u <= v counts its
+// weight, twice for u < v: the CSR is symmetric), and entries to higher vertices are looked at
+// only while their row has not been found active yet, which the lower ones settle for almost every
+// row of such a pass. The result is the push's: v is active iff a neighbour moved and now sits in
+// another community (the symmetric relation), I is the exact integer sum (integer weights).
+// A warp takes kFullChunk consecutive entries, whatever rows they belong to, 32 rows at a time.
+constexpr uint32_t kFullChunk = 2048;
+constexpr int kFullBatch = 4;
+template <bool WINT>
+__global__ void __launch_bounds__(256) k_apply_full(int dslot) {
+  const Dev& D = c_dev[dslot];
+  using Tr = WTraits<WINT>;
+  using Wt = typename Tr::W;
+  const Wt* __restrict__ w = reinterpret_cast<const Wt*>(D.w);
+  Ctrl* C = D.ctrl;
+  if (!heavy_pass(C)) return;
+  __shared__ uint32_t s_act[8][32];
+  __shared__ unsigned long long s_row[8][32];  // sums per row, where 32 rows are of several graphs
+  unsigned long long* row = s_row[threadIdx.x >> 5];
+  const uint32_t n = C->n, E = D.row[n], it = C->it;  // (the refine view has fewer entries than C->E)
+  const bool unit = unit_weights<WINT>(C);
+  const int lane = threadIdx.x & 31;
+  volatile uint32_t* act = s_act[threadIdx.x >> 5];
+  const uint32_t nwarps = (gridDim.x * blockDim.x) >> 5;
+  uint32_t gcur = 0;  // graph of the running sum
+  unsigned long long si = 0;
+  double sf = 0.0;
+  auto flush = [&]() {
+    add_by_graph<WINT>(D, &GraphState::I_full, gcur, (long long)si, sf);
+    si = 0;
+    sf = 0.0;
+  };
+  const uint32_t nch = (E + kFullChunk - 1) / kFullChunk;
+  for (uint32_t ch = (blockIdx.x * blockDim.x + threadIdx.x) >> 5; ch < nch; ch += nwarps) {
+    const uint32_t c0 = ch * kFullChunk, c1 = min(E, c0 + kFullChunk);
+    // the last row starting at or before c0 (32 probes at a time)
+    uint32_t lo = 0, hi = n;
+    while (hi - lo > 1) {
+      const uint32_t step = (hi - lo + 31u) / 32u;
+      const uint32_t p = lo + (uint32_t)(lane + 1) * step;
+      const unsigned le = __ballot_sync(kFull, p < hi && D.row[p] <= c0);
+      const uint32_t k = __popc(le);
+      hi = min(hi, lo + (k + 1u) * step);
+      lo += k * step;
+    }
+    for (uint32_t vb = lo; vb < n; vb += 32) {
+      const uint32_t cnt = min(32u, n - vb);
+      const uint32_t v = vb + min((uint32_t)lane, cnt - 1u);
+      const bool live = lane < (int)cnt;
+      const uint32_t rs = D.row[v], re = D.row[v + 1];
+      const uint32_t s0 = max(c0, __shfl_sync(kFull, rs, 0));
+      if (s0 >= c1) break;
+      const uint32_t s1 = min(c1, __shfl_sync(kFull, re, (int)cnt - 1));
+      const uint32_t off = live ? rs : kEmpty;
+      const uint32_t post = (uint32_t)(D.cn[v] >> 32);
+      const uint32_t g = D.gid ? D.gid[v] : 0u;
+      const bool on = D.gs[g].phase == kIterating;
+      const uint32_t g0 = __shfl_sync(kFull, g, 0);
+      const bool one = __all_sync(kFull, g == g0);
+      if (one) {
+        if (g0 != gcur) {
+          flush();
+          gcur = g0;
+        }
+        if (!__shfl_sync(kFull, (int)on, 0)) continue;
+      }
+      act[lane] = 0;
+      if (!one) row[lane] = 0ull;
+      __syncwarp();
+      for (uint32_t jb = s0; jb < s1; jb += 32u * kFullBatch) {
+        uint32_t uu[kFullBatch], kk[kFullBatch], po[kFullBatch];
+        unsigned long long x[kFullBatch];
+#pragma unroll
+        for (int q = 0; q < kFullBatch; ++q) {
+          const uint32_t e = jb + (uint32_t)q * 32u + lane;
+          uu[q] = e < s1 ? D.col[e] : kEmpty;
+          int k = 0;  // the entry's row: the last one starting at or before e
+#pragma unroll
+          for (int st = 16; st >= 1; st >>= 1)
+            if (__shfl_sync(kFull, off, k + st) <= e) k += st;
+          kk[q] = (uint32_t)k;
+          po[q] = __shfl_sync(kFull, post, k);
+          if (!one && !__shfl_sync(kFull, (int)on, k)) uu[q] = kEmpty;
+        }
+#pragma unroll
+        for (int q = 0; q < kFullBatch; ++q)
+          x[q] = uu[q] <= vb + kk[q] ? D.cn[uu[q]] : 0ull;  // (kEmpty is above every vertex)
+#pragma unroll
+        for (int q = 0; q < kFullBatch; ++q) {
+          if (uu[q] > vb + kk[q]) continue;
+          const uint32_t pu = (uint32_t)(x[q] >> 32);
+          if (pu == po[q]) {
+            const uint32_t e = jb + (uint32_t)q * 32u + lane, f = uu[q] == vb + kk[q] ? 1u : 2u;
+            if (one) {
+              if (WINT) si += (unsigned long long)f * (unit ? 1u : (uint32_t)w[e]);
+              else sf += (double)f * Tr::w_double(w[e]);
+            } else {
+              if (WINT) atomicAdd(&row[kk[q]], (unsigned long long)f * (unit ? 1u : (uint32_t)w[e]));
+              else atomicAdd(reinterpret_cast<double*>(&row[kk[q]]), (double)f * Tr::w_double(w[e]));
+            }
+          } else if (pu != (uint32_t)x[q]) {
+            act[kk[q]] = 1;
+          }
+        }
+        __syncwarp();
+#pragma unroll
+        for (int q = 0; q < kFullBatch; ++q)
+          x[q] = uu[q] != kEmpty && uu[q] > vb + kk[q] && !act[kk[q]] ? D.cn[uu[q]] : 0ull;
+#pragma unroll
+        for (int q = 0; q < kFullBatch; ++q) {
+          const uint32_t pu = (uint32_t)(x[q] >> 32);  // (not gathered: 0 moved nowhere)
+          if (pu != (uint32_t)x[q] && pu != po[q]) act[kk[q]] = 1;
+        }
+        __syncwarp();
+      }
+      if (live && act[lane]) D.active_it[v] = it + 1;
+      if (!one)
+        add_by_graph<WINT>(D, &GraphState::I_full, g, (long long)row[lane], __longlong_as_double((long long)row[lane]));
+      __syncwarp();
+    }
+  }
+  flush();
 }
 
 __device__ __forceinline__ double modularity_of(double I, double S, double m) {
@@ -1500,9 +1690,14 @@ __device__ __forceinline__ void finalize(const Dev& D, const PassEnd& pe, const 
     __syncthreads();
   }
   uint32_t iterating = 0;
+  const bool heavy = heavy_pass(C);
   for (uint32_t g = threadIdx.x; g < C->G; g += blockDim.x) {
     GraphState* st = &D.gs[g];
     if (st->phase != kIterating) continue;
+    if (heavy) {  // (k_apply_full summed it afresh)
+      st->I = __ldcg(&st->I_full);
+      st->I_full = 0;
+    }
     const unsigned long long ib = __ldcg(&st->I), sb = __ldcg(&st->S);
     const double I = WINT ? (double)ib : __longlong_as_double((long long)ib);
     const double S = WINT ? (double)sb : __longlong_as_double((long long)sb);
@@ -1542,6 +1737,7 @@ __device__ __forceinline__ void finalize(const Dev& D, const PassEnd& pe, const 
     C->loop_continue = tot > 0;
     for (int b = 0; b < kListBins; ++b) C->bin_count[b] = 0;
     C->mover_count = 0;
+    C->mover_entries = 0;
     C->long_movers = 0;
     C->hub_mover_count = 0;
     C->hub_items = 0;
@@ -1701,6 +1897,7 @@ __global__ void k_level_init(int dslot, uint32_t min_deg, uint32_t block_cap) {
     for (int i = threadIdx.x; i < kMaxChunks; i += blockDim.x) C->chunk_any[i] = 0;
   if (blockIdx.x == 0 && threadIdx.x == 0) {
     C->mover_count = 0;
+    C->mover_entries = 0;
     C->long_movers = 0;
     C->hub_mover_count = 0;
     C->hub_items = 0;

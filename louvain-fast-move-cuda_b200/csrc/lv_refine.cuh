@@ -55,6 +55,7 @@ __global__ void k_ref_init(int dslot, uint32_t max_levels) {
     r.phase = on ? kIterating : kFinished;
     r.agg = on ? 1u : 0u;
     r.I = 0ull;
+    r.I_full = 0ull;
     r.S = 0ull;
     r.iters = 0;
     r.total_iters = 0;

@@ -202,7 +202,7 @@ __device__ __forceinline__ void small_gains(SmallRun<WINT, NT>& R, int par, bool
   const Dev& D = R.D;
   const Dev& L = R.L;
   // (the list of movers with long rows lies in `members`, unused during passes)
-  MoverStage mv{s_mov[R.wid], 0u, D.members + R.vb, &R.cnt->long_movers[par]};
+  MoverStage mv{s_mov[R.wid], 0u, D.members + R.vb, &R.cnt->long_movers[par], nullptr, 0u};
   uint32_t nl_[kSmallLists];
 #pragma unroll
   for (int q = 0; q < kSmallLists; ++q) nl_[q] = R.cnt->list[par][q];
@@ -234,7 +234,7 @@ __device__ __forceinline__ void small_gains(SmallRun<WINT, NT>& R, int par, bool
     if (R.wid == 0) {
       best = team_max<32>(R.lane < (NT / 32) ? red[R.lane] : 0ull, kFull);
       const uint32_t c = key_comm(best, lowest);
-      mv.add(D, R.lane == 0 && best && c != x.cv && (!fast || v <= c), v, x.cv, c);
+      mv.add(D, R.lane == 0 && best && c != x.cv && (!fast || v <= c), v, x.cv, c, 0u);
     }
     __syncthreads();
   }
@@ -267,7 +267,7 @@ __device__ __forceinline__ void small_gains(SmallRun<WINT, NT>& R, int par, bool
       best = team_max<32>(best, kFull);
       __syncwarp();  // the listed slots are empty again before the next row inserts
       const uint32_t c = key_comm(best, lowest);
-      mv.add(D, R.lane == 0 && best && c != x.cv, v, x.cv, c);
+      mv.add(D, R.lane == 0 && best && c != x.cv, v, x.cv, c, 0u);
     }
     mv.switch_to(D.movers + R.vb, &R.cnt->movers[par]);
     w0 = (w0 + R.nw - nl_[2] % R.nw) % R.nw;
@@ -301,7 +301,7 @@ __device__ __forceinline__ void small_apply(SmallRun<WINT, NT>& R, uint32_t coun
       atomicAdd(&D.a[nw], kv);
       atomicAdd(&D.a[old], -kv);
     }
-    apply_rows<WINT, kSmallApply<NT>>(R.L, rs, len, old, nw, it, R.unit, [&](uint32_t, int f, double wt, uint32_t wi) {
+    apply_rows<WINT, kSmallApply<NT>>(R.L, rs, len, old, nw, it, R.unit, [&](int, int f, double wt, uint32_t wi) {
       if (WINT) di += (long long)f * (long long)wi;
       else df += (double)f * wt;
     });
