@@ -26,6 +26,7 @@
 #include "lv_kernels.cuh"
 #include "lv_refine.cuh"
 #include "lv_small.cuh"
+#include "lv_stage.cuh"
 
 namespace lv {
 
@@ -49,14 +50,46 @@ static bool g_slot_used[kMaxDevSlots] = {};
 struct DevSlot {
   int id = -1;                  // index into c_dev
   const void* owner = nullptr;  // the run whose Dev is in c_dev[id]
-  cudaGraph_t graph = nullptr;
-  cudaGraphExec_t exec = nullptr;
-  GraphKey key{};
-  GraphCtl gc{};
-  int64_t k_pass = 0, k_level = 0, k_contract = 0, k_ok = 0, k_final = 0;  // kernels per segment
+  // The level loops captured against this slot, most recently used first. A slot sees more than one
+  // configuration -- single graphs and packed batches, with and without the walk of heavy passes
+  // -- and an instantiation costs some milliseconds, more than most runs.
+  struct Loop {
+    cudaGraph_t graph = nullptr;
+    cudaGraphExec_t exec = nullptr;
+    GraphKey key{};
+    GraphCtl gc{};
+    int64_t k_pass = 0, k_level = 0, k_contract = 0, k_ok = 0, k_final = 0;  // kernels per segment
+    void release() {
+      if (exec) cudaGraphExecDestroy(exec);
+      if (graph) cudaGraphDestroy(graph);
+      exec = nullptr;
+      graph = nullptr;
+    }
+  };
+  static constexpr size_t kMaxLoops = 6;
+  std::vector<Loop> loops;
   cudaStream_t cs[3] = {nullptr, nullptr, nullptr};  // capture streams of nested bodies
   cudaStream_t bs[5] = {};                           // and of the branches inside a body
   cudaEvent_t be[6] = {};                            // fork, and the end of each branch
+
+  // The loop captured for `key` moved to the front, or nullptr. (A run waits for its launches before
+  // it ends, so no loop is in flight when another is looked up.)
+  Loop* find(const GraphKey& key) {
+    for (size_t i = 0; i < loops.size(); ++i)
+      if (std::memcmp(&loops[i].key, &key, sizeof(key)) == 0) {
+        std::rotate(loops.begin(), loops.begin() + (long)i, loops.begin() + (long)i + 1);
+        return &loops[0];
+      }
+    return nullptr;
+  }
+  Loop* add(const Loop& l) {
+    if (loops.size() >= kMaxLoops) {
+      loops.back().release();
+      loops.pop_back();
+    }
+    loops.insert(loops.begin(), l);
+    return &loops[0];
+  }
 
   cudaError_t create() {
     std::lock_guard<std::mutex> lk(g_slot_mu);
@@ -68,14 +101,9 @@ struct DevSlot {
       }
     return cudaErrorMemoryAllocation;
   }
-  void release_graph() {
-    if (exec) cudaGraphExecDestroy(exec);
-    if (graph) cudaGraphDestroy(graph);
-    exec = nullptr;
-    graph = nullptr;
-  }
   void destroy() {
-    release_graph();
+    for (Loop& l : loops) l.release();
+    loops.clear();
     for (auto& x : cs)
       if (x) cudaStreamDestroy(x);
     for (auto& x : bs)
@@ -108,6 +136,7 @@ struct lv_context {
   std::mutex pool_mu;                 // runs of the serving loop allocate concurrently
   uint32_t* pinned = nullptr;         // small host readbacks
   cudaEvent_t ev[8] = {};
+  lv::Stager stager{4};               // host copies of calls on `stream`
 
   // A pooled block of at least `bytes` (and not wastefully larger), or nullptr; *got = its size.
   void* take(size_t bytes, size_t* got) {
@@ -277,6 +306,7 @@ class Run {
   cudaEvent_t ev[6];
   std::vector<Block> arena_blocks;
   DevSlot* slot = nullptr;
+  Stager* stage = nullptr;  // host copies on `st`
   int Dd = -1;           // the slot whose c_dev entry kernels read D from
   bool dev_dirty = true;
 
@@ -294,8 +324,9 @@ class Run {
   // context lock); otherwise a private stream, as the serving loop runs several at once, with
   // the caller's 64-byte pinned readback buffer (or one of the run's own if none is given).
   explicit Run(lv_context* c, cudaStream_t stream = nullptr, uint32_t* pinned_buf = nullptr,
-               DevSlot* dslot = nullptr)
+               DevSlot* dslot = nullptr, Stager* stager = nullptr)
       : ctx(c), cfg(c->cfg) {
+    stage = stager ? stager : &c->stager;
     for (auto& e : ev) e = nullptr;
     st = stream ? stream : c->stream;
     pinned = stream ? pinned_buf : c->pinned;
@@ -438,9 +469,9 @@ class Run {
     // (k_prep writes the engine's copy of the columns and weights as it validates them)
     PrepIn in{reinterpret_cast<const long long*>(row_ptr), reinterpret_cast<const uint32_t*>(col), w, nullptr, 0};
     if (in_mem != LV_MEM_DEVICE) {
-      if (w) LV_CUDA(cudaMemcpyAsync(D.w, w, (size_t)E * 4, cudaMemcpyHostToDevice, st));
-      LV_CUDA(cudaMemcpyAsync(D.col, col, (size_t)E * 4, cudaMemcpyHostToDevice, st));
-      LV_CUDA(cudaMemcpyAsync(row64(), row_ptr, (size_t)(n + 1) * 8, cudaMemcpyHostToDevice, st));
+      if (w) LV_CUDA(stage->to_device(D.w, w, (size_t)E * 4, st));
+      LV_CUDA(stage->to_device(D.col, col, (size_t)E * 4, st));
+      LV_CUDA(stage->to_device(row64(), row_ptr, (size_t)(n + 1) * 8, st));
       in = uploaded(w != nullptr);
     }
     choose_weight_mode(in.wf);
@@ -527,10 +558,9 @@ class Run {
     long long* r64 = row64();
     for (size_t g = 0; g < ps.size(); ++g) {
       if (weighted)
-        LV_CUDA(cudaMemcpyAsync(reinterpret_cast<float*>(D.w) + eo[g], ps[g].w, (size_t)ps[g].E * 4,
-                                cudaMemcpyHostToDevice, st));
-      LV_CUDA(cudaMemcpyAsync(D.col + eo[g], ps[g].col, (size_t)ps[g].E * 4, cudaMemcpyHostToDevice, st));
-      LV_CUDA(cudaMemcpyAsync(r64 + ho[g], ps[g].row, (size_t)ps[g].n * 8, cudaMemcpyHostToDevice, st));
+        LV_CUDA(stage->to_device(reinterpret_cast<float*>(D.w) + eo[g], ps[g].w, (size_t)ps[g].E * 4, st));
+      LV_CUDA(stage->to_device(D.col + eo[g], ps[g].col, (size_t)ps[g].E * 4, st));
+      LV_CUDA(stage->to_device(r64 + ho[g], ps[g].row, (size_t)ps[g].n * 8, st));
     }
     long long* doffs = dalloc<long long>(ctx, owned, 2 * ((size_t)G + 1), st);
     LV_CUDA(cudaMemcpyAsync(doffs, ho.data(), (G + 1) * 8, cudaMemcpyHostToDevice, st));
@@ -803,7 +833,7 @@ class Run {
   }
 
   void ensure_arena(uint64_t need_slots) {
-    if (need_slots <= arena_slots) return;
+    if (need_slots <= arena_slots && arena_slots > 0) return;
     if (need_slots >= 0xFFFFFFFFull) throw Fail{LV_ERR_RANGE, "hub hash-table arena beyond 2^32 slots"};
     if (!arena_blocks.empty()) {
       sync();
@@ -813,10 +843,37 @@ class Run {
       D.arena_vals = nullptr;
     }
     uint64_t slots = std::max<uint64_t>(need_slots + need_slots / 4, 1 << 16);
+    // The first allocation also covers what the aggregations of most graphs will want (0.1-1.2 slots
+    // per entry on the benchmark graphs with whole-number weights, 1.7 with fp32 ones), so that a captured run
+    // does not stop for a larger arena in its first aggregation (0.5 ms a stop: a sixth of a run
+    // of 300,000 vertices). Bounded, and only if the memory is there.
+    const uint64_t guess = std::min<uint64_t>(2ull * E, kArenaGuess);
+    if (arena_slots == 0 && slots < guess && try_arena(guess)) return;
     slots = std::min<uint64_t>(slots, 0xFFFFFFFEull);
-    D.arena_keys = dalloc<uint32_t>(ctx, arena_blocks, slots, st);
+    if (!wint) D.arena_keys = dalloc<uint32_t>(ctx, arena_blocks, slots, st);  // packed slots otherwise
     D.arena_vals = dalloc<unsigned long long>(ctx, arena_blocks, slots, st);
     D.hub_owner = dalloc<uint32_t>(ctx, arena_blocks, slots / kHubChunk + 1, st);
+    set_arena(slots);
+  }
+  static constexpr uint64_t kArenaGuess = 48ull << 20;  // slots: 384 MB of packed ones
+  bool try_arena(uint64_t slots) {
+    try {
+      if (!wint) D.arena_keys = dalloc<uint32_t>(ctx, arena_blocks, slots, st);
+      D.arena_vals = dalloc<unsigned long long>(ctx, arena_blocks, slots, st);
+      D.hub_owner = dalloc<uint32_t>(ctx, arena_blocks, slots / kHubChunk + 1, st);
+    } catch (const Fail&) {
+      cudaGetLastError();
+      sync();
+      for (const Block& b : arena_blocks) ctx->give(b.p, b.bytes);
+      arena_blocks.clear();
+      D.arena_keys = nullptr;
+      D.arena_vals = nullptr;
+      return false;
+    }
+    set_arena(slots);
+    return true;
+  }
+  void set_arena(uint64_t slots) {
     arena_slots = slots;
     dev_dirty = true;
     bind();
@@ -1189,8 +1246,8 @@ class Run {
   }
 
   template <bool WI>
-  void build_graph() {
-    slot->release_graph();
+  DevSlot::Loop* build_graph() {
+    DevSlot::Loop loop;
     for (auto& x : slot->cs)
       if (!x) LV_CUDA(cudaStreamCreateWithFlags(&x, cudaStreamNonBlocking));
     for (auto& x : slot->bs)
@@ -1200,7 +1257,7 @@ class Run {
     cudaStream_t* cs = slot->cs;
     cudaGraph_t graph = nullptr;
     LV_CUDA(cudaGraphCreate(&graph, 0));
-    slot->graph = graph;
+    loop.graph = graph;
     // each handle belongs to the graph that holds its conditional node; the level and pass loops'
     // handles have a launch default (a launch begins at a level start), later values are set by the
     // kernel before the node (pass: also by the level start that ends the level's body)
@@ -1228,40 +1285,41 @@ class Run {
         cudaGraph_t* pb = add_cond(st, hP, cudaGraphCondTypeWhile, 1);
         a = launches;
         capture_into(pb[0], cs[1], [&] { launch_pass<WI>(); });
-        slot->k_pass = launches - a;
+        loop.k_pass = launches - a;
         b = launches;
         agg_prefix<WI>(-1);
         cudaGraph_t* cb = add_cond(st, hC, cudaGraphCondTypeIf, 2);
-        slot->k_level = launches - b;
+        loop.k_level = launches - b;
         LV_CUDA(cudaGraphConditionalHandleCreate(&hO, cb[0], 0, 0));
         gc.ok = hO;
         c = launches;
         capture_into(cb[0], cs[1], [&] {
           agg_contract_a<WI>();
           cudaGraph_t* ob = add_cond(st, hO, cudaGraphCondTypeIf, 1);
-          slot->k_contract = launches - c;
+          loop.k_contract = launches - c;
           d = launches;
           capture_into(ob[0], cs[2], [&] {
             agg_contract_b<WI>();
             level_start_kernels();
           });
-          slot->k_ok = launches - d;
+          loop.k_ok = launches - d;
         });
         e = launches;
         capture_into(cb[1], cs[1], [&] { agg_final(); });
-        slot->k_final = launches - e;
+        loop.k_final = launches - e;
       });
-      LV_CUDA(cudaGraphInstantiate(&slot->exec, graph, 0));
+      LV_CUDA(cudaGraphInstantiate(&loop.exec, graph, 0));
     } catch (...) {
       gc.on = 0;
       launches = l0;
-      slot->release_graph();
+      loop.release();
       throw;
     }
-    slot->gc = gc;
-    slot->key = graph_key();
+    loop.gc = gc;
+    loop.key = graph_key();
     gc.on = 0;
     launches = l0;
+    return slot->add(loop);
   }
 
   // Waits for the stream, giving up (with an error; the work may still be running) after
@@ -1302,21 +1360,21 @@ class Run {
     bool reset_abort = false;
     // the launch after a stop begins at a level start, which is where the host left the run
     for (int launch = 0;; ++launch) {
-      const GraphKey key = graph_key();
-      if (!slot->exec || std::memcmp(&key, &slot->key, sizeof(key)) != 0) build_graph<WI>();
+      DevSlot::Loop* loop = slot->find(graph_key());
+      if (!loop) loop = build_graph<WI>();
       bind();
       if (reset_abort) write_ctrl_u32(offsetof(Ctrl, abort), 0);
-      LV_CUDA(cudaGraphLaunch(slot->exec, st));
+      LV_CUDA(cudaGraphLaunch(loop->exec, st));
       ++graph_launches;
       wait_bounded(600.0);
       const LaunchEnd end = read_ctrl<LaunchEnd>(offsetof(Ctrl, abort));
       // kernels that ran: the level body entry + aggregation prefix per level body, the pass
       // body per pass, and each branch as often as it was taken (the gate counters)
-      launches += (int64_t)(end.seg.passes - prev.passes) * slot->k_pass +
-                  (int64_t)(end.seg.aggs - prev.aggs) * slot->k_level +
-                  (int64_t)(end.seg.contract - prev.contract) * slot->k_contract +
-                  (int64_t)(end.seg.contract_ok - prev.contract_ok) * slot->k_ok +
-                  (int64_t)(end.seg.final_ - prev.final_) * slot->k_final;
+      launches += (int64_t)(end.seg.passes - prev.passes) * loop->k_pass +
+                  (int64_t)(end.seg.aggs - prev.aggs) * loop->k_level +
+                  (int64_t)(end.seg.contract - prev.contract) * loop->k_contract +
+                  (int64_t)(end.seg.contract_ok - prev.contract_ok) * loop->k_ok +
+                  (int64_t)(end.seg.final_ - prev.final_) * loop->k_final;
       check_device_errors();
       if (end.abort == 0) break;
       ensure_arena(end.abort_need);
@@ -1508,6 +1566,7 @@ lv_status lv_destroy(lv_context* ctx) {
   ctx->slot.destroy();
   ctx->rslot.destroy();
   ctx->drain_pool();
+  ctx->stager.release();
   if (ctx->pinned) cudaFreeHost(ctx->pinned);
   for (auto& ev : ctx->ev)
     if (ev) cudaEventDestroy(ev);
@@ -1733,8 +1792,10 @@ static lv_status run_common(lv_context* ctx, uint32_t G, const int64_t* offs, in
     r.init(G, offs, n, row_ptr, col, w, in_mem);
     LV_CUDA(cudaEventRecord(t1, ctx->stream));
     r.louvain();
-    LV_CUDA(cudaMemcpyAsync(out_comm, r.D.out, (size_t)r.n0 * 4,
-                            out_mem == LV_MEM_DEVICE ? cudaMemcpyDeviceToDevice : cudaMemcpyDeviceToHost, ctx->stream));
+    if (out_mem == LV_MEM_DEVICE)
+      LV_CUDA(cudaMemcpyAsync(out_comm, r.D.out, (size_t)r.n0 * 4, cudaMemcpyDeviceToDevice, ctx->stream));
+    else
+      LV_CUDA(ctx->stager.to_host(out_comm, r.D.out, (size_t)r.n0 * 4, ctx->stream));
     std::vector<lv::GraphState> hs(G);
     LV_CUDA(cudaMemcpyAsync(hs.data(), r.D.gs, sizeof(lv::GraphState) * G, cudaMemcpyDeviceToHost, ctx->stream));
     LV_CUDA(cudaEventRecord(t2, ctx->stream));

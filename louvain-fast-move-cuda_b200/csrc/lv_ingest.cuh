@@ -514,27 +514,44 @@ struct lv_ingest {
   int64_t n = 0, n_links = 0, E = 0, min_id = 0;
   int64_t* row_ptr = nullptr;  // device, n + 1
   int32_t* col = nullptr;      // device, E
+  size_t row_bytes = 0, col_bytes = 0;  // their pool blocks
 };
 
 namespace lv {
 
-// A device allocation of a single temporary buffer (plain cudaMalloc/cudaFree: ingest runs
-// once per graph, outside the engine's pool).
+// A buffer of the context's pool, on the context's stream (an ingest uses some twenty; with a
+// cudaMalloc and a synchronising cudaFree for each they cost more than the kernels). It goes back to
+// the pool, whose blocks any stream may take next, so reset() and the destructor may only run once the
+// work on it is done: ingest_run synchronises before it leaves, on errors too.
 struct DevBuf {
+  lv_context* ctx;
   void* p = nullptr;
-  DevBuf() = default;
+  size_t bytes = 0;
+  explicit DevBuf(lv_context* c) : ctx(c) {}
   DevBuf(const DevBuf&) = delete;
   DevBuf& operator=(const DevBuf&) = delete;
   ~DevBuf() { reset(); }
   void reset() {
-    if (p) cudaFree(p);
+    if (!p) return;
+    cudaStreamSynchronize(ctx->stream);
+    ctx->give(p, bytes);
     p = nullptr;
   }
   template <class T>
   T* alloc(size_t count) {
     reset();
-    LV_CUDA(cudaMalloc(&p, std::max<size_t>(count, 1) * sizeof(T)));
+    std::vector<Block> b;
+    dalloc<T>(ctx, b, count, ctx->stream);
+    p = b[0].p;
+    bytes = b[0].bytes;
     return reinterpret_cast<T*>(p);
+  }
+  // Hands the block over (the caller gives it back to the pool).
+  void* release(size_t* n) {
+    void* q = p;
+    *n = bytes;
+    p = nullptr;
+    return q;
   }
 };
 
@@ -582,19 +599,19 @@ static void ingest_run(lv_context* ctx, const char* text_in, int64_t len, int32_
   }
   const uint64_t L = (uint64_t)(len - start);
   if (L == 0) throw Fail{LV_ERR_INPUT, "Error during parsing: no node found"};
-  DevBuf btext;
+  DevBuf btext(ctx);
   const unsigned char* text;
   if (in_mem == LV_MEM_DEVICE) {
     text = reinterpret_cast<const unsigned char*>(text_in) + start;
   } else {
     unsigned char* t = btext.alloc<unsigned char>(L);
-    LV_CUDA(cudaMemcpyAsync(t, text_in + start, L, cudaMemcpyHostToDevice, st));
+    LV_CUDA(ctx->stager.to_device(t, text_in + start, L, st));
     text = t;
   }
   // token starts
   const uint64_t nchunks = (L + kIngestChunk - 1) / kIngestChunk;
   if (nchunks >= 0xFFFFFFFFull) throw Fail{LV_ERR_RANGE, "edge-list text too large"};
-  DevBuf bcnt, boff, btmp;
+  DevBuf bcnt(ctx), boff(ctx), btmp(ctx), btmp2(ctx), btmp3(ctx);  // (one scan scratch per scan in flight)
   uint32_t* cnt = bcnt.alloc<uint32_t>(nchunks + 1);
   uint32_t* off = boff.alloc<uint32_t>(nchunks + 1);
   k_tok_count<<<grid, 256, 0, st>>>(text, L, cnt, nchunks);
@@ -605,7 +622,7 @@ static void ingest_run(lv_context* ctx, const char* text_in, int64_t len, int32_
   LV_CUDA(cudaStreamSynchronize(st));
   const uint64_t ntok = ntok32;
   if (ntok < 2) throw Fail{LV_ERR_INPUT, "Error during parsing: no node found"};
-  DevBuf bpos, bval, bbad;
+  DevBuf bpos(ctx), bval(ctx), bbad(ctx);
   uint64_t* pos = bpos.alloc<uint64_t>(ntok);
   k_tok_place<<<grid, 256, 0, st>>>(text, L, off, nchunks, pos);
   int32_t* val = bval.alloc<int32_t>(ntok);
@@ -623,7 +640,7 @@ static void ingest_run(lv_context* ctx, const char* text_in, int64_t len, int32_
   boff.reset();
   bpos.reset();
   // id range
-  DevBuf bmm;
+  DevBuf bmm(ctx);
   int* mm = bmm.alloc<int>(2);
   const int init[2] = {INT32_MAX, INT32_MIN};
   LV_CUDA(cudaMemcpyAsync(mm, init, 8, cudaMemcpyHostToDevice, st));
@@ -636,7 +653,7 @@ static void ingest_run(lv_context* ctx, const char* text_in, int64_t len, int32_
   if (range > 2 * npairs) throw Fail{LV_ERR_INPUT, "vertex IDs must be contiguous (the reference indexes by id - min_id)"};
   if (range >= 0x7FFFFFFFull) throw Fail{LV_ERR_RANGE, "more than 2^31-1 vertices"};
   // entries per row (both ends of every pair); every id must have one
-  DevBuf bcntr, bstart, bcount;
+  DevBuf bcntr(ctx), bstart(ctx), bcount(ctx);
   uint32_t* cntr = bcntr.alloc<uint32_t>(range + 1);
   LV_CUDA(cudaMemsetAsync(cntr, 0, (range + 1) * 4, st));
   k_pair_count<<<grid, 256, 0, st>>>(val, npairs, hmm[0], cntr);
@@ -649,15 +666,14 @@ static void ingest_run(lv_context* ctx, const char* text_in, int64_t len, int32_
   if (nn != range) throw Fail{LV_ERR_INPUT, "vertex IDs must be contiguous (the reference indexes by id - min_id)"};
   // rows placed by a scan of the counts, filled by the pairs
   uint32_t* rstart = bstart.alloc<uint32_t>(range + 1);
-  iscan<uint32_t>(ctx, st, btmp, cntr, range + 1, rstart);
-  DevBuf bcur, bbuf;
+  iscan<uint32_t>(ctx, st, btmp2, cntr, range + 1, rstart);
+  DevBuf bcur(ctx), bbuf(ctx);
   uint32_t* cursor = bcur.alloc<uint32_t>(range);
   LV_CUDA(cudaMemcpyAsync(cursor, rstart, range * 4, cudaMemcpyDeviceToDevice, st));
   uint32_t* buf = bbuf.alloc<uint32_t>(2 * npairs);
   k_pair_scatter<<<grid, 256, 0, st>>>(val, npairs, hmm[0], cursor, buf);
-  bval.reset();
   // each row sorted and deduplicated in place: warp, block or bitmap by its length
-  DevBuf bmid, bbig, bmid8, bmid32, bcls, bulen;
+  DevBuf bmid(ctx), bbig(ctx), bmid8(ctx), bmid32(ctx), bcls(ctx), bulen(ctx);
   uint32_t* mid = bmid.alloc<uint32_t>(range);
   uint32_t* big = bbig.alloc<uint32_t>(range);
   uint32_t* mid8 = bmid8.alloc<uint32_t>(range);
@@ -674,7 +690,7 @@ static void ingest_run(lv_context* ctx, const char* text_in, int64_t len, int32_
   k_rows_warpn<32><<<grid, 256, 0, st>>>(rstart, cntr, mid32, cls + 3, buf, ulen);
   k_rows_block<<<ctx->sms * 2, kIngestBlockNT, 0, st>>>(rstart, cntr, mid, cls, buf, ulen);
   LV_CUDA(cudaStreamSynchronize(st));
-  DevBuf bbm;
+  DevBuf bbm(ctx);
   if (hcls[1] > 0) {
     // a bitmap per block, each as wide as the whole id range; blocks limited to 1 GiB of them
     const uint64_t bmw = (range >> 5) + 1;
@@ -684,31 +700,19 @@ static void ingest_run(lv_context* ctx, const char* text_in, int64_t len, int32_
     k_rows_bitmap<<<(unsigned)nb, kIngestBlockNT, 0, st>>>(rstart, cntr, big, cls, bitmaps, bmw, buf, ulen);
   }
   // the dense CSR: row offsets from a scan of the distinct lengths
-  int64_t* row_ptr = nullptr;
-  int32_t* col = nullptr;
-  LV_CUDA(cudaMalloc(&row_ptr, (range + 1) * sizeof(int64_t)));
-  iscan<int64_t>(ctx, st, btmp, ulen, range + 1, row_ptr);
+  DevBuf brow(ctx), bcol(ctx);
+  int64_t* row_ptr = brow.alloc<int64_t>(range + 1);
+  iscan<int64_t>(ctx, st, btmp3, ulen, range + 1, row_ptr);
   int64_t ne64 = 0;
   LV_CUDA(cudaMemcpyAsync(&ne64, row_ptr + range, 8, cudaMemcpyDeviceToHost, st));
-  const cudaError_t e0 = cudaStreamSynchronize(st);
-  if (e0 != cudaSuccess) {
-    cudaFree(row_ptr);
-    throw Fail{LV_ERR_CUDA, std::string("ingest: ") + cudaGetErrorString(e0)};
-  }
+  LV_CUDA(cudaStreamSynchronize(st));
   const uint64_t ne = (uint64_t)ne64;
   const int64_t nl = ne64 / 2;  // each distinct pair is two entries (a self-loop: its id twice)
-  if (cudaMalloc(&col, std::max<uint64_t>(ne, 1) * sizeof(int32_t)) != cudaSuccess) {
-    cudaFree(row_ptr);
-    cudaGetLastError();
-    throw Fail{LV_ERR_NOMEM, "cudaMalloc of the CSR destinations failed"};
-  }
+  int32_t* col = bcol.alloc<int32_t>(ne);
   k_rows_copy<<<grid, 256, 0, st>>>(rstart, row_ptr, (uint32_t)range, ne, buf, col);
-  const cudaError_t e = cudaStreamSynchronize(st);
-  if (e != cudaSuccess) {
-    cudaFree(row_ptr);
-    cudaFree(col);
-    throw Fail{LV_ERR_CUDA, std::string("ingest: ") + cudaGetErrorString(e)};
-  }
+  LV_CUDA(cudaStreamSynchronize(st));
+  brow.release(&out->row_bytes);
+  bcol.release(&out->col_bytes);
   out->ctx = ctx;
   out->n = (int64_t)range;
   out->n_links = nl;
@@ -748,14 +752,20 @@ lv_status lv_ingest_info(const lv_ingest* g, int64_t* n_nodes, int64_t* n_links,
 
 lv_status lv_ingest_copy_csr(const lv_ingest* g, int64_t* row_ptr, int32_t* col, int32_t out_mem) {
   if (!g || !row_ptr || !col) return LV_ERR_ARGUMENT;
-  const cudaMemcpyKind k = out_mem == LV_MEM_DEVICE ? cudaMemcpyDeviceToDevice : cudaMemcpyDeviceToHost;
-  cudaSetDevice(g->ctx->device);
-  if (cudaMemcpy(row_ptr, g->row_ptr, (size_t)(g->n + 1) * 8, k) != cudaSuccess ||
-      cudaMemcpy(col, g->col, (size_t)g->E * 4, k) != cudaSuccess) {
-    cudaGetLastError();
-    return LV_ERR_CUDA;
-  }
-  return LV_OK;
+  lv_context* ctx = g->ctx;
+  std::lock_guard<std::mutex> lk(ctx->mu);
+  return guarded(ctx, [&] {
+    cudaSetDevice(ctx->device);
+    const size_t rb = (size_t)(g->n + 1) * 8, cb = (size_t)g->E * 4;
+    if (out_mem == LV_MEM_DEVICE) {
+      LV_CUDA(cudaMemcpyAsync(row_ptr, g->row_ptr, rb, cudaMemcpyDeviceToDevice, ctx->stream));
+      LV_CUDA(cudaMemcpyAsync(col, g->col, cb, cudaMemcpyDeviceToDevice, ctx->stream));
+    } else {
+      LV_CUDA(ctx->stager.to_host(row_ptr, g->row_ptr, rb, ctx->stream));
+      LV_CUDA(ctx->stager.to_host(col, g->col, cb, ctx->stream));
+    }
+    LV_CUDA(cudaStreamSynchronize(ctx->stream));
+  });
 }
 
 lv_status lv_ingest_run(lv_ingest* g, int32_t* out_comm, int32_t out_mem, double* out_modularity, lv_stats* stats) {
@@ -766,9 +776,9 @@ lv_status lv_ingest_run(lv_ingest* g, int32_t* out_comm, int32_t out_mem, double
 
 lv_status lv_ingest_destroy(lv_ingest* g) {
   if (!g) return LV_ERR_ARGUMENT;
-  if (g->ctx) cudaSetDevice(g->ctx->device);
-  if (g->row_ptr) cudaFree(g->row_ptr);
-  if (g->col) cudaFree(g->col);
+  // (every call that reads the CSR waits for its work)
+  if (g->row_ptr) g->ctx->give(g->row_ptr, g->row_bytes);
+  if (g->col) g->ctx->give(g->col, g->col_bytes);
   delete g;
   return LV_OK;
 }

@@ -62,6 +62,7 @@ struct lv_server {
   std::vector<std::thread> workers;
   std::vector<cudaStream_t> streams;
   std::vector<uint32_t*> pinned;  // per slot: 64-byte readback buffer
+  std::vector<std::unique_ptr<lv::Stager>> stagers;  // per slot: pinned buffers of its host copies
   std::vector<std::unique_ptr<lv::DevSlot>> dslots;  // per slot: Dev buffer and captured graph
 
   // Continuous batching: a free slot takes the request at the head of the queue and, when
@@ -137,7 +138,7 @@ struct lv_server {
 
   void run_batch(const std::vector<lv::Request*>& batch, int slot) {
     try {
-      lv::Run run(ctx, streams[slot], pinned[slot], dslots[slot].get());
+      lv::Run run(ctx, streams[slot], pinned[slot], dslots[slot].get(), stagers[slot].get());
       run.small_ok = true;
       std::vector<lv::Run::Piece> ps;
       ps.reserve(batch.size());
@@ -152,7 +153,7 @@ struct lv_server {
       int64_t vb = 0;
       for (lv::Request* r : batch) {
         r->out.resize((size_t)r->n);
-        LV_CUDA(cudaMemcpyAsync(r->out.data(), run.D.out + vb, (size_t)r->n * 4, cudaMemcpyDeviceToHost, run.st));
+        LV_CUDA(run.stage->to_host(r->out.data(), run.D.out + vb, (size_t)r->n * 4, run.st));
         vb += r->n;
       }
       LV_CUDA(cudaMemcpyAsync(gs.data(), run.D.gs, sizeof(lv::GraphState) * batch.size(),
@@ -209,6 +210,7 @@ lv_status lv_server_create(lv_context* ctx, int64_t budget_bytes, int32_t max_sl
       return LV_ERR_CUDA;
     }
     s->pinned.push_back(pb);
+    s->stagers.push_back(std::make_unique<lv::Stager>(1));  // the slots copy side by side
     auto ds = std::make_unique<lv::DevSlot>();
     if (ds->create() != cudaSuccess) {
       for (cudaStream_t x : s->streams) cudaStreamDestroy(x);
