@@ -460,40 +460,12 @@ __device__ __forceinline__ unsigned long long team_max(unsigned long long x, uns
   return x;
 }
 
-// Load-balanced walk over the rows of up to 32 vertices held one per lane: calls
-// f(entry index, pa, pb) for every entry of every row -- pa/pb being the payload of the lane
-// that owns the row -- with all 32 lanes busy however the row lengths are spread. Lane i holds
-// (rs_i, len_i, pa_i, pb_i); every lane of the warp must call it.
-template <class F>
-__device__ __forceinline__ void warp_expand_rows(uint32_t rs, uint32_t len, uint32_t pa, uint32_t pb,
-                                                 F&& f) {
-  const int lane = threadIdx.x & 31;
-  uint32_t incl = len;
-#pragma unroll
-  for (int o = 1; o < 32; o <<= 1) {
-    const uint32_t y = __shfl_up_sync(kFull, incl, o);
-    if (lane >= o) incl += y;
-  }
-  const uint32_t total = __shfl_sync(kFull, incl, 31);
-  const uint32_t excl = incl - len;
-  for (uint32_t jb = 0; jb < total; jb += 32) {
-    const uint32_t j = jb + lane;
-    // owner lane: the last lane whose exclusive offset is <= j
-    int k = 0;
-#pragma unroll
-    for (int step = 16; step >= 1; step >>= 1) {
-      const uint32_t ex = __shfl_sync(kFull, excl, k + step);
-      if (ex <= j) k += step;
-    }
-    const uint32_t base = __shfl_sync(kFull, rs, k) - __shfl_sync(kFull, excl, k);
-    const uint32_t a = __shfl_sync(kFull, pa, k), b = __shfl_sync(kFull, pb, k);
-    if (j < total) f(base + j, a, b);
-  }
-}
-
-// warp_expand_rows that calls f(entry index, valid) on every lane in every step (lanes past
-// the last entry with valid = false), so that f may use warp-wide votes.
-template <class F>
+// Load-balanced walk over the rows of up to 32 vertices held one per lane (row start rs, length len),
+// with all 32 lanes busy however the row lengths are spread; every lane of the warp must call it.
+// In steps of NB entries per lane: f(entry indexes, valid) on every lane in every step
+// (lanes past the last entry with valid = false), so that f may use warp-wide votes and has the
+// loads of NB entries to issue before it uses any.
+template <int NB, class F>
 __device__ __forceinline__ void warp_expand_rows_all(uint32_t rs, uint32_t len, F&& f) {
   const int lane = threadIdx.x & 31;
   uint32_t incl = len;
@@ -504,23 +476,28 @@ __device__ __forceinline__ void warp_expand_rows_all(uint32_t rs, uint32_t len, 
   }
   const uint32_t total = __shfl_sync(kFull, incl, 31);
   const uint32_t excl = incl - len;
-  for (uint32_t jb = 0; jb < total; jb += 32) {
-    const uint32_t j = jb + lane;
-    int k = 0;
+  for (uint32_t jb = 0; jb < total; jb += 32u * NB) {
+    uint32_t ee[NB];
+    bool ok[NB];
 #pragma unroll
-    for (int step = 16; step >= 1; step >>= 1) {
-      const uint32_t ex = __shfl_sync(kFull, excl, k + step);
-      if (ex <= j) k += step;
+    for (int q = 0; q < NB; ++q) {
+      const uint32_t j = jb + (uint32_t)q * 32u + lane;
+      int k = 0;
+#pragma unroll
+      for (int step = 16; step >= 1; step >>= 1) {
+        const uint32_t ex = __shfl_sync(kFull, excl, k + step);
+        if (ex <= j) k += step;
+      }
+      ee[q] = __shfl_sync(kFull, rs, k) - __shfl_sync(kFull, excl, k) + j;
+      ok[q] = j < total;
     }
-    const uint32_t base = __shfl_sync(kFull, rs, k) - __shfl_sync(kFull, excl, k);
-    f(base + j, j < total);
+    f(ee, ok);
   }
 }
 
-// The same with three payload words per row: f(entry index, pa, pb, pc).
-template <class F>
-__device__ __forceinline__ void warp_expand_rows3(uint32_t rs, uint32_t len, uint32_t pa, uint32_t pb,
-                                                  uint32_t pc, F&& f) {
+// The same, telling the lane that owns each entry's row: f(entry indexes, owner lanes, valid).
+template <int NB, class F>
+__device__ __forceinline__ void warp_expand_rows_owner(uint32_t rs, uint32_t len, F&& f) {
   const int lane = threadIdx.x & 31;
   uint32_t incl = len;
 #pragma unroll
@@ -530,18 +507,24 @@ __device__ __forceinline__ void warp_expand_rows3(uint32_t rs, uint32_t len, uin
   }
   const uint32_t total = __shfl_sync(kFull, incl, 31);
   const uint32_t excl = incl - len;
-  for (uint32_t jb = 0; jb < total; jb += 32) {
-    const uint32_t j = jb + lane;
-    int k = 0;
+  for (uint32_t jb = 0; jb < total; jb += 32u * NB) {
+    uint32_t ee[NB];
+    int kk[NB];
+    bool ok[NB];
 #pragma unroll
-    for (int step = 16; step >= 1; step >>= 1) {
-      const uint32_t ex = __shfl_sync(kFull, excl, k + step);
-      if (ex <= j) k += step;
+    for (int q = 0; q < NB; ++q) {
+      const uint32_t j = jb + (uint32_t)q * 32u + lane;
+      int k = 0;
+#pragma unroll
+      for (int step = 16; step >= 1; step >>= 1) {
+        const uint32_t ex = __shfl_sync(kFull, excl, k + step);
+        if (ex <= j) k += step;
+      }
+      ee[q] = __shfl_sync(kFull, rs, k) - __shfl_sync(kFull, excl, k) + j;
+      kk[q] = k;
+      ok[q] = j < total;
     }
-    const uint32_t base = __shfl_sync(kFull, rs, k) - __shfl_sync(kFull, excl, k);
-    const uint32_t a = __shfl_sync(kFull, pa, k), b = __shfl_sync(kFull, pb, k),
-                   c = __shfl_sync(kFull, pc, k);
-    if (j < total) f(base + j, a, b, c);
+    f(ee, kk, ok);
   }
 }
 

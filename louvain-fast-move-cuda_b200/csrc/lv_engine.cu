@@ -205,9 +205,8 @@ static const int32_t kTuneCandidates[][7] = {
     {4, 8, 16, 32, 128, 1024, 4096}, {8, 16, 32, 64, 256, 1024, 4096}, {8, 16, 32, 64, 128, 512, 2048},
 };
 constexpr int kTuneN = sizeof(kTuneCandidates) / sizeof(kTuneCandidates[0]);
-static const int kTeamT[6] = {4, 8, 16, 32, 32, 32};
-// Lanes per vertex of the gain kernels' bins: fewer than the contraction's for the short bins (a
-// quarter for rows up to 32 entries, half for rows up to 128), so each lane takes up to four
+// Lanes per vertex of the gain kernels' bins: a quarter of the row's entries for the short bins, half
+// a warp for rows up to 128, so each lane takes up to four
 // entries of its row per step (kBatch) and a warp works on several vertices at once, sharing
 // the per-vertex instructions among them.
 static const int kOptT[6] = {1, 2, 4, 8, 16, 32};
@@ -398,7 +397,7 @@ class Run {
     if ((size_t)block_cap * slot > (size_t)max_smem - 1024 || block_cap > 65536)
       throw Fail{LV_ERR_ARGUMENT, "bin 6 table does not fit shared memory"};
     for (int b = 0; b < 6; ++b)
-      if ((size_t)(256 / std::min(kTeamT[b], kOptT[b])) * team_cap[b] * slot > (size_t)max_smem - 1024)
+      if ((size_t)(256 / kOptT[b]) * team_cap[b] * slot > (size_t)max_smem - 1024)
         throw Fail{LV_ERR_ARGUMENT, "team bin table does not fit shared memory"};
   }
 
@@ -408,11 +407,11 @@ class Run {
   size_t con_slot_bytes() const { return 4 + acc_size() + 1; }
   size_t opt_slot_bytes() const { return 4 + acc_size() + 1 + (wint ? 2 : 0); }
 
-  // T: the contraction kernel's lanes per row, TO: the gain kernel's
-  template <int T, int TO>
+  // TO: the gain kernel's lanes per row (the contraction takes a warp per community)
+  template <int TO>
   void team_grid(int b, const void* opt_fn, const void* con_fn) {
     const size_t osmem = (size_t)(256 / TO) * team_cap[b] * opt_slot_bytes();
-    const size_t csmem = (size_t)(256 / T) * team_cap[b] * con_slot_bytes();
+    const size_t csmem = (size_t)8 * team_cap[b] * con_slot_bytes();
     ensure_dyn_smem(ctx->device, opt_fn, osmem);
     ensure_dyn_smem(ctx->device, con_fn, csmem);
     grid_team[b] = ctx->sms * std::max(1, occupancy(ctx->device, opt_fn, 256, osmem));
@@ -420,12 +419,12 @@ class Run {
 
   template <bool WI>
   void configure_kernels() {
-    team_grid<4, 1>(0, (const void*)k_opt_team<1, WI>, (const void*)k_contract_team<4, WI>);
-    team_grid<8, 2>(1, (const void*)k_opt_team<2, WI>, (const void*)k_contract_team<8, WI>);
-    team_grid<16, 4>(2, (const void*)k_opt_team<4, WI>, (const void*)k_contract_team<16, WI>);
-    team_grid<32, 8>(3, (const void*)k_opt_team<8, WI>, (const void*)k_contract_team<32, WI>);
-    team_grid<32, 16>(4, (const void*)k_opt_team<16, WI>, (const void*)k_contract_team<32, WI>);
-    team_grid<32, 32>(5, (const void*)k_opt_team<32, WI>, (const void*)k_contract_team<32, WI>);
+    team_grid<1>(0, (const void*)k_opt_team<1, WI>, (const void*)k_contract_warp<WI>);
+    team_grid<2>(1, (const void*)k_opt_team<2, WI>, (const void*)k_contract_warp<WI>);
+    team_grid<4>(2, (const void*)k_opt_team<4, WI>, (const void*)k_contract_warp<WI>);
+    team_grid<8>(3, (const void*)k_opt_team<8, WI>, (const void*)k_contract_warp<WI>);
+    team_grid<16>(4, (const void*)k_opt_team<16, WI>, (const void*)k_contract_warp<WI>);
+    team_grid<32>(5, (const void*)k_opt_team<32, WI>, (const void*)k_contract_warp<WI>);
     grid_short = ctx->sms * std::max(1, occupancy(ctx->device, (const void*)k_opt_short<WI>, 256, 0));
     const size_t bsmem = (size_t)block_cap * opt_slot_bytes();
     ensure_dyn_smem(ctx->device, (const void*)k_opt_block<WI>, bsmem);
@@ -1079,14 +1078,20 @@ class Run {
     k_hub_insert_long<WI><<<ctx->sms * 8, 256, 0, st>>>(Dd);
     k_hub_emit<WI><<<ctx->sms * 8, 512, 0, st>>>(Dd);
     on(1);
-    k_contract_team<32, WI><<<grid_team[5], 256, (256 / 32) * team_cap[5] * slot, st>>>(Dd, 5, team_cap[5]);
-    k_contract_team<4, WI><<<grid_team[0], 256, (256 / 4) * team_cap[0] * slot, st>>>(Dd, 0, team_cap[0]);
+    k_contract_warp<WI><<<grid_team[5], 256, 8 * team_cap[5] * slot, st>>>(Dd, 5, team_cap[5]);
     on(2);
-    k_contract_team<32, WI><<<grid_team[4], 256, (256 / 32) * team_cap[4] * slot, st>>>(Dd, 4, team_cap[4]);
-    k_contract_team<8, WI><<<grid_team[1], 256, (256 / 8) * team_cap[1] * slot, st>>>(Dd, 1, team_cap[1]);
+    k_contract_warp<WI><<<grid_team[4], 256, 8 * team_cap[4] * slot, st>>>(Dd, 4, team_cap[4]);
     on(3);
-    k_contract_team<32, WI><<<grid_team[3], 256, (256 / 32) * team_cap[3] * slot, st>>>(Dd, 3, team_cap[3]);
-    k_contract_team<16, WI><<<grid_team[2], 256, (256 / 16) * team_cap[2] * slot, st>>>(Dd, 2, team_cap[2]);
+    // the bins of up to kPairMax entries by all pairs, wider ones (configured) by warps
+    uint32_t pairs = 0;
+    for (int b = 0; b < kShortBins; ++b)
+      if (bins.maxdeg[b] <= kPairMax) pairs |= 1u << b;
+    if (pairs) { k_contract_short<WI><<<ctx->sms * 8, 256, 0, st>>>(Dd, pairs); ++launches; }
+    for (int b = 0; b < kShortBins; ++b)
+      if (!(pairs >> b & 1u)) {
+        k_contract_warp<WI><<<grid_team[b], 256, 8 * team_cap[b] * slot, st>>>(Dd, b, team_cap[b]);
+        ++launches;
+      }
     on(4);
     k_contract_block<WI><<<grid_block[0], 512, block_cap * slot, st>>>(Dd, 6, block_cap);
     on(5);
@@ -1096,7 +1101,7 @@ class Run {
     scan<uint32_t, false, kScanDeg>();
     k_agg_compact<WI><<<grid_n, 256, 0, st>>>(Dd);
     agg_finish();
-    launches += 14;
+    launches += 10;
   }
   void agg_finish() {
     k_agg_finish<<<grid_n, 256, 0, st>>>(Dd);

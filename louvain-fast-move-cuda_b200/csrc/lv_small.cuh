@@ -39,7 +39,6 @@ constexpr int kSmallMaxCtas = 8;
 template <int NT> constexpr bool kCompact = NT != 512;
 template <int NT> constexpr int kSmallBatch = kCompact<NT> ? 2 : kBatch;
 template <int NT> constexpr int kSmallApply = kCompact<NT> ? 2 : kApplyBatch;
-constexpr uint32_t kPairMax = 32;  // degree sum up to which a community is contracted by all pairs
 constexpr int kSmallShare = 2048;  // entries that make a further CTA of the cluster worth its barriers
 constexpr int kSmallLists = 4;  // rows of up to 8 and 32 entries, rows for a warp, rows for a CTA
 
@@ -373,10 +372,7 @@ __device__ __forceinline__ void small_contract(SmallRun<WINT, NT>& R, uint32_t* 
   const Wt* w = reinterpret_cast<const Wt*>(R.L.w);
   const uint32_t n2 = R.cnt->n2;
   const uint32_t lt = lanemask_lt();
-  auto out_w = [](Acc x) -> Wt {
-    if (WINT) return (Wt)x;
-    return (Wt)__double2float_rn((double)x);
-  };
+  auto out_w = [](Acc x) { return contracted_weight<WINT>(x); };
   auto finish = [&](uint32_t s, uint32_t tb, uint32_t nl, Acc self, double ksum) {  // one thread
     const bool has = self != Acc(0);  // weights are positive
     if (has) {
@@ -476,76 +472,9 @@ __device__ __forceinline__ void small_contract(SmallRun<WINT, NT>& R, uint32_t* 
       }
     }
     if (!__any_sync(kFull, dsum > 0)) continue;
-    // entry p of the members' rows in order goes to lane p % 8, place p / 8
-    uint32_t ent[4], cc[4];
-    Acc ss[4];
-    Wt ww[4];
-#pragma unroll
-    for (int q = 0; q < 4; ++q) ent[q] = kEmpty;
-    uint32_t pos = 0;
-    const uint32_t mmax = __reduce_max_sync(kFull, mc);
-    for (uint32_t mo = 0; mo < mmax; mo += 8) {
-      uint32_t rs = 0, len = 0;
-      if (mo + tl < mc) {
-        const uint32_t v = D.members[mb + mo + tl];
-        rs = R.rs[v];
-        len = R.len[v];
-      }
-#pragma unroll 1
-      for (int j = 0; j < 8; ++j) {
-        const uint32_t r0 = __shfl_sync(kFull, rs, j, 8), l0 = __shfl_sync(kFull, len, j, 8);
-#pragma unroll
-        for (int q = 0; q < 4; ++q) {
-          const uint32_t p = (uint32_t)q * 8u + tl;
-          if (p - pos < l0) ent[q] = r0 + (p - pos);
-        }
-        pos += l0;
-      }
-    }
-    Acc self = Acc(0);
-#pragma unroll
-    for (int q = 0; q < 4; ++q) {
-      cc[q] = ent[q] != kEmpty ? D.new_comm[R.L.col[ent[q]]] : kEmpty;
-      ww[q] = ent[q] != kEmpty ? (R.unit ? Wt(1) : w[ent[q]]) : Wt(0);
-      ss[q] = Acc(0);
-      if (cc[q] == s) {  // (no vertex id is kEmpty)
-        self += (Acc)ww[q];
-        cc[q] = kEmpty;
-      }
-    }
-    pair_sums<8, WINT, false, kCompact<NT>>(cc, ww, __reduce_max_sync(kFull, dsum), ss);
-    self = team_sum<8>(self);
-    // the first entry of each community emits it
-    bool first[4];
-#pragma unroll
-    for (int q = 0; q < 4; ++q) first[q] = cc[q] != kEmpty;
-#pragma unroll
-    for (int p = 0; p < 4; ++p) {
-#pragma unroll 1
-      for (uint32_t j = 0; j < 8; ++j) {
-        const uint32_t c = __shfl_sync(kFull, cc[p], j, 8);
-        if (c == cc[p] && j < tl) first[p] = false;
-#pragma unroll
-        for (int q = p + 1; q < 4; ++q)
-          if (c == cc[q]) first[q] = false;
-      }
-    }
-    uint32_t nl = 0;
-    double ksum = 0.0;
-#pragma unroll
-    for (int q = 0; q < 4; ++q) {
-      const unsigned mk = (__ballot_sync(kFull, first[q]) >> (R.lane & 24)) & 0xFFu;
-      if (first[q]) {
-        const uint32_t at = tb + nl + __popc(mk & ((1u << tl) - 1u));
-        const Wt x = out_w(ss[q]);
-        colN[at] = cc[q];
-        wN[at] = x;
-        ksum += Tr::w_double(x);
-      }
-      nl += __popc(mk);
-    }
-    ksum = team_sum<8>(ksum);
-    if (dsum > 0 && tl == 0) finish(s, tb, nl, self, ksum);
+    contract_pairs<WINT, kCompact<NT>>(
+        D.members, D.new_comm, R.L.col, w, R.unit, s, mb, mc, tb, dsum, colN, wN,
+        [&](uint32_t v, uint32_t& rs, uint32_t& len) { rs = R.rs[v]; len = R.len[v]; }, finish);
   }
   // other communities for a warp: members 32 at a time, entries spread over the lanes
   uint16_t* list = R.list + R.wid * (R.wcap / 2);
@@ -562,24 +491,7 @@ __device__ __forceinline__ void small_contract(SmallRun<WINT, NT>& R, uint32_t* 
         rs = R.rs[v];
         len = R.len[v];
       }
-      warp_expand_rows_all(rs, len, [&](uint32_t e, bool valid) {
-        bool made = false;
-        uint32_t slot = 0;
-        if (valid) {
-          const uint32_t d = D.new_comm[R.L.col[e]];
-          const Acc wv = R.unit ? Acc(1) : (Acc)w[e];
-          if (d == s) {
-            self += wv;
-          } else {
-            const int r = tbl.add_at(d, wv, slot);
-            if (!r) R.err |= kErrTableFull;
-            made = r == 2;
-          }
-        }
-        const unsigned mk = __ballot_sync(kFull, made);
-        if (made) list[nl + __popc(mk & lt)] = (uint16_t)slot;
-        nl += __popc(mk);
-      });
+      contract_rows<WINT, kCompact<NT> ? 1 : kContractBatch>(D.new_comm, R.L.col, w, R.unit, rs, len, s, tbl, list, nl, self, R.err);
     }
     self = warp_sum(self);
     __syncwarp();
