@@ -903,9 +903,11 @@ __device__ __forceinline__ void fast_rows(const Dev& D, const uint32_t* vlist, u
 // few graphs in flight and in L2 (a contiguous share per block instead: 1.61
 // against 1.22 ms for the first pass over 768 graphs with 20 M vertices). The runs of different bins
 // start at different blocks, so that small lists spread over the GPU.
+// (64 registers, four blocks per SM: planted partition with fp32 weights 14.81 ms at 80 registers,
+// 14.29 at 64, 14.7 at 48, 15.3 at 40 with spills.)
 constexpr uint32_t kShortRun = 8;
 template <bool WINT>
-__global__ void __launch_bounds__(256, WINT ? 4 : 3) k_opt_short(int dslot, uint32_t mask) {
+__global__ void __launch_bounds__(256, 4) k_opt_short(int dslot, uint32_t mask) {
   const Dev& D = c_dev[dslot];
   Ctrl* C = D.ctrl;
   __shared__ uint32_t s_mov[8][64];
