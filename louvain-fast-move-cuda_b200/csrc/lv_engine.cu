@@ -33,6 +33,8 @@ namespace lv {
 // Everything that fixes the kernel sequence of a captured run apart from the data: when two
 // runs agree on it, the second reuses the first one's instantiated graph.
 struct GraphKey {
+  int32_t kind;      // 0: the level loop; a refined run's pass loops: 1 its own passes, 2 the refinement's
+  uint32_t max_pass;
   int32_t wint, single, full_walk, mode, fast_first, max_levels, sms, grid_n, grid_sq, grid_block;
   int64_t chunk_edges;
   uint32_t maxdeg[kNumBins], block_cap, team_cap[6];
@@ -825,7 +827,8 @@ class Run {
   // ---- level start ------------------------------------------------------------------------------
   // view: a refinement pass (regular passes only: no fast pass, no trace record)
   void commit(int level_start_flag, bool view = false) {
-    const PassEnd pe{single() ? 1 : 0, level_start_flag, cfg.mode, view ? 0 : cfg.fast_first, view ? 1 : 0};
+    const PassEnd pe{single() ? 1 : 0, level_start_flag, cfg.mode, view ? 0 : cfg.fast_first, view ? 1 : 0,
+                     view ? (uint32_t)std::max(0, cfg.refine_passes) : 0u};
     if (wint) k_commit<true><<<grid_sq, 256, 0, st>>>(Dd, pe, gc);
     else k_commit<false><<<grid_sq, 256, 0, st>>>(Dd, pe, gc);
     ++launches;
@@ -1040,6 +1043,9 @@ class Run {
     Dd = Dr;
     try {
       commit(1, true);
+      if (loops_captured()) {
+        if (ctrl_u32(offsetof(Ctrl, n_iterating)) > 0) refine_passes_run += run_passes<WI>(true);
+      } else
       for (int64_t p = 0;; ++p) {
         const uint32_t left = ctrl_u32(offsetof(Ctrl, n_iterating));
         if (left == 0 || (cfg.refine_passes > 0 && p >= cfg.refine_passes)) break;
@@ -1253,12 +1259,7 @@ class Run {
   template <bool WI>
   DevSlot::Loop* build_graph() {
     DevSlot::Loop loop;
-    for (auto& x : slot->cs)
-      if (!x) LV_CUDA(cudaStreamCreateWithFlags(&x, cudaStreamNonBlocking));
-    for (auto& x : slot->bs)
-      if (!x) LV_CUDA(cudaStreamCreateWithFlags(&x, cudaStreamNonBlocking));
-    for (auto& x : slot->be)
-      if (!x) LV_CUDA(cudaEventCreateWithFlags(&x, cudaEventDisableTiming));
+    make_capture_streams();
     cudaStream_t* cs = slot->cs;
     cudaGraph_t graph = nullptr;
     LV_CUDA(cudaGraphCreate(&graph, 0));
@@ -1325,6 +1326,72 @@ class Run {
     gc.on = 0;
     launches = l0;
     return slot->add(loop);
+  }
+
+  // A refined run is driven by the host between its phases, but the passes of a phase are one captured
+  // loop -- the level's own, or the refinement's through the refine view -- instead of a dozen
+  // launches and a readback each.
+  bool in_louvain = false;
+  bool loops_captured() const { return cfg.use_graphs && cfg.refine && !debug && in_louvain; }
+  template <bool WI>
+  uint32_t run_passes(bool view) {
+    GraphKey key = graph_key();
+    key.kind = view ? 2 : 1;
+    key.max_pass = view ? (uint32_t)std::max(0, cfg.refine_passes) : 0u;
+    DevSlot::Loop* loop = slot->find(key);
+    if (!loop) {
+      DevSlot::Loop l;
+      make_capture_streams();
+      LV_CUDA(cudaGraphCreate(&l.graph, 0));
+      const int64_t l0 = launches;
+      try {
+        cudaGraphConditionalHandle h;
+        LV_CUDA(cudaGraphConditionalHandleCreate(&h, l.graph, 1, cudaGraphCondAssignDefault));
+        gc = GraphCtl{};
+        gc.pass = h;
+        gc.on = 1;
+        cudaGraphNodeParams p{};
+        p.type = cudaGraphNodeTypeConditional;
+        p.conditional.handle = h;
+        p.conditional.type = cudaGraphCondTypeWhile;
+        p.conditional.size = 1;
+        cudaGraphNode_t top;
+        LV_CUDA(cudaGraphAddNode(&top, l.graph, nullptr, 0, &p));
+        capture_into(p.conditional.phGraph_out[0], slot->cs[0], [&] {
+          if (view) {
+            k_ref_select<<<grid_n, 256, 0, st>>>(Dd);
+            ++launches;
+          }
+          launch_pass<WI>(view);
+        });
+        l.k_pass = launches - l0;
+        LV_CUDA(cudaGraphInstantiate(&l.exec, l.graph, 0));
+      } catch (...) {
+        gc.on = 0;
+        launches = l0;
+        l.release();
+        throw;
+      }
+      l.key = key;
+      l.gc = gc;
+      gc.on = 0;
+      launches = l0;
+      loop = slot->add(l);
+    }
+    LV_CUDA(cudaGraphLaunch(loop->exec, st));
+    wait_bounded(600.0);
+    const uint32_t passes = ctrl_u32(offsetof(Ctrl, pass));
+    launches += (int64_t)passes * loop->k_pass;
+    check_device_errors();
+    return passes;
+  }
+  void make_capture_streams() {
+    for (auto& x : slot->cs)
+      if (!x) LV_CUDA(cudaStreamCreateWithFlags(&x, cudaStreamNonBlocking));
+    for (auto& x : slot->bs)
+      if (!x) LV_CUDA(cudaStreamCreateWithFlags(&x, cudaStreamNonBlocking));
+    for (auto& x : slot->be)
+      if (!x) LV_CUDA(cudaEventCreateWithFlags(&x, cudaEventDisableTiming));
   }
 
   // Waits for the stream, giving up (with an error; the work may still be running) after
@@ -1399,9 +1466,21 @@ class Run {
   int32_t optimization_run() {
     int32_t passes = 0;
     const double before = t_opt_ms;
-    while (true) {
-      ++passes;
-      if (pass() == 0) break;
+    if (loops_captured()) {
+      const double k0 = read_ctrl<unsigned long long>(offsetof(Ctrl, t_optk_ns)) * 1e-6;
+      LV_CUDA(cudaEventRecord(ev[0], st));
+      passes = (int32_t)(wint ? run_passes<true>(false) : run_passes<false>(false));
+      LV_CUDA(cudaEventRecord(ev[1], st));
+      LV_CUDA(cudaEventSynchronize(ev[1]));
+      float ms = 0;
+      LV_CUDA(cudaEventElapsedTime(&ms, ev[0], ev[1]));
+      t_opt_ms += ms;
+      t_optk_ms += read_ctrl<unsigned long long>(offsetof(Ctrl, t_optk_ns)) * 1e-6 - k0;
+    } else {
+      while (true) {
+        ++passes;
+        if (pass() == 0) break;
+      }
     }
     if (t_opt0 < 0) t_opt0 = t_opt_ms - before;
     check_device_errors();
@@ -1425,6 +1504,8 @@ class Run {
       if (wint) louvain_graph<true>(); else louvain_graph<false>();
       return;
     }
+    in_louvain = true;
+    struct Reset { bool& b; ~Reset() { b = false; } } reset{in_louvain};
     while (!finished) {
       optimization_run();
       aggregate(-1);

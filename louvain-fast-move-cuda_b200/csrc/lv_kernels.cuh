@@ -1664,6 +1664,7 @@ __global__ void k_set_pass(Ctrl* C, uint32_t p, int mode, int fast_first) {
 // previous level's end). view = 1: a refinement pass (no trace record, no pass statistics).
 struct PassEnd {
   int single, level_start, mode, fast_first, view;
+  uint32_t max_pass;  // captured pass loops end after this many passes (0: no limit)
 };
 
 // The part after every block's commit, by the last block of k_commit (256 threads).
@@ -1773,9 +1774,9 @@ __device__ __forceinline__ void finalize(const Dev& D, const PassEnd& pe, const 
         C->seg_passes += 1;
         C->t_opt_ns += global_ns() - C->t_pass0;
       }
-      if (C->seg_passes > kGuardPasses) atomicOr(&C->err, kErrLoop);
+      if (C->seg_passes > kGuardPasses || C->pass > kGuardPasses) atomicOr(&C->err, kErrLoop);
       // the captured pass loop runs while a graph iterates (and no guard has tripped)
-      set_cond(gc, gc.pass, tot > 0 && !(C->err & kErrLoop));
+      set_cond(gc, gc.pass, tot > 0 && (pe.max_pass == 0 || C->pass < pe.max_pass) && !(C->err & kErrLoop));
     }
     set_pass_rule(C, C->pass, pe.mode, pe.fast_first);
   }
