@@ -58,6 +58,7 @@ struct GraphState {
   uint32_t total_iters;
   uint32_t moved;     // moves of the last pass
   uint32_t n_next;    // aggregation: vertices of this graph at the next level
+  uint32_t next_base, pad_next;  // and the first of their ids
   unsigned long long I_full;  // internal weight summed by k_apply_full (u64 or double bits)
   double inv_m;       // rn(1/m) and rn(1/two_m2), for the gain upper bound only
   double inv_2m2;
@@ -137,6 +138,10 @@ struct Ctrl {
   uint32_t commit_ticket, scan_ticket, bin_ticket;  // blocks done: the last one does the kernel's tail
   uint32_t pad_ticket;
   unsigned long long mover_entries;  // entries of this pass's movers
+  // aggregation: the communities contracted by ranges (k_range_*), their entries and ranges, the
+  // 32-member groups they are walked in and the next group of the count and of the scatter
+  uint32_t range_comms, range_entries, range_buckets, range_groups, range_work[2];
+  uint32_t range_slices, pad_range;
   TraceRec trace[kTraceCap];
 };
 

@@ -35,7 +35,7 @@ namespace lv {
 struct GraphKey {
   int32_t kind;      // 0: the level loop; a refined run's pass loops: 1 its own passes, 2 the refinement's
   uint32_t max_pass;
-  int32_t wint, single, full_walk, mode, fast_first, max_levels, sms, grid_n, grid_sq, grid_block;
+  int32_t wint, single, full_walk, ranges, mode, fast_first, max_levels, sms, grid_n, grid_sq, grid_block;
   int64_t chunk_edges;
   uint32_t maxdeg[kNumBins], block_cap, team_cap[6];
   int32_t grid_team[6];
@@ -71,8 +71,8 @@ struct DevSlot {
   static constexpr size_t kMaxLoops = 6;
   std::vector<Loop> loops;
   cudaStream_t cs[3] = {nullptr, nullptr, nullptr};  // capture streams of nested bodies
-  cudaStream_t bs[5] = {};                           // and of the branches inside a body
-  cudaEvent_t be[6] = {};                            // fork, and the end of each branch
+  cudaStream_t bs[6] = {};                           // and of the branches inside a body
+  cudaEvent_t be[7] = {};                            // fork, and the end of each branch
 
   // The loop captured for `key` moved to the front, or nullptr. (A run waits for its launches before
   // it ends, so no loop is in flight when another is looked up.)
@@ -296,6 +296,7 @@ class Run {
   bool own_pinned = false;
   bool finished = false;
   bool chunked = false;        // level 0 spans several edge chunks (later levels have fewer entries)
+  bool ranges = false;         // large communities may be contracted by ranges
   bool full_walk = false;      // some level can have a heavy pass (later levels have fewer entries)
   bool small_ok = false;       // a whole run from its input: k_small may take its small graphs
   int32_t levels_run = 0;
@@ -781,6 +782,15 @@ class Run {
     launches += 4;
     chunked = single() && cfg.chunk_edges > 0 && (int64_t)E > cfg.chunk_edges;
     full_walk = E >= kFullMinE;
+    ranges = wint && E >= kRangeMinE;
+    if (ranges) {
+      const size_t nr = (size_t)E / kRangeMin + 64;
+      D.range_owner = dalloc<uint32_t>(ctx, owned, nr, st);
+      D.range_count = dalloc<uint32_t>(ctx, owned, nr, st);
+      D.range_cur = dalloc<uint32_t>(ctx, owned, nr, st);
+      dev_dirty = true;
+      bind();
+    }
     plan_small(ho, eo);
     if (small_count()) return;  // louvain() starts with them
     check_device_errors();
@@ -1070,7 +1080,7 @@ class Run {
   void agg_contract_a() {
     k_agg_count<<<grid_n, 256, 0, st>>>(Dd);
     scan<unsigned long long, false, kScanCd>();
-    k_agg_scatter_bin<<<grid_n, 256, 0, st>>>(Dd, bins, gc);
+    k_agg_scatter_bin<<<grid_n, 256, 0, st>>>(Dd, bins, ranges ? (int)kRangeLog : 0, gc);
     launches += 2;
   }
   template <bool WI>
@@ -1078,7 +1088,24 @@ class Run {
     const size_t slot = con_slot_bytes();
     // independent: the largest new communities (many blocks insert into their global tables), the
     // others by team or block, and the input vertices' new communities
-    fork(5);
+    fork(ranges ? 6 : 5);
+    if (ranges) {
+      on(6);
+      const int g = ctx->sms * 8;
+      k_range_setup<<<ctx->sms * 2, 256, 0, st>>>(Dd);
+      k_range_rows<false><<<g, 256, 0, st>>>(Dd);
+      k_range_rows_long<false><<<g, 256, 0, st>>>(Dd);
+      k_range_place<<<ctx->sms, 256, 0, st>>>(Dd);
+      k_range_rows<true><<<g, 256, 0, st>>>(Dd);
+      k_range_rows_long<true><<<g, 256, 0, st>>>(Dd);
+      const size_t rsmem = sizeof(uint32_t) << kRangeLog;
+      ensure_dyn_smem(ctx->device, (const void*)k_range_fold, rsmem);
+      ensure_dyn_smem(ctx->device, (const void*)k_range_emit, rsmem);
+      k_range_fold<<<ctx->sms * 3, 512, rsmem, st>>>(Dd);
+      k_range_emit<<<ctx->sms * 3, 512, rsmem, st>>>(Dd);
+      launches += 8;
+      on(0);
+    }
     k_hub_setup<WI><<<ctx->sms * 8, 256, 0, st>>>(Dd);
     k_hub_insert<WI><<<grid_n, 256, 0, st>>>(Dd);
     k_hub_insert_long<WI><<<ctx->sms * 8, 256, 0, st>>>(Dd);
@@ -1145,7 +1172,7 @@ class Run {
         k_ref_prev<<<grid_n, 256, 0, st>>>(Dd);
         launches += 2;
       }
-      const uint32_t need = ctrl_u32(offsetof(Ctrl, hub_cursor));
+      const uint32_t need = ctrl_u32(offsetof(Ctrl, hub_cursor)) + ctrl_u32(offsetof(Ctrl, range_entries));
       if (debug) {
         uint32_t bc[kNumBins];
         LV_CUDA(cudaMemcpy(bc, reinterpret_cast<char*>(D.ctrl) + offsetof(Ctrl, bin_count), sizeof(bc), cudaMemcpyDeviceToHost));
@@ -1199,6 +1226,7 @@ class Run {
     k.wint = wint;
     k.single = single();
     k.full_walk = full_walk;
+    k.ranges = ranges;
     k.mode = cfg.mode;
     k.fast_first = cfg.fast_first;
     k.max_levels = cfg.max_levels;

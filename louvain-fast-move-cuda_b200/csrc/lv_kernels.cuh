@@ -67,6 +67,8 @@ struct Dev {
   // k_bin_vertices, so that an entry's community and that community's total (a u32: integer
   // totals stay below 2m < 2^32) arrive with one gather
   unsigned long long* ca;
+  // contraction by ranges: per (community, range) its community's index, entry count, write cursor
+  uint32_t *range_owner, *range_count, *range_cur;  // [E / kRangeMin + 64]
   // refinement (allocated only when it is on; lv_refine.cuh)
   uint32_t* ref;             // [n] refined partition
   uint32_t* ref_new;         // [n] its pass targets
@@ -101,6 +103,23 @@ constexpr uint32_t kHubInsPiece = 8192;
 constexpr uint32_t kHubPiece = 8192;
 
 constexpr int kMaxPartials = 2048;
+
+// Contraction by ranges (k_range_*): the next-level ids are split over up to kRangeMax ranges of
+// 2^log ids, at least kRangeMin entries per range on average; 2^kRangeLog ids at most, whose sums
+// (u32: integer weights only) fill 64 KB of shared memory, three blocks per SM.
+constexpr uint32_t kRangeLog = 14;
+constexpr uint32_t kRangeSlice = 32768;  // entries of a range folded by one block (k_range_fold)
+constexpr uint32_t kRangeMax = 64, kRangeMin = 2048;
+constexpr uint32_t kRangeMinE = 1u << 24;  // entries of level 0 from which on it is used at all
+__host__ __device__ __forceinline__ uint32_t range_log(uint32_t dsum, uint32_t ids) {
+  uint32_t nr = dsum / kRangeMin;
+  nr = nr < 1 ? 1 : nr > kRangeMax ? kRangeMax : nr;
+  const uint32_t per = (ids + nr - 1) / nr;
+  uint32_t log = 0;
+  while ((1u << log) < per) ++log;
+  return log;  // (ids + 2^log - 1) >> log ranges, at most nr
+}
+constexpr uint32_t kRangeLongRow = 1024;  // longer member rows: a block per 8192-entry piece
 
 // Capacity of a bin-7 vertex's global optimisation table: table_cap rounded up to a whole
 // kHubChunk, so every chunk of the arena belongs to one vertex.
@@ -2382,6 +2401,7 @@ __global__ void __launch_bounds__(1024) k_agg_meta(int dslot, GraphCtl gc) {
     st->map_base = (uint32_t)(before >> 32);
     st->n_best = (uint32_t)(end >> 32) - st->map_base;
     st->n_next = (uint32_t)end - (uint32_t)before;
+    st->next_base = (uint32_t)before;
   }
   if (threadIdx.x == 0) {
     const uint32_t n2 = n ? (uint32_t)D.map[n - 1] : 0u;
@@ -2449,7 +2469,7 @@ __device__ __forceinline__ uint32_t contract_cap(uint32_t dsum, uint32_t ng, boo
 // The same kernel places the members (independent work), and its last block checks (captured run)
 // that the global tables fit the arena; if not, the run stops here (nothing of this aggregation is
 // final yet) and the host grows the arena and redoes it.
-__global__ void __launch_bounds__(256) k_agg_scatter_bin(int dslot, BinCfg B, GraphCtl gc) {
+__global__ void __launch_bounds__(256) k_agg_scatter_bin(int dslot, BinCfg B, int max_log, GraphCtl gc) {
   const Dev& D = c_dev[dslot];
   Ctrl* C = D.ctrl;
   const uint32_t n = C->n, n2 = C->n_next;
@@ -2471,6 +2491,19 @@ __global__ void __launch_bounds__(256) k_agg_scatter_bin(int dslot, BinCfg B, Gr
         cap = contract_cap(dsum, D.gs[g].n_next, bin == kNumBins - 1);
         // a bin-6 community whose table fits half the block table: the half-block list
         if (bin == kNumBins - 2 && 2u * cap <= B.block_cap) bin = kHalfBin;
+        // a bin-7 community with entries enough per range of next-level ids: contracted by ranges
+        // (max_log > 0: on)
+        if (bin == kNumBins - 1 && max_log > 0) {
+          const uint32_t ids = D.gs[g].n_next, log = range_log(dsum, ids);
+          const uint32_t nr = (ids + (1u << log) - 1u) >> log;
+          if (log <= (uint32_t)max_log) {
+            const uint32_t i = atomicAdd(&C->range_comms, 1u);
+            const uint32_t eo = atomicAdd(&C->range_entries, dsum), bo = atomicAdd(&C->range_buckets, nr);
+            D.movers[i] = s;  // (free between passes, as are cn and active_it)
+            D.cn[i] = ((unsigned long long)eo << 32) | bo;
+            bin = -1;
+          }
+        }
       }
     }
     // lane b claims bin b's space: one atomic latency for all bins
@@ -2494,7 +2527,7 @@ __global__ void __launch_bounds__(256) k_agg_scatter_bin(int dslot, BinCfg B, Gr
     }
   }
   if (gc.on && last_block(&C->bin_ticket) && threadIdx.x == 0) {
-    const uint32_t used = __ldcg(&C->hub_cursor);
+    const uint32_t used = __ldcg(&C->hub_cursor) + __ldcg(&C->range_entries);
     const bool ok = used <= C->arena_slots;
     if (ok) {
       C->seg_contract_ok += 1;
@@ -3234,6 +3267,369 @@ __global__ void __launch_bounds__(NT) k_contract_block(int dslot, int bin, uint3
   if (err) report_err(C, err, 8);  // k_contract_block
 }
 
+// ---- contraction by ranges ------------------------------------------------------------------------
+// Large communities (bin 7) with entries enough for their number of possible neighbours (range_log):
+// the entries are counted per (community, range of next-level ids), scattered to their range's place
+// behind the global tables in the arena (id and weight in one word), then each range is summed by one
+// block in an array indexed by id in shared memory and emitted. Two mostly coalesced passes and sums
+// on chip, instead of a read and an atomic per entry on tables that live in DRAM, with their
+// clearing and scanning. R-MAT scale 22 32.8 -> 30.0 ms (its second and third contractions took 4.1 and
+// 2.4 ms in the global tables), scale 20 11.24 -> 11.06; levels 0 of fewer than kRangeMinE entries and fp32
+// weights stay with the tables (R-MAT 300,000 3.50 -> 3.69 ms, planted partition 13.93 -> 14.21 with it).
+// Set-up, one warp per community; where its 32-member groups start among all groups (exclusive
+// prefix, in active_it) by the last block.
+__global__ void __launch_bounds__(256) k_range_setup(int dslot) {
+  const Dev& D = c_dev[dslot];
+  Ctrl* C = D.ctrl;
+  __shared__ uint32_t sh[33];
+  const uint32_t count = C->range_comms;
+  if (blockIdx.x == gridDim.x - 1) {
+    uint32_t run = 0;
+    for (uint32_t base = 0; base < count; base += 256) {
+      const uint32_t i = base + threadIdx.x;
+      uint32_t m = 0;
+      if (i < count) {
+        const uint32_t s = D.movers[i];
+        m = ((uint32_t)(D.cd[s + 1] >> 32) - (uint32_t)(D.cd[s] >> 32) + 31u) / 32u;
+      }
+      uint32_t tot;
+      const uint32_t ex = block_excl_scan<uint32_t, 256>(m, sh, &tot);
+      if (i < count) D.active_it[i] = run + ex;
+      run += tot;
+    }
+    if (threadIdx.x == 0) C->range_groups = run;
+  }
+  const uint32_t nb = C->range_buckets;
+  const uint32_t tid = blockIdx.x * blockDim.x + threadIdx.x, nth = gridDim.x * blockDim.x;
+  for (uint32_t i = tid; i < nb; i += nth) D.range_count[i] = 0;
+  for (uint32_t i = tid; i < count; i += nth) {
+    const uint32_t s = D.movers[i];
+    D.newdeg[s] = 0;
+    D.kB[s] = 0.0;
+    D.hubself[s] = 0ull;
+    D.hubtab[s] = i;  // (k_range_rows_long's way from a vertex to its community's index)
+  }
+}
+
+// One community as the range kernels see it.
+struct RangeComm {
+  uint32_t s, eo, bo, nr, log, base;
+};
+__device__ __forceinline__ RangeComm range_comm(const Dev& D, uint32_t i) {
+  RangeComm r;
+  r.s = D.movers[i];
+  const unsigned long long x = D.cn[i];
+  r.eo = (uint32_t)(x >> 32);
+  r.bo = (uint32_t)x;
+  const GraphState& st = D.gs[D.gidB ? D.gidB[r.s] : 0u];
+  r.base = st.next_base;
+  r.log = range_log((uint32_t)D.cd[r.s + 1] - (uint32_t)D.cd[r.s], st.n_next);
+  r.nr = (st.n_next + (1u << r.log) - 1u) >> r.log;
+  return r;
+}
+
+// SCATTER false: entries counted per range; true: counted again per group, the group's places
+// claimed (one atomic per range), and written. A warp takes 32 members of one community; rows over
+// kRangeLongRow entries are queued in pieces for k_range_rows_long (by the count).
+template <bool SCATTER>
+__global__ void __launch_bounds__(256) k_range_rows(int dslot) {
+  const Dev& D = c_dev[dslot];
+  using Acc = uint32_t;
+  using Wt = uint32_t;
+  Ctrl* C = D.ctrl;
+  __shared__ uint32_t s_hist[8][kRangeMax];
+  uint32_t* hist = s_hist[threadIdx.x >> 5];
+  const uint32_t count = C->range_comms, groups = C->range_groups;
+  const Wt* __restrict__ w = reinterpret_cast<const Wt*>(D.w);
+  const bool unit = unit_weights<true>(C);
+  unsigned long long* out = reinterpret_cast<unsigned long long*>(D.arena_vals);
+  const uint32_t lane = threadIdx.x & 31;
+  for (;;) {
+    uint32_t gi = 0;
+    if (lane == 0) gi = atomicAdd(&C->range_work[SCATTER ? 1 : 0], 1u);
+    gi = __shfl_sync(kFull, gi, 0);
+    if (gi >= groups) break;
+    uint32_t lo = 0, hi = count;  // the last community whose groups start at or before gi
+    while (hi - lo > 1) {
+      const uint32_t mid = (lo + hi) >> 1;
+      if (D.active_it[mid] <= gi) lo = mid; else hi = mid;
+    }
+    const RangeComm c = range_comm(D, lo);
+    const uint32_t mb = (uint32_t)(D.cd[c.s] >> 32) + (gi - D.active_it[lo]) * 32u;
+    const uint32_t me = (uint32_t)(D.cd[c.s + 1] >> 32);
+    uint32_t rs = 0, len = 0;
+    if (mb + lane < me) {
+      const uint32_t v = D.members[mb + lane];
+      rs = D.row[v];
+      len = D.row[v + 1] - rs;
+      if (len > kRangeLongRow) {
+        if (!SCATTER) {
+          const uint32_t np = (len + kHubPiece - 1) / kHubPiece;
+          const uint32_t p0 = atomicAdd(&C->apply_items, np);
+          for (uint32_t k = 0; k < np; ++k) D.apply_items[p0 + k] = ((unsigned long long)v << 32) | k;
+        }
+        len = 0;
+      }
+    }
+    for (uint32_t b = lane; b < c.nr; b += 32) hist[b] = 0;
+    __syncwarp();
+    Acc self = Acc(0);
+    warp_expand_rows_all<kContractBatch>(rs, len, [&](const uint32_t (&ee)[kContractBatch], const bool (&ok)[kContractBatch]) {
+      uint32_t dd[kContractBatch];
+#pragma unroll
+      for (int q = 0; q < kContractBatch; ++q) dd[q] = ok[q] ? D.col[ee[q]] : 0u;
+#pragma unroll
+      for (int q = 0; q < kContractBatch; ++q) dd[q] = ok[q] ? D.new_comm[dd[q]] : c.s;
+#pragma unroll
+      for (int q = 0; q < kContractBatch; ++q) {
+        if (dd[q] != c.s) atomicAdd(&hist[(dd[q] - c.base) >> c.log], 1u);
+        else if (SCATTER && ok[q]) self += unit ? Acc(1) : (Acc)w[ee[q]];
+      }
+    });
+    __syncwarp();
+    for (uint32_t b = lane; b < c.nr; b += 32) {
+      const uint32_t h = hist[b];
+      if (!SCATTER) { if (h) atomicAdd(&D.range_count[c.bo + b], h); }
+      else hist[b] = h ? atomicAdd(&D.range_cur[c.bo + b], h) : 0u;
+    }
+    __syncwarp();
+    if (SCATTER) {
+      warp_expand_rows_all<kContractBatch>(rs, len, [&](const uint32_t (&ee)[kContractBatch], const bool (&ok)[kContractBatch]) {
+        uint32_t dd[kContractBatch];
+        Wt wv[kContractBatch];
+#pragma unroll
+        for (int q = 0; q < kContractBatch; ++q) {
+          dd[q] = ok[q] ? D.col[ee[q]] : 0u;
+          wv[q] = ok[q] && !unit ? w[ee[q]] : Wt(1);
+        }
+#pragma unroll
+        for (int q = 0; q < kContractBatch; ++q) dd[q] = ok[q] ? D.new_comm[dd[q]] : c.s;
+#pragma unroll
+        for (int q = 0; q < kContractBatch; ++q)
+          if (dd[q] != c.s) {
+            const uint32_t at = atomicAdd(&hist[(dd[q] - c.base) >> c.log], 1u);
+            out[at] = ((unsigned long long)dd[q] << 32) | wv[q];
+          }
+      });
+      self = warp_sum(self);
+      if (lane == 0 && self != Acc(0)) {
+        atomicAdd(&D.hubself[c.s], (unsigned long long)self);
+      }
+      __syncwarp();
+    }
+  }
+}
+
+// The queued pieces of long rows, a block each.
+template <bool SCATTER>
+__global__ void __launch_bounds__(256) k_range_rows_long(int dslot) {
+  const Dev& D = c_dev[dslot];
+  using Acc = uint32_t;
+  using Wt = uint32_t;
+  Ctrl* C = D.ctrl;
+  __shared__ uint32_t hist[kRangeMax];
+  __shared__ Acc sh[33];
+  const Wt* __restrict__ w = reinterpret_cast<const Wt*>(D.w);
+  const bool unit = unit_weights<true>(C);
+  unsigned long long* out = reinterpret_cast<unsigned long long*>(D.arena_vals);
+  const uint32_t count = C->apply_items;
+  constexpr int NB = 4;
+  for (uint32_t i = blockIdx.x; i < count; i += gridDim.x) {
+    const unsigned long long it = D.apply_items[i];
+    const uint32_t v = (uint32_t)(it >> 32), piece = (uint32_t)it;
+    const RangeComm c = range_comm(D, D.hubtab[D.new_comm[v]]);
+    const uint32_t rs = D.row[v] + piece * kHubPiece, re = min(D.row[v + 1], rs + kHubPiece);
+    for (uint32_t b = threadIdx.x; b < c.nr; b += 256) hist[b] = 0;
+    __syncthreads();
+    Acc self = Acc(0);
+    for (uint32_t e0 = rs + threadIdx.x; e0 < re; e0 += NB * 256u) {
+      uint32_t dd[NB];
+#pragma unroll
+      for (int q = 0; q < NB; ++q) dd[q] = e0 + q * 256u < re ? D.col[e0 + q * 256u] : 0u;
+#pragma unroll
+      for (int q = 0; q < NB; ++q) dd[q] = e0 + q * 256u < re ? D.new_comm[dd[q]] : kEmpty;
+#pragma unroll
+      for (int q = 0; q < NB; ++q) {
+        if (dd[q] == kEmpty) continue;
+        if (dd[q] != c.s) atomicAdd(&hist[(dd[q] - c.base) >> c.log], 1u);
+        else if (SCATTER) self += unit ? Acc(1) : (Acc)w[e0 + q * 256u];
+      }
+    }
+    __syncthreads();
+    for (uint32_t b = threadIdx.x; b < c.nr; b += 256) {
+      const uint32_t h = hist[b];
+      if (!SCATTER) { if (h) atomicAdd(&D.range_count[c.bo + b], h); }
+      else hist[b] = h ? atomicAdd(&D.range_cur[c.bo + b], h) : 0u;
+    }
+    __syncthreads();
+    if (SCATTER) {
+      for (uint32_t e0 = rs + threadIdx.x; e0 < re; e0 += NB * 256u) {
+        uint32_t dd[NB];
+        Wt wv[NB];
+#pragma unroll
+        for (int q = 0; q < NB; ++q) {
+          const bool in = e0 + q * 256u < re;
+          dd[q] = in ? D.col[e0 + q * 256u] : 0u;
+          wv[q] = in && !unit ? w[e0 + q * 256u] : Wt(1);
+        }
+#pragma unroll
+        for (int q = 0; q < NB; ++q) dd[q] = e0 + q * 256u < re ? D.new_comm[dd[q]] : c.s;
+#pragma unroll
+        for (int q = 0; q < NB; ++q)
+          if (dd[q] != c.s) {
+            const uint32_t at = atomicAdd(&hist[(dd[q] - c.base) >> c.log], 1u);
+            out[at] = ((unsigned long long)dd[q] << 32) | wv[q];
+          }
+      }
+      self = block_sum<256>(self, sh);
+      if (threadIdx.x == 0 && self != Acc(0)) {
+        atomicAdd(&D.hubself[c.s], (unsigned long long)self);
+      }
+    }
+    __syncthreads();
+  }
+}
+
+// Between count and scatter, a warp per community: where each range's entries begin (in the arena,
+// behind the tables), whose each range is, and the slices of the long ones (in ca).
+__global__ void __launch_bounds__(256) k_range_place(int dslot) {
+  const Dev& D = c_dev[dslot];
+  Ctrl* C = D.ctrl;
+  const uint32_t count = C->range_comms, lane = threadIdx.x & 31;
+  const uint32_t nwarps = (gridDim.x * blockDim.x) >> 5;
+  for (uint32_t i = (blockIdx.x * blockDim.x + threadIdx.x) >> 5; i < count; i += nwarps) {
+    const RangeComm c = range_comm(D, i);
+    uint32_t run = C->hub_cursor + c.eo;
+    for (uint32_t b0 = 0; b0 < c.nr; b0 += 32) {
+      const uint32_t b = b0 + lane;
+      const uint32_t x = b < c.nr ? D.range_count[c.bo + b] : 0u;
+      const uint32_t inc = warp_incl_scan(x, (int)lane);
+      if (b < c.nr) {
+        D.range_cur[c.bo + b] = run + inc - x;
+        D.range_owner[c.bo + b] = i;
+        if (x >= 2u * kRangeSlice) {  // (a slice beyond the list's n places is left as it is)
+          const uint32_t ns = x / kRangeSlice, p0 = atomicAdd(&C->range_slices, ns);
+          for (uint32_t k = 0; k < ns && p0 + k < C->n; ++k) D.ca[p0 + k] = ((unsigned long long)(c.bo + b) << 32) | k;
+        }
+      }
+      run += __shfl_sync(kFull, inc, 31);
+    }
+  }
+}
+
+// Entries [0, cnt) at `in` added to the sums of their ids (acc[id - id0]), four in flight per thread.
+__device__ __forceinline__ void range_sum(uint32_t* acc, uint32_t id0, const unsigned long long* in, uint32_t cnt) {
+  for (uint32_t e0 = threadIdx.x; e0 < cnt; e0 += 4 * 512u) {
+    unsigned long long x[4];
+#pragma unroll
+    for (int q = 0; q < 4; ++q) x[q] = e0 + q * 512u < cnt ? in[e0 + q * 512u] : 0ull;
+#pragma unroll
+    for (int q = 0; q < 4; ++q)
+      if (e0 + q * 512u < cnt) atomicAdd(&acc[(uint32_t)(x[q] >> 32) - id0], (uint32_t)x[q]);
+  }
+}
+
+// The slices of kRangeSlice entries of long ranges, listed by k_range_place, a block each: replaced by
+// the slice's distinct ids and their sums at its front, their number in its last word (with kEmpty
+// as the id). The entries of a level's largest communities go to few next-level vertices (tens of
+// entries each), and a range holding one of those may have millions: 0.77 ms for the block that
+// emitted it alone.
+__global__ void __launch_bounds__(512) k_range_fold(int dslot) {
+  const Dev& D = c_dev[dslot];
+  Ctrl* C = D.ctrl;
+  extern __shared__ __align__(16) unsigned char smem[];
+  uint32_t* acc = reinterpret_cast<uint32_t*>(smem);
+  __shared__ uint32_t shu[33];
+  unsigned long long* arena = reinterpret_cast<unsigned long long*>(D.arena_vals);
+  const uint32_t count = min(C->range_slices, C->n);
+  for (uint32_t i = blockIdx.x; i < count; i += gridDim.x) {
+    const unsigned long long it = D.ca[i];
+    const uint32_t bk = (uint32_t)(it >> 32), sl = (uint32_t)it;
+    const RangeComm c = range_comm(D, D.range_owner[bk]);
+    unsigned long long* in = arena + (D.range_cur[bk] - D.range_count[bk]) + sl * kRangeSlice;
+    const uint32_t id0 = c.base + ((bk - c.bo) << c.log), IDS = 1u << c.log;
+    for (uint32_t k = threadIdx.x; k < (IDS + 3u) / 4u; k += 512) reinterpret_cast<uint4*>(smem)[k] = uint4{0, 0, 0, 0};
+    __syncthreads();
+    range_sum(acc, id0, in, kRangeSlice);
+    __syncthreads();
+    uint32_t own = 0;
+    for (uint32_t k = threadIdx.x; k < IDS; k += 512) own += acc[k] != 0u;
+    uint32_t total;
+    uint32_t at = block_excl_scan<uint32_t, 512>(own, shu, &total);
+    for (uint32_t k = threadIdx.x; k < IDS; k += 512)
+      if (acc[k]) in[at++] = ((unsigned long long)(id0 + k) << 32) | acc[k];
+    if (threadIdx.x == 0) in[kRangeSlice - 1u] = ((unsigned long long)kEmpty << 32) | total;  // (total <= 2^14)
+    __syncthreads();
+  }
+}
+
+// One block per range: sums in shared memory, then the nonzero ones to the community's row (positions
+// claimed with one atomic per block), k' and the self-loop as k_hub_emit.
+__global__ void __launch_bounds__(512) k_range_emit(int dslot) {
+  const Dev& D = c_dev[dslot];
+  using Acc = uint32_t;
+  using Wt = uint32_t;
+  Ctrl* C = D.ctrl;
+  extern __shared__ __align__(16) unsigned char smem[];
+  uint32_t* acc = reinterpret_cast<uint32_t*>(smem);
+  __shared__ uint32_t shu[33];
+  __shared__ double shd[33];
+  __shared__ uint32_t base_sh;
+  Wt* __restrict__ wout = reinterpret_cast<Wt*>(D.wB);
+  const unsigned long long* in = reinterpret_cast<const unsigned long long*>(D.arena_vals);
+  const uint32_t nb = C->range_buckets;
+  for (uint32_t i = blockIdx.x; i < nb; i += gridDim.x) {
+    const RangeComm c = range_comm(D, D.range_owner[i]);
+    const uint32_t cnt = D.range_count[i], first = D.range_cur[i] - cnt;  // (the cursor ended behind them)
+    const uint32_t id0 = c.base + ((i - c.bo) << c.log), IDS = 1u << c.log;
+    const uint32_t tb = (uint32_t)D.cd[c.s];
+    double ktot = 0.0, stot = 0.0;
+    if (cnt) {
+      for (uint32_t k = threadIdx.x; k < (IDS + 3u) / 4u; k += 512) reinterpret_cast<uint4*>(smem)[k] = uint4{0, 0, 0, 0};
+      __syncthreads();
+      uint32_t e = 0;
+      for (; cnt - e >= kRangeSlice && cnt >= 2u * kRangeSlice; e += kRangeSlice) {  // folded, unless the list was full
+        const unsigned long long y = in[first + e + kRangeSlice - 1u];
+        range_sum(acc, id0, in + first + e, (uint32_t)(y >> 32) == kEmpty ? (uint32_t)y : kRangeSlice);
+      }
+      range_sum(acc, id0, in + first + e, cnt - e);
+      __syncthreads();
+      uint32_t own = 0;
+      for (uint32_t k = threadIdx.x; k < IDS; k += 512) own += acc[k] != Acc(0);  // weights are positive
+      uint32_t total;
+      uint32_t at = block_excl_scan<uint32_t, 512>(own, shu, &total);
+      if (threadIdx.x == 0) base_sh = atomicAdd(&D.newdeg[c.s], total);
+      __syncthreads();
+      at += tb + base_sh;
+      double ksum = 0.0;
+      for (uint32_t k = threadIdx.x; k < IDS; k += 512) {
+        const Acc a = acc[k];
+        if (a == Acc(0)) continue;
+        const Wt x = a;
+        D.colB[at] = id0 + k;
+        wout[at] = x;
+        ++at;
+        ksum += (double)x;
+      }
+      ktot = block_sum<512>(ksum, shd);
+    }
+    if (threadIdx.x == 0) {
+      if (i == c.bo && D.hubself[c.s] != 0ull) {  // the first range also emits the self-loop
+        const unsigned long long hs = D.hubself[c.s];
+        const Wt x = (Wt)hs;
+        const uint32_t pos = atomicAdd(&D.newdeg[c.s], 1u);
+        D.colB[tb + pos] = c.s;
+        wout[tb + pos] = x;
+        ktot += (double)x;
+        stot = (double)x;
+      }
+      if (ktot != 0.0) atomicAdd(&D.kB[c.s], ktot);
+      if (stot != 0.0) atomicAdd(&D.gs[D.gidB ? D.gidB[c.s] : 0u].I, (unsigned long long)stot);
+    }
+    __syncthreads();
+  }
+}
+
 // Copy the gapped contracted rows into the dense next-level CSR (col/w), move k' and gid'.
 // The output is cut into chunks of kCompactChunk entries, one block per chunk, so a row of any
 // length is copied by as many blocks as it spans; each block stages the offsets (dense and
@@ -3346,6 +3742,9 @@ __global__ void k_agg_begin(int dslot, int force, uint32_t max_levels, int defer
     C->hub_cursor = 0;
     C->long_count = 0;  // k_hub_insert queues this aggregation's long rows from zero
     C->hub_work = 0;    // and takes its member groups from zero
+    C->range_comms = C->range_entries = C->range_buckets = C->range_slices = 0;
+    C->range_work[0] = C->range_work[1] = 0;
+    C->apply_items = 0;  // (k_range_rows queues its long rows there)
   }
   for (uint32_t g = tid; g < C->G; g += nth) {
     GraphState* st = &D.gs[g];
@@ -3377,6 +3776,9 @@ __global__ void k_agg_clear(int dslot) {
     C->hub_cursor = 0;
     C->long_count = 0;
     C->hub_work = 0;
+    C->range_comms = C->range_entries = C->range_buckets = C->range_slices = 0;
+    C->range_work[0] = C->range_work[1] = 0;
+    C->apply_items = 0;
   }
 }
 
