@@ -3,11 +3,11 @@
 // One pass of the optimisation phase (the reference's optimize() + fast_move_update() +
 // compute_modularity(), phaseOptimization.cuh:116-181) is, here:
 //   [k_chunk_flags ->] k_bin_vertices -> { k_opt_short | k_opt_team<T> x2 | k_opt_block x2 |
-//   k_opt_hub_* x4 } -> { k_apply -> k_apply_long | k_apply_hub } -> k_commit
+//   k_opt_hub_* x4 } -> { k_apply -> k_apply_long | k_apply_hub | k_apply_full } -> k_commit
 // and aggregation (phaseAggregation.cuh:19-190) with the next level's start is:
 //   k_agg_begin -> k_agg_mark -> scan x2 -> k_agg_meta -> k_agg_count -> scan x2 ->
 //   k_agg_scatter_bin -> { k_hub_* x4 | k_contract_short | k_contract_warp x2 | k_contract_block x2 |
-//   k_agg_best } -> scan x2 -> k_agg_compact -> k_agg_finish -> k_level_init -> k_commit
+//   k_agg_best | k_range_* x8 } -> scan x2 -> k_agg_compact -> k_agg_finish -> k_level_init -> k_commit
 // ({ a | b }: independent, side by side in a captured run.) A launch in the captured loop costs
 // about 4 us beyond its work, so steps that need only "all blocks done" before a few words of
 // work (scan sums, modularity and the stop rule, the loop conditions) are done by the last block
@@ -3635,15 +3635,31 @@ __global__ void __launch_bounds__(512) k_range_emit(int dslot) {
 // length is copied by as many blocks as it spans; each block stages the offsets (dense and
 // gapped) of the rows that overlap its chunk in shared memory and finds every entry's row by
 // binary search there. (Warps taking whole rows instead measured 2.8x slower: most contracted
-// rows are short.)
+// rows are short.) A chunk's rows are found by two warps, 33 parts of the offsets per step: a thread
+// bisecting for both ends, some 40 dependent loads per chunk, was most of the kernel. With four entries
+// per thread in flight as well, the first two levels of R-MAT scale 22 903 -> 416 and 319 -> 153 us (the
+// run 29.8 -> 29.1 ms), scale 20 10.46 -> 10.30 ms.
 constexpr uint32_t kCompactChunk = 2048;
+constexpr int kCompactBatch = 4;
+
+// The last row r with off[r] <= x, of n rows (off[0] = 0, x < off[n]): 33 parts per step by one warp.
+__device__ __forceinline__ uint32_t row_of(const uint32_t* __restrict__ off, uint32_t n, uint32_t x) {
+  uint32_t lo = 0, hi = n;  // off[lo] <= x < off[hi]
+  while (hi - lo > 1) {
+    const uint32_t step = (hi - lo + 32) / 33, p = lo + ((threadIdx.x & 31) + 1) * step;
+    const int c = __popc(__ballot_sync(kFull, p < hi && off[p] <= x));
+    hi = min(hi, lo + (c + 1) * step);
+    lo += c * step;
+  }
+  return lo;
+}
 
 template <bool WINT>
 __global__ void __launch_bounds__(256) k_agg_compact(int dslot) {
   const Dev& D = c_dev[dslot];
   using Wt = typename WTraits<WINT>::W;
   __shared__ uint32_t rs[kCompactChunk + 2], src0[kCompactChunk + 1];
-  __shared__ uint32_t r0_sh, nr_sh;
+  __shared__ uint32_t r0_sh, r1_sh;
   Ctrl* C = D.ctrl;
   const uint32_t n2 = C->n_next;
   const uint32_t E2 = D.rowB[n2];
@@ -3653,30 +3669,34 @@ __global__ void __launch_bounds__(256) k_agg_compact(int dslot) {
   for (uint32_t ch = blockIdx.x; ch < nchunks; ch += gridDim.x) {
     const uint32_t start = ch * kCompactChunk;
     const uint32_t end = min(start + kCompactChunk, E2);
-    if (threadIdx.x == 0) {
-      uint32_t lo = 0, hi = n2;  // last row with rowB[r] <= start
-      while (hi - lo > 1) { const uint32_t mid = (lo + hi) >> 1; if (D.rowB[mid] <= start) lo = mid; else hi = mid; }
-      uint32_t r1 = lo;           // first row with rowB[r] >= end
-      hi = n2;
-      uint32_t lo2 = lo;
-      while (hi - lo2 > 1) { const uint32_t mid = (lo2 + hi) >> 1; if (D.rowB[mid] < end) lo2 = mid; else hi = mid; }
-      r1 = lo2 + 1;
-      r0_sh = lo;
-      nr_sh = r1 - lo;  // rows lo..r1-1 overlap the chunk (every row has an entry: <= kCompactChunk)
+    if (threadIdx.x < 64) {  // the rows overlapping the chunk: at most kCompactChunk, as each has an entry
+      const uint32_t r = row_of(D.rowB, n2, threadIdx.x < 32 ? start : end - 1);
+      if ((threadIdx.x & 31) == 0) (threadIdx.x < 32 ? r0_sh : r1_sh) = r;
     }
     __syncthreads();
-    const uint32_t r0 = r0_sh, nr = nr_sh;
+    const uint32_t r0 = r0_sh, nr = r1_sh - r0_sh + 1;
     for (uint32_t i = threadIdx.x; i <= nr; i += blockDim.x) {
       rs[i] = D.rowB[r0 + i];
       if (i < nr) src0[i] = (uint32_t)D.cd[r0 + i];  // the row's start in the gapped rows
     }
     __syncthreads();
-    for (uint32_t p = start + threadIdx.x; p < end; p += blockDim.x) {
-      uint32_t lo = 0, hi = nr;  // rs[lo] <= p < rs[lo + 1]
-      while (hi - lo > 1) { const uint32_t mid = (lo + hi) >> 1; if (rs[mid] <= p) lo = mid; else hi = mid; }
-      const uint32_t src = src0[lo] + (p - rs[lo]);
-      D.col[p] = D.colB[src];
-      wout[p] = win[src];
+    for (uint32_t p0 = start + threadIdx.x; p0 < end; p0 += kCompactBatch * blockDim.x) {
+      uint32_t src[kCompactBatch], c[kCompactBatch];
+      Wt x[kCompactBatch];
+#pragma unroll
+      for (int k = 0; k < kCompactBatch; ++k) {
+        const uint32_t p = min(p0 + k * blockDim.x, end - 1);
+        uint32_t lo = 0, hi = nr;  // rs[lo] <= p < rs[lo + 1]
+        while (hi - lo > 1) { const uint32_t mid = (lo + hi) >> 1; if (rs[mid] <= p) lo = mid; else hi = mid; }
+        src[k] = src0[lo] + (p - rs[lo]);
+      }
+#pragma unroll
+      for (int k = 0; k < kCompactBatch; ++k) { c[k] = D.colB[src[k]]; x[k] = win[src[k]]; }
+#pragma unroll
+      for (int k = 0; k < kCompactBatch; ++k) {
+        const uint32_t p = p0 + k * blockDim.x;
+        if (p < end) { D.col[p] = c[k]; wout[p] = x[k]; }
+      }
     }
     __syncthreads();
   }
