@@ -73,7 +73,7 @@ def parse():
     ap.add_argument("--rates", default="10,50,200,1000,2000", help="served: arrival rates, req/s")
     ap.add_argument("--refine", action="store_true",
                     help="rmat / reference arm: Leiden-style refinement before each aggregation "
-                         "(lv_config.refine; host-driven level loop)")
+                         "(lv_config.refine; levels host-driven, passes captured)")
     ap.add_argument("--no-autotune", action="store_true",
                     help="keep the built-in degree-bin table (default: tune on a sample first)")
     ap.add_argument("--captured", type=int, default=-1, choices=[-1, 0, 1],

@@ -82,8 +82,9 @@ typedef struct {
   int32_t refine;           /* 1 = refine each level's partition before aggregating it (a
                                Leiden-style refinement behind the reference's empty
                                RefinePhase hook, phaseRefine.cuh:1-3; no reference
-                               counterpart). Host-driven runs only (use_graphs is ignored);
-                               not available to the server or lv_community_resume. Default 0 */
+                               counterpart). The levels are host-driven, the passes of a
+                               phase a captured loop (use_graphs = 1) or launched one by one
+                               (0); not available to the server or lv_community_resume. Default 0 */
   int32_t refine_passes;    /* refinement passes per level at most; 0 = until a pass raises the
                                refined partition's modularity by no more than `threshold` */
   int32_t reserved_i[5];

@@ -193,14 +193,15 @@ struct Fail {
                  std::string(#call) + ": " + cudaGetErrorString(e_)};                 \
   } while (0)
 
-// Default degree bins: team sizes 4/8/16/32 lanes with tables of 2x the bin's maximum
-// degree, a block per vertex up to 4096 entries (8K-slot shared table, several blocks per SM),
-// multi-block global tables above. lv_autotune replaces the table per workload.
+// Default degree bins: rows of up to 32 entries by all pairs in registers (one launch for the four
+// shortest bins), teams of 16 and 32 lanes with tables of 2x the bin's maximum degree up to 512, a
+// block per vertex up to 4096 entries (8K-slot shared table, several blocks per SM), multi-block
+// global tables above. lv_autotune replaces the table per workload.
 static const uint32_t kDefaultMaxDeg[kNumBins] = {4, 8, 16, 32, 128, 512, 4096, 0xFFFFFFFFu};
 
 // The autotuner's candidate tables (bins 0-6; bin 7 is open). Each moves the boundaries that
-// decide how many lanes serve a row (4 / 8 / 16 / 32 / 32 / 32 / a block / many blocks) and so
-// the table capacity each row gets (2x its bin's maximum degree, rounded to a power of two).
+// decide how many lanes serve a row (below; then a block, then many blocks) and so the table
+// capacity each row gets (2x its bin's maximum degree, rounded to a power of two).
 static const int32_t kTuneCandidates[][7] = {
     {4, 8, 16, 32, 128, 512, 4096},  {4, 8, 16, 32, 128, 512, 8192},  {4, 8, 16, 32, 128, 512, 2048},
     {8, 16, 32, 64, 128, 512, 4096}, {2, 4, 8, 16, 64, 512, 4096},    {4, 8, 16, 32, 64, 256, 4096},
@@ -284,7 +285,7 @@ class Run {
   std::vector<Block> owned;
   uint64_t arena_slots = 0;
   int grid_n = 0;           // blocks for vertex-parallel kernels
-  int grid_sq = 0;          // blocks of k_commit_sq (partials)
+  int grid_sq = 0;          // blocks of k_commit (partials)
   int grid_team[6] = {0};
   int grid_block[2] = {0};
   int grid_short = 0;
