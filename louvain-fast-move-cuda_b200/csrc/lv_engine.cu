@@ -785,7 +785,7 @@ class Run {
     full_walk = E >= kFullMinE;
     ranges = wint && E >= kRangeMinE;
     if (ranges) {
-      const size_t nr = (size_t)E / kRangeMin + 64;
+      const size_t nr = range_room(E);
       D.range_owner = dalloc<uint32_t>(ctx, owned, nr, st);
       D.range_count = dalloc<uint32_t>(ctx, owned, nr, st);
       D.range_cur = dalloc<uint32_t>(ctx, owned, nr, st);

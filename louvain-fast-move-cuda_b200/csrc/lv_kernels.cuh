@@ -68,7 +68,7 @@ struct Dev {
   // totals stay below 2m < 2^32) arrive with one gather
   unsigned long long* ca;
   // contraction by ranges: per (community, range) its community's index, entry count, write cursor
-  uint32_t *range_owner, *range_count, *range_cur;  // [E / kRangeMin + 64]
+  uint32_t *range_owner, *range_count, *range_cur;  // [range_room(E)]
   // refinement (allocated only when it is on; lv_refine.cuh)
   uint32_t* ref;             // [n] refined partition
   uint32_t* ref_new;         // [n] its pass targets
@@ -119,6 +119,17 @@ __host__ __device__ __forceinline__ uint32_t range_log(uint32_t dsum, uint32_t i
   while ((1u << log) < per) ++log;
   return log;  // (ids + 2^log - 1) >> log ranges, at most nr
 }
+// Ranges of a bin-7 community of dsum entries among `ids` next-level vertices; 0: it is not contracted
+// by ranges but in a global table (max_log < 1: none is). A community of fewer than kRangeMin entries
+// never is, wherever the configured degree bins let bin 7 begin: every range then stands for at
+// least kRangeMin entries, so that all ranges of a level fit range_room.
+__host__ __device__ __forceinline__ uint32_t range_buckets(uint32_t dsum, uint32_t ids, int max_log) {
+  if (max_log < 1 || dsum < kRangeMin) return 0;
+  const uint32_t log = range_log(dsum, ids);
+  return log <= (uint32_t)max_log ? (ids + (1u << log) - 1u) >> log : 0u;
+}
+// Room for the ranges of all communities of a level of E entries.
+__host__ __device__ __forceinline__ uint32_t range_room(uint32_t E) { return E / kRangeMin; }
 constexpr uint32_t kRangeLongRow = 1024;  // longer member rows: a block per 8192-entry piece
 
 // Capacity of a bin-7 vertex's global optimisation table: table_cap rounded up to a whole
@@ -2492,11 +2503,9 @@ __global__ void __launch_bounds__(256) k_agg_scatter_bin(int dslot, BinCfg B, in
         // a bin-6 community whose table fits half the block table: the half-block list
         if (bin == kNumBins - 2 && 2u * cap <= B.block_cap) bin = kHalfBin;
         // a bin-7 community with entries enough per range of next-level ids: contracted by ranges
-        // (max_log > 0: on)
-        if (bin == kNumBins - 1 && max_log > 0) {
-          const uint32_t ids = D.gs[g].n_next, log = range_log(dsum, ids);
-          const uint32_t nr = (ids + (1u << log) - 1u) >> log;
-          if (log <= (uint32_t)max_log) {
+        if (bin == kNumBins - 1) {
+          const uint32_t nr = range_buckets(dsum, D.gs[g].n_next, max_log);
+          if (nr > 0) {
             const uint32_t i = atomicAdd(&C->range_comms, 1u);
             const uint32_t eo = atomicAdd(&C->range_entries, dsum), bo = atomicAdd(&C->range_buckets, nr);
             D.movers[i] = s;  // (free between passes, as are cn and active_it)
