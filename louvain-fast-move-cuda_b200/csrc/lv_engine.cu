@@ -6,6 +6,7 @@
 // phaseOptimization.cuh:50-68, and 2E entries per modularity evaluation, community.h:69,85).
 // The level loop mirrors ModularityAlgorithms::modularity_routine (modularityAlgorithms.h:
 // 14-81); each pass is a fixed kernel sequence whose sizes live on the device.
+#include <cuda.h>  // types only: the driver is reached through cudaGetDriverEntryPoint
 #include <cuda_runtime.h>
 
 #include <algorithm>
@@ -243,6 +244,35 @@ static T* dalloc(lv_context* ctx, std::vector<Block>& owned, size_t count, cudaS
   return reinterpret_cast<T*>(p);
 }
 
+// Whether kernels on `device` can read `bytes` bytes at p as elements of `align` bytes where they are: an
+// aligned address in that device's own memory, all of it inside one allocation. Everything else
+// that a copy takes, or refuses with an error -- another GPU's memory, pinned or managed memory, an odd
+// address, an array that ends early -- is left to a copy.
+static bool readable_in_place(int device, const void* p, size_t bytes, size_t align) {
+  if (reinterpret_cast<uintptr_t>(p) % align != 0) return false;
+  cudaPointerAttributes a{};
+  if (cudaPointerGetAttributes(&a, p) != cudaSuccess) {
+    cudaGetLastError();
+    return false;
+  }
+  if (a.type != cudaMemoryTypeDevice || a.device != device) return false;
+  using RangeFn = CUresult (*)(CUdeviceptr*, size_t*, CUdeviceptr);
+  static const RangeFn range_of = [] {
+    void* fn = nullptr;
+    cudaDriverEntryPointQueryResult found;
+    if (cudaGetDriverEntryPoint("cuMemGetAddressRange", &fn, cudaEnableDefault, &found) != cudaSuccess ||
+        found != cudaDriverEntryPointSuccess) {
+      cudaGetLastError();
+      fn = nullptr;
+    }
+    return reinterpret_cast<RangeFn>(fn);
+  }();
+  CUdeviceptr base = 0;
+  size_t size = 0;
+  const CUdeviceptr at = reinterpret_cast<CUdeviceptr>(p);
+  return range_of && range_of(&base, &size, at) == CUDA_SUCCESS && at - base <= size && bytes <= size - (at - base);
+}
+
 // Raises a kernel's dynamic shared-memory limit to at least `bytes` on the current device.
 // The limit is per process and device, and runs on several host threads (the serving loop)
 // launch the same kernels with different table sizes, so it only ever grows: lowering it for
@@ -469,13 +499,24 @@ class Run {
     }
     allocate(G_, n_, E64);
     // host arrays are uploaded into the engine's buffers; device arrays are read where they lie
-    // (k_prep writes the engine's copy of the columns and weights as it validates them)
+    // (k_prep writes the engine's copy of the columns and weights as it validates them), unless the
+    // kernels cannot read them there: those are copied
     PrepIn in{reinterpret_cast<const long long*>(row_ptr), reinterpret_cast<const uint32_t*>(col), w, nullptr, 0};
     if (in_mem != LV_MEM_DEVICE) {
       if (w) LV_CUDA(stage->to_device(D.w, w, (size_t)E * 4, st));
       LV_CUDA(stage->to_device(D.col, col, (size_t)E * 4, st));
       LV_CUDA(stage->to_device(row64(), row_ptr, (size_t)(n + 1) * 8, st));
       in = uploaded(w != nullptr);
+    } else {
+      const PrepIn own = uploaded(w != nullptr);
+      auto copied = [&](const void* p, void* buf, size_t bytes, size_t align) {
+        if (readable_in_place(ctx->device, p, bytes, align)) return false;
+        LV_CUDA(cudaMemcpyAsync(buf, p, bytes, cudaMemcpyDeviceToDevice, st));
+        return true;
+      };
+      if (w && copied(w, D.w, (size_t)E * 4, 4)) in.wf = own.wf;
+      if (copied(col, D.col, (size_t)E * 4, 4)) in.col = own.col;
+      if (copied(row_ptr, row64(), (size_t)(n + 1) * 8, 8)) in.row64 = own.row64;
     }
     choose_weight_mode(in.wf);
     long long* doffs = nullptr;
