@@ -223,25 +223,34 @@ struct Block {
 // Device allocation through the context's pool; blocks go back to the pool when the run ends.
 // A miss allocates from the device's stream-ordered pool on the run's stream (cudaMallocAsync):
 // unlike cudaMalloc it does not synchronise the device, so a serving slot that meets a new
-// size does not stall the batches running on the other slots' streams.
-template <class T>
-static T* dalloc(lv_context* ctx, std::vector<Block>& owned, size_t count, cudaStream_t st) {
-  if (count == 0) count = 1;
-  const size_t bytes = ((count * sizeof(T) + 255) / 256) * 256;
+// size does not stall the batches running on the other slots' streams. Where there is no memory,
+// `drain` gives the pool's blocks back to the device and tries once more, then throws (it waits for
+// the whole device, and the other slots' next runs have to allocate again); without it: nullptr.
+static void* block_or_null(lv_context* ctx, std::vector<Block>& owned, size_t bytes, cudaStream_t st, bool drain) {
   size_t got = bytes;
   void* p = ctx->take(bytes, &got);
   if (!p) {
     got = bytes;
     cudaError_t e = cudaMallocAsync(&p, bytes, st);
-    if (e == cudaErrorMemoryAllocation && !ctx->pool_empty()) {
+    if (e == cudaErrorMemoryAllocation && drain && !ctx->pool_empty()) {
       cudaGetLastError();
       ctx->drain_pool();
       e = cudaMallocAsync(&p, bytes, st);
     }
+    if (e == cudaErrorMemoryAllocation && !drain) {
+      cudaGetLastError();
+      return nullptr;
+    }
     LV_CUDA(e);
   }
   owned.push_back({p, got});
-  return reinterpret_cast<T*>(p);
+  return p;
+}
+template <class T>
+static size_t block_bytes(size_t count) { return ((std::max<size_t>(count, 1) * sizeof(T) + 255) / 256) * 256; }
+template <class T>
+static T* dalloc(lv_context* ctx, std::vector<Block>& owned, size_t count, cudaStream_t st) {
+  return reinterpret_cast<T*>(block_or_null(ctx, owned, block_bytes<T>(count), st, true));
 }
 
 // Whether kernels on `device` can read `bytes` bytes at p as elements of `align` bytes where they are: an
@@ -910,20 +919,21 @@ class Run {
     set_arena(slots);
   }
   static constexpr uint64_t kArenaGuess = 48ull << 20;  // slots: 384 MB of packed ones
+  // An arena of `slots` slots if the pool or the device has the memory to spare: no other slot's pooled
+  // blocks are given up for it.
   bool try_arena(uint64_t slots) {
-    try {
-      if (!wint) D.arena_keys = dalloc<uint32_t>(ctx, arena_blocks, slots, st);
-      D.arena_vals = dalloc<unsigned long long>(ctx, arena_blocks, slots, st);
-      D.hub_owner = dalloc<uint32_t>(ctx, arena_blocks, slots / kHubChunk + 1, st);
-    } catch (const Fail&) {
-      cudaGetLastError();
-      sync();
+    void* keys = wint ? nullptr : block_or_null(ctx, arena_blocks, block_bytes<uint32_t>(slots), st, false);
+    void* vals = wint || keys ? block_or_null(ctx, arena_blocks, block_bytes<unsigned long long>(slots), st, false) : nullptr;
+    void* owner = vals ? block_or_null(ctx, arena_blocks, block_bytes<uint32_t>(slots / kHubChunk + 1), st, false) : nullptr;
+    if (!owner) {
+      sync();  // (pooled blocks are any stream's)
       for (const Block& b : arena_blocks) ctx->give(b.p, b.bytes);
       arena_blocks.clear();
-      D.arena_keys = nullptr;
-      D.arena_vals = nullptr;
       return false;
     }
+    D.arena_keys = reinterpret_cast<uint32_t*>(keys);
+    D.arena_vals = vals;
+    D.hub_owner = reinterpret_cast<uint32_t*>(owner);
     set_arena(slots);
     return true;
   }
