@@ -284,8 +284,9 @@ lv_status lv_ingest_destroy(lv_ingest* g);
 
 /* ---- serving ---------------------------------------------------------------------------
  * Continuous batching with graph state resident in HBM. No reference counterpart.
- * Requests are admitted while the device memory they need fits `budget_bytes` and a slot is
- * free (1 <= max_slots <= 64); a free slot takes the request at the head of the queue and the
+ * Requests are admitted while the device memory they need (estimated from their size: 16 bytes per
+ * CSR entry, 124 per vertex) fits `budget_bytes` and a slot is
+ * free (1 <= max_slots <= 64); hash tables taken ahead of need count against it too; a free slot takes the request at the head of the queue and the
  * other queued small requests (up to 4M entries each) as one batch, and slots run concurrently
  * on their own streams. With cfg.use_graphs each slot replays one captured level loop. */
 typedef struct lv_server lv_server;

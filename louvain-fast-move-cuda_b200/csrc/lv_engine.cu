@@ -15,6 +15,7 @@
 #include <cstdio>
 #include <cstdlib>
 #include <cstring>
+#include <functional>
 #include <map>
 #include <memory>
 #include <mutex>
@@ -339,6 +340,8 @@ class Run {
   bool ranges = false;         // large communities may be contracted by ranges
   bool full_walk = false;      // some level can have a heavy pass (later levels have fewer entries)
   bool small_ok = false;       // a whole run from its input: k_small may take its small graphs
+  // asked before the run takes that many bytes ahead of its need (ensure_arena); empty: always allowed
+  std::function<bool(size_t)> may_spare;
   int32_t levels_run = 0;
   double t_opt_ms = 0, t_agg_ms = 0, t_opt0 = -1, t_agg0 = -1, t_optk_ms = 0;
   int64_t launches = 0;
@@ -911,7 +914,7 @@ class Run {
     // does not stop for a larger arena in its first aggregation (0.5 ms a stop: a sixth of a run
     // of 300,000 vertices). Bounded, and only if the memory is there.
     const uint64_t guess = std::min<uint64_t>(2ull * E, kArenaGuess);
-    if (arena_slots == 0 && slots < guess && try_arena(guess)) return;
+    if (arena_slots == 0 && slots < guess && (!may_spare || may_spare(guess * (wint ? 8 : 12))) && try_arena(guess)) return;
     slots = std::min<uint64_t>(slots, 0xFFFFFFFEull);
     if (!wint) D.arena_keys = dalloc<uint32_t>(ctx, arena_blocks, slots, st);  // packed slots otherwise
     D.arena_vals = dalloc<unsigned long long>(ctx, arena_blocks, slots, st);

@@ -40,8 +40,10 @@ struct Request {
   std::chrono::steady_clock::time_point t_submit, t_done;
 };
 
-// Device bytes a run of this size holds: 16 B per CSR entry (two entry buffers of destination
-// and weight) and about 124 B per vertex of state and scratch, plus the control block.
+// Device bytes that a request is admitted for: 16 B per CSR entry (two entry buffers of destination
+// and weight) and 124 B per vertex of state and scratch, plus the control block. (What hash tables a
+// level turns out to need comes on top; what a run would like to have ahead of that need is taken
+// only as far as the budget has room: lv_server::spare.)
 inline size_t footprint(int64_t n, int64_t E) {
   return (size_t)E * 16 + (size_t)n * 124 + (size_t)(1u << 20) + sizeof(Ctrl);
 }
@@ -136,10 +138,35 @@ struct lv_server {
     }
   }
 
+  // Bytes that a batch admitted with est_bytes takes ahead of its need count against the budget like
+  // the batch itself, and stay within its slot's share of the budget, so that they keep no later
+  // request of up to that share waiting, nor the one at the head of the queue.
+  bool spare(size_t est_bytes, size_t bytes) {
+    std::lock_guard<std::mutex> lk(mu);
+    if ((int64_t)(est_bytes + bytes) > budget / max_slots) return false;
+    const int64_t head = queue.empty() ? 0 : (int64_t)queue.front()->est_bytes;
+    if (used_bytes + (int64_t)bytes + head > budget) return false;
+    used_bytes += (int64_t)bytes;
+    return true;
+  }
+
   void run_batch(const std::vector<lv::Request*>& batch, int slot) {
+    size_t est = 0, spared = 0;
+    for (const lv::Request* r : batch) est += r->est_bytes;
+    run_admitted(batch, slot, est, spared);  // (the run has given its memory back when it returns)
+    std::lock_guard<std::mutex> lk(mu);
+    used_bytes -= (int64_t)spared;
+  }
+
+  void run_admitted(const std::vector<lv::Request*>& batch, int slot, size_t est, size_t& spared) {
     try {
       lv::Run run(ctx, streams[slot], pinned[slot], dslots[slot].get(), stagers[slot].get());
       run.small_ok = true;
+      run.may_spare = [&](size_t bytes) {
+        if (!spare(est, bytes)) return false;
+        spared += bytes;
+        return true;
+      };
       std::vector<lv::Run::Piece> ps;
       ps.reserve(batch.size());
       for (lv::Request* r : batch) {
