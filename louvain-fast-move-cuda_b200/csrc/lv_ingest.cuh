@@ -750,22 +750,32 @@ lv_status lv_ingest_info(const lv_ingest* g, int64_t* n_nodes, int64_t* n_links,
   return LV_OK;
 }
 
+// A copy is ordered as cudaMemcpy orders it: behind what the caller has queued on the default stream
+// for the destination. It does not wait for other calls of the context: into device memory it needs
+// nothing of the context's, and into host memory it goes through the context's pinned buffers and stream
+// only while no other call has them. (On return it is done: the CSR may be destroyed, and its memory
+// another run's.)
 lv_status lv_ingest_copy_csr(const lv_ingest* g, int64_t* row_ptr, int32_t* col, int32_t out_mem) {
   if (!g || !row_ptr || !col) return LV_ERR_ARGUMENT;
   lv_context* ctx = g->ctx;
-  std::lock_guard<std::mutex> lk(ctx->mu);
-  return guarded(ctx, [&] {
-    cudaSetDevice(ctx->device);
-    const size_t rb = (size_t)(g->n + 1) * 8, cb = (size_t)g->E * 4;
-    if (out_mem == LV_MEM_DEVICE) {
-      LV_CUDA(cudaMemcpyAsync(row_ptr, g->row_ptr, rb, cudaMemcpyDeviceToDevice, ctx->stream));
-      LV_CUDA(cudaMemcpyAsync(col, g->col, cb, cudaMemcpyDeviceToDevice, ctx->stream));
-    } else {
+  const size_t rb = (size_t)(g->n + 1) * 8, cb = (size_t)g->E * 4;
+  cudaSetDevice(ctx->device);
+  std::unique_lock<std::mutex> lk(ctx->mu, std::defer_lock);
+  if (out_mem != LV_MEM_DEVICE && lk.try_lock())
+    return guarded(ctx, [&] {
+      LV_CUDA(cudaEventRecord(ctx->ev[3], cudaStreamLegacy));
+      LV_CUDA(cudaStreamWaitEvent(ctx->stream, ctx->ev[3], 0));
       LV_CUDA(ctx->stager.to_host(row_ptr, g->row_ptr, rb, ctx->stream));
       LV_CUDA(ctx->stager.to_host(col, g->col, cb, ctx->stream));
-    }
-    LV_CUDA(cudaStreamSynchronize(ctx->stream));
-  });
+      LV_CUDA(cudaStreamSynchronize(ctx->stream));
+    });
+  const cudaMemcpyKind k = out_mem == LV_MEM_DEVICE ? cudaMemcpyDeviceToDevice : cudaMemcpyDeviceToHost;
+  if (cudaMemcpy(row_ptr, g->row_ptr, rb, k) != cudaSuccess || cudaMemcpy(col, g->col, cb, k) != cudaSuccess ||
+      cudaStreamSynchronize(cudaStreamLegacy) != cudaSuccess) {
+    cudaGetLastError();
+    return LV_ERR_CUDA;
+  }
+  return LV_OK;
 }
 
 lv_status lv_ingest_run(lv_ingest* g, int32_t* out_comm, int32_t out_mem, double* out_modularity, lv_stats* stats) {
