@@ -690,6 +690,7 @@ static void ingest_run(lv_context* ctx, const char* text_in, int64_t len, int32_
   k_rows_warpn<32><<<grid, 256, 0, st>>>(rstart, cntr, mid32, cls + 3, buf, ulen);
   k_rows_block<<<ctx->sms * 2, kIngestBlockNT, 0, st>>>(rstart, cntr, mid, cls, buf, ulen);
   LV_CUDA(cudaStreamSynchronize(st));
+  bval.reset();  // (its block serves the CSR's destinations)
   DevBuf bbm(ctx);
   if (hcls[1] > 0) {
     // a bitmap per block, each as wide as the whole id range; blocks limited to 1 GiB of them
