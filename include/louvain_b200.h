@@ -275,11 +275,14 @@ lv_status lv_ingest_edge_list(lv_context* ctx, const char* text, int64_t len, in
 /* n_nodes, n_links (graphHost.cuh:8-9), CSR entries (2 n_links), min_id (graphHost.cuh:11). */
 lv_status lv_ingest_info(const lv_ingest* g, int64_t* n_nodes, int64_t* n_links, int64_t* entries,
                          int64_t* min_id);
-/* row_ptr int64[n_nodes + 1], col int32[entries], into host or device memory. */
+/* row_ptr int64[n_nodes + 1], col int32[entries], into host or device memory, ordered behind the default
+ * stream's work (as cudaMemcpy); does not wait for other calls of the context. */
 lv_status lv_ingest_copy_csr(const lv_ingest* g, int64_t* row_ptr, int32_t* col, int32_t out_mem);
 /* lv_run_csr on the ingested graph without leaving the device. */
 lv_status lv_ingest_run(lv_ingest* g, int32_t* out_comm, int32_t out_mem, double* out_modularity,
                         lv_stats* stats);
+/* Up to 1 GiB of an ingest's device memory is kept for the context's next one, until lv_destroy or
+ * until an allocation needs it; the rest is freed. */
 lv_status lv_ingest_destroy(lv_ingest* g);
 
 /* ---- serving ---------------------------------------------------------------------------

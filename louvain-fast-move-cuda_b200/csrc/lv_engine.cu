@@ -124,6 +124,53 @@ struct DevSlot {
 
 }  // namespace lv
 
+namespace lv {
+
+// Free device blocks by size, handed out again by any of a context's streams. Every block came from
+// cudaMallocAsync, and the work on it is done when it comes back.
+struct BlockPool {
+  explicit BlockPool(size_t most) : limit(most) {}
+  const size_t limit;  // bytes it keeps at most
+  std::multimap<size_t, void*> blocks;
+  size_t bytes = 0;
+  std::mutex mu;  // runs of the serving loop allocate concurrently
+
+  // A pooled block of at least `want` bytes (and not wastefully larger), or nullptr; *got = its size.
+  void* take(size_t want, size_t* got) {
+    std::lock_guard<std::mutex> lk(mu);
+    auto it = blocks.lower_bound(want);
+    if (it != blocks.end() && it->first <= want * 2 + (1u << 20)) {
+      void* p = it->second;
+      *got = it->first;
+      bytes -= it->first;
+      blocks.erase(it);
+      return p;
+    }
+    return nullptr;
+  }
+  // False: it would hold more than it may, the caller frees the block.
+  bool give(void* p, size_t size) {
+    std::lock_guard<std::mutex> lk(mu);
+    if (size > limit - bytes) return false;
+    blocks.emplace(size, p);
+    bytes += size;
+    return true;
+  }
+  // Frees every block, stream-ordered on the null stream.
+  void drain() {
+    std::lock_guard<std::mutex> lk(mu);
+    for (auto& kv : blocks) cudaFreeAsync(kv.second, nullptr);
+    blocks.clear();
+    bytes = 0;
+  }
+  bool empty() {
+    std::lock_guard<std::mutex> lk(mu);
+    return blocks.empty();
+  }
+};
+
+}  // namespace lv
+
 // A context keeps the device memory of finished runs in a pool and hands it to the next run,
 // so repeated calls allocate nothing (cudaMalloc / cudaFree synchronise the whole device).
 struct lv_context {
@@ -135,44 +182,28 @@ struct lv_context {
   cudaStream_t stream = nullptr;
   std::string err;
   std::mutex mu;
-  std::multimap<size_t, void*> pool;  // free device blocks by size
-  size_t pool_bytes = 0;
-  std::mutex pool_mu;                 // runs of the serving loop allocate concurrently
+  lv::BlockPool pool{SIZE_MAX};
+  // The buffers and CSRs of ended ingests. A program often reads one graph and is done with them, so
+  // only 1 GiB (all of an ingest of some 200 MB of text) waits for a next one; the rest goes back to the
+  // device at once.
+  lv::BlockPool ingest_pool{(size_t)1 << 30};
   uint32_t* pinned = nullptr;         // small host readbacks
   cudaEvent_t ev[8] = {};
   lv::Stager stager{4};               // host copies of calls on `stream`
 
-  // A pooled block of at least `bytes` (and not wastefully larger), or nullptr; *got = its size.
-  void* take(size_t bytes, size_t* got) {
-    std::lock_guard<std::mutex> lk(pool_mu);
-    auto it = pool.lower_bound(bytes);
-    if (it != pool.end() && it->first <= bytes * 2 + (1u << 20)) {
-      void* p = it->second;
-      *got = it->first;
-      pool_bytes -= it->first;
-      pool.erase(it);
-      return p;
-    }
-    return nullptr;
+  void give(void* p, size_t bytes) { pool.give(p, bytes); }
+  void give_ingest(void* p, size_t bytes) {
+    if (ingest_pool.give(p, bytes)) return;
+    cudaFreeAsync(p, stream);
+    cudaStreamSynchronize(stream);  // (the allocator returns memory to the device when a stream is waited for)
   }
-  void give(void* p, size_t bytes) {
-    std::lock_guard<std::mutex> lk(pool_mu);
-    pool.emplace(bytes, p);
-    pool_bytes += bytes;
-  }
-  // Every pooled block came from cudaMallocAsync: freed stream-ordered on the null stream,
-  // then the device is synchronised so that the memory is really back before a retry.
+  // The device is synchronised so that the memory is really back before a retry.
   void drain_pool() {
-    std::lock_guard<std::mutex> lk(pool_mu);
-    for (auto& kv : pool) cudaFreeAsync(kv.second, nullptr);
-    pool.clear();
-    pool_bytes = 0;
+    pool.drain();
+    ingest_pool.drain();
     cudaDeviceSynchronize();
   }
-  bool pool_empty() {
-    std::lock_guard<std::mutex> lk(pool_mu);
-    return pool.empty();
-  }
+  bool pool_empty() { return pool.empty() && ingest_pool.empty(); }
 };
 
 namespace lv {
@@ -227,9 +258,10 @@ struct Block {
 // size does not stall the batches running on the other slots' streams. Where there is no memory,
 // `drain` gives the pool's blocks back to the device and tries once more, then throws (it waits for
 // the whole device, and the other slots' next runs have to allocate again); without it: nullptr.
-static void* block_or_null(lv_context* ctx, std::vector<Block>& owned, size_t bytes, cudaStream_t st, bool drain) {
+static void* block_or_null(lv_context* ctx, BlockPool& pool, std::vector<Block>& owned, size_t bytes, cudaStream_t st,
+                           bool drain) {
   size_t got = bytes;
-  void* p = ctx->take(bytes, &got);
+  void* p = pool.take(bytes, &got);
   if (!p) {
     got = bytes;
     cudaError_t e = cudaMallocAsync(&p, bytes, st);
@@ -251,7 +283,7 @@ template <class T>
 static size_t block_bytes(size_t count) { return ((std::max<size_t>(count, 1) * sizeof(T) + 255) / 256) * 256; }
 template <class T>
 static T* dalloc(lv_context* ctx, std::vector<Block>& owned, size_t count, cudaStream_t st) {
-  return reinterpret_cast<T*>(block_or_null(ctx, owned, block_bytes<T>(count), st, true));
+  return reinterpret_cast<T*>(block_or_null(ctx, ctx->pool, owned, block_bytes<T>(count), st, true));
 }
 
 // Whether kernels on `device` can read `bytes` bytes at p as elements of `align` bytes where they are: an
@@ -925,9 +957,9 @@ class Run {
   // An arena of `slots` slots if the pool or the device has the memory to spare: no other slot's pooled
   // blocks are given up for it.
   bool try_arena(uint64_t slots) {
-    void* keys = wint ? nullptr : block_or_null(ctx, arena_blocks, block_bytes<uint32_t>(slots), st, false);
-    void* vals = wint || keys ? block_or_null(ctx, arena_blocks, block_bytes<unsigned long long>(slots), st, false) : nullptr;
-    void* owner = vals ? block_or_null(ctx, arena_blocks, block_bytes<uint32_t>(slots / kHubChunk + 1), st, false) : nullptr;
+    void* keys = wint ? nullptr : block_or_null(ctx, ctx->pool, arena_blocks, block_bytes<uint32_t>(slots), st, false);
+    void* vals = wint || keys ? block_or_null(ctx, ctx->pool, arena_blocks, block_bytes<unsigned long long>(slots), st, false) : nullptr;
+    void* owner = vals ? block_or_null(ctx, ctx->pool, arena_blocks, block_bytes<uint32_t>(slots / kHubChunk + 1), st, false) : nullptr;
     if (!owner) {
       sync();  // (pooled blocks are any stream's)
       for (const Block& b : arena_blocks) ctx->give(b.p, b.bytes);

@@ -519,7 +519,7 @@ struct lv_ingest {
 
 namespace lv {
 
-// A buffer of the context's pool, on the context's stream (an ingest uses some twenty; with a
+// A buffer of the context's ingest pool, on the context's stream (an ingest uses some twenty; with a
 // cudaMalloc and a synchronising cudaFree for each they cost more than the kernels). It goes back to
 // the pool, whose blocks any stream may take next, so reset() and the destructor may only run once the
 // work on it is done: ingest_run synchronises before it leaves, on errors too.
@@ -534,14 +534,14 @@ struct DevBuf {
   void reset() {
     if (!p) return;
     cudaStreamSynchronize(ctx->stream);
-    ctx->give(p, bytes);
+    ctx->give_ingest(p, bytes);
     p = nullptr;
   }
   template <class T>
   T* alloc(size_t count) {
     reset();
     std::vector<Block> b;
-    dalloc<T>(ctx, b, count, ctx->stream);
+    block_or_null(ctx, ctx->ingest_pool, b, block_bytes<T>(count), ctx->stream, true);
     p = b[0].p;
     bytes = b[0].bytes;
     return reinterpret_cast<T*>(p);
@@ -788,8 +788,8 @@ lv_status lv_ingest_run(lv_ingest* g, int32_t* out_comm, int32_t out_mem, double
 lv_status lv_ingest_destroy(lv_ingest* g) {
   if (!g) return LV_ERR_ARGUMENT;
   // (every call that reads the CSR waits for its work)
-  if (g->row_ptr) g->ctx->give(g->row_ptr, g->row_bytes);
-  if (g->col) g->ctx->give(g->col, g->col_bytes);
+  if (g->row_ptr) g->ctx->give_ingest(g->row_ptr, g->row_bytes);
+  if (g->col) g->ctx->give_ingest(g->col, g->col_bytes);
   delete g;
   return LV_OK;
 }

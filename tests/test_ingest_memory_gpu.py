@@ -40,3 +40,27 @@ def test_taken(lv):
     ing.close()
     eng.close()
     assert taken <= text.size + 2 * pairs * 12 + n * 40 + 64 * MB, taken // MB
+
+
+def test_kept(lv):
+    """After it, the engine keeps no more than a gigabyte, whatever it was; and a small ingest's buffers, which
+    the next one takes again."""
+    small, large = _text(lv, 200_000, 1_000_000), _text(lv, 1_000_000, 45_000_000)
+    eng = _warm(lv)
+    start = _free()
+    eng.ingest(small).close()
+    one = start - _free()
+    eng.ingest(small).close()
+    assert start - _free() == one
+    ing = eng.ingest(large)
+    want = ing.csr()
+    ing.close()
+    assert start - _free() <= 1024 * MB + 64 * MB, (start - _free()) // MB
+    again = eng.ingest(large)
+    got = again.csr()
+    np.testing.assert_array_equal(got.row_ptr, want.row_ptr)
+    np.testing.assert_array_equal(got.col, want.col)
+    again.close()
+    assert start - _free() <= 1024 * MB + 64 * MB, (start - _free()) // MB
+    eng.close()
+    assert start - _free() <= 64 * MB
