@@ -107,8 +107,8 @@ struct Ctrl {
   uint32_t hub_work;           // aggregation: next group of bin-7 members a k_hub_insert warp takes
   uint32_t hub_items;          // pass: pieces of the bin-7 (global-table) vertices' rows
   uint32_t apply_items;        // pass: pieces of the rows of movers found by block kernels
-  uint32_t hub_cursor;         // global hash-table arena cursor (slots)
   uint32_t arena_slots;        // arena capacity (slots)
+  unsigned long long hub_cursor;  // global hash-table arena cursor (slots; an aggregation may ask for more than 2^32)
   uint32_t n_next, E_next;     // aggregation outputs
   uint32_t n_chunks;           // chunk early-return emulation (single graph)
   uint32_t chunk_lo[kMaxChunks + 1];

@@ -1259,13 +1259,13 @@ class Run {
         k_ref_prev<<<grid_n, 256, 0, st>>>(Dd);
         launches += 2;
       }
-      const uint32_t need = ctrl_u32(offsetof(Ctrl, hub_cursor)) + ctrl_u32(offsetof(Ctrl, range_entries));
+      const uint64_t need = read_ctrl<unsigned long long>(offsetof(Ctrl, hub_cursor)) + ctrl_u32(offsetof(Ctrl, range_entries));
       if (debug) {
         uint32_t bc[kNumBins];
         LV_CUDA(cudaMemcpy(bc, reinterpret_cast<char*>(D.ctrl) + offsetof(Ctrl, bin_count), sizeof(bc), cudaMemcpyDeviceToHost));
         std::fprintf(stderr, "[lv] contract n=%u E=%u -> n'=%u bins", n, E, n2);
         for (uint32_t b : bc) std::fprintf(stderr, " %u", b);
-        std::fprintf(stderr, " hub_slots=%u\n", need);
+        std::fprintf(stderr, " hub_slots=%llu\n", (unsigned long long)need);
       }
       ensure_arena(need);
       agg_contract_b<WI>();

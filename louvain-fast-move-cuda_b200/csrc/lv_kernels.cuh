@@ -139,6 +139,11 @@ __device__ __forceinline__ uint32_t hub_table_cap(uint32_t d, uint32_t ng) {
   return c < kHubChunk ? kHubChunk : c;
 }
 
+// Slots of the arena that the global tables of this pass or aggregation take.
+__device__ __forceinline__ uint32_t hub_slots(const Ctrl* C) {
+  return (uint32_t)min(C->hub_cursor, (unsigned long long)C->arena_slots);
+}
+
 // Error bits found by a kernel, and which kernel found them (Ctrl::err_site, bit `site`), so
 // that a failed device check names the kernel.
 __device__ __forceinline__ void report_err(Ctrl* C, uint32_t err, int site) {
@@ -316,9 +321,9 @@ __global__ void __launch_bounds__(kBinNT) k_bin_vertices(int dslot, BinCfg B, in
           // whole number of kHubChunk-slot chunks, each chunk recording its owner
           if (want_off) {
             const uint32_t hc = cap[j] < kHubChunk ? kHubChunk : cap[j];
-            const uint32_t off = atomicAdd(&C->hub_cursor, hc);
-            D.hub_off[pos] = off;
-            if ((unsigned long long)off + hc <= C->arena_slots)
+            const unsigned long long off = atomicAdd(&C->hub_cursor, (unsigned long long)hc);
+            D.hub_off[pos] = (uint32_t)off;
+            if (off + hc <= C->arena_slots)
               for (uint32_t q = 0; q < hc / kHubChunk; ++q) D.hub_owner[off / kHubChunk + q] = pos;
           }
           const uint32_t np = (dd[j] + kHubPiece - 1) / kHubPiece;
@@ -1124,7 +1129,7 @@ __global__ void k_opt_hub_prep(int dslot) {
     D.hubself[i] = 0ull;
   }
   if (!C->fast) {
-    const uint32_t slots = min(C->hub_cursor, C->arena_slots);
+    const uint32_t slots = hub_slots(C);
     for (uint32_t s = tid; s < slots; s += nth) arena_clear_slot<WINT>(D, s);
   }
 }
@@ -1188,7 +1193,7 @@ __global__ void __launch_bounds__(256) k_opt_hub_eval(int dslot) {
   Ctrl* C = D.ctrl;
   if (C->fast) return;
   const bool lowest = C->rule_sort != 0;
-  const uint32_t nchunks = min(C->hub_cursor, C->arena_slots) / kHubChunk;
+  const uint32_t nchunks = hub_slots(C) / kHubChunk;
   const Acc* vals = reinterpret_cast<const Acc*>(D.arena_vals);
   for (uint32_t c = blockIdx.x; c < nchunks; c += gridDim.x) {
     const uint32_t pos = D.hub_owner[c];
@@ -2529,14 +2534,15 @@ __global__ void __launch_bounds__(256) k_agg_scatter_bin(int dslot, BinCfg B, in
     if (bin >= 0) {
       D.bins[bin][pos] = s;
       if (bin == kNumBins - 1) {
-        const uint32_t off = atomicAdd(&C->hub_cursor, cap);
+        // (beyond the arena, 2^32 slots at most, nothing is contracted: the caller looks at the cursor first)
+        const uint32_t off = (uint32_t)atomicAdd(&C->hub_cursor, (unsigned long long)cap);
         D.hub_off[pos] = off;
         D.hubtab[s] = off;
       }
     }
   }
   if (gc.on && last_block(&C->bin_ticket) && threadIdx.x == 0) {
-    const uint32_t used = __ldcg(&C->hub_cursor) + __ldcg(&C->range_entries);
+    const unsigned long long used = __ldcg(&C->hub_cursor) + __ldcg(&C->range_entries);
     const bool ok = used <= C->arena_slots;
     if (ok) {
       C->seg_contract_ok += 1;
@@ -2588,7 +2594,7 @@ __global__ void __launch_bounds__(256) k_hub_setup(int dslot) {
       D.hubself[s] = 0ull;
     }
   }
-  const uint32_t used = min(C->hub_cursor, C->arena_slots);
+  const uint32_t used = hub_slots(C);
   for (uint32_t s = blockIdx.x * blockDim.x + threadIdx.x; s < used; s += gridDim.x * blockDim.x)
     arena_clear_slot<WINT>(D, s);
 }
@@ -2773,7 +2779,7 @@ __global__ void __launch_bounds__(256) k_hub_insert_long(int dslot) {
 template <bool WINT>
 __global__ void __launch_bounds__(512) k_hub_emit(int dslot) {
   const Dev& D = c_dev[dslot];
-  const uint32_t nchunks = min(D.ctrl->hub_cursor, D.ctrl->arena_slots) / kHubChunk;
+  const uint32_t nchunks = hub_slots(D.ctrl) / kHubChunk;
   using Tr = WTraits<WINT>;
   using Acc = typename Tr::Acc;
   using Wt = typename Tr::W;
@@ -3508,7 +3514,7 @@ __global__ void __launch_bounds__(256) k_range_place(int dslot) {
   const uint32_t nwarps = (gridDim.x * blockDim.x) >> 5;
   for (uint32_t i = (blockIdx.x * blockDim.x + threadIdx.x) >> 5; i < count; i += nwarps) {
     const RangeComm c = range_comm(D, i);
-    uint32_t run = C->hub_cursor + c.eo;
+    uint32_t run = (uint32_t)C->hub_cursor + c.eo;
     for (uint32_t b0 = 0; b0 < c.nr; b0 += 32) {
       const uint32_t b = b0 + lane;
       const uint32_t x = b < c.nr ? D.range_count[c.bo + b] : 0u;
