@@ -796,7 +796,7 @@ class Run {
     uint32_t* dids = dalloc<uint32_t>(ctx, owned, ids.size(), st);
     LV_CUDA(cudaMemcpyAsync(dids, ids.data(), ids.size() * 4, cudaMemcpyHostToDevice, st));
     auto* fn = k_small<WI, kSmallNT[C], kSmallMinB[C]>;
-    const SmallCfg sc{cfg.mode, cfg.fast_first, single() ? 1 : 0, (uint32_t)std::max(0, cfg.max_levels),
+    const SmallCfg sc{cfg.mode, cfg.fast_first, (uint32_t)std::max(0, cfg.max_levels),
                       2u * (C == 0 ? kPackN : kSmallN)};
     const size_t smem = (size_t)sc.cap * opt_slot_bytes();
     ensure_dyn_smem(ctx->device, (const void*)fn, smem);

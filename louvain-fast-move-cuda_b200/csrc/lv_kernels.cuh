@@ -1687,10 +1687,6 @@ __device__ __forceinline__ void set_pass_rule(Ctrl* C, uint32_t p, int mode, int
   C->rule_sort = sort_rule;
 }
 
-__global__ void k_set_pass(Ctrl* C, uint32_t p, int mode, int fast_first) {
-  if (threadIdx.x == 0 && blockIdx.x == 0) set_pass_rule(C, p, mode, fast_first);
-}
-
 // ---- pass end: commit moves, sum_c a_c^2, modularity, stop rule, counters -------------------------
 // phaseOptimization.cuh:167-179: dQ = Q_after - Q_before; the level's passes stop when
 // dQ <= threshold (or after EARLY_STOP_LIMIT passes). `level_start` = 1 evaluates the level's

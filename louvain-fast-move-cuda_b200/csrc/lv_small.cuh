@@ -43,7 +43,7 @@ constexpr int kSmallShare = 2048;  // entries that make a further CTA of the clu
 constexpr int kSmallLists = 4;  // rows of up to 8 and 32 entries, rows for a warp, rows for a CTA
 
 struct SmallCfg {
-  int mode, fast_first, single;
+  int mode, fast_first;
   uint32_t max_levels;
   uint32_t cap;   // table slots of a CTA (2 x the class's vertex limit)
 };
@@ -639,16 +639,6 @@ __global__ void __launch_bounds__(NT, MINB) k_small(int dslot, const uint32_t* i
           ++iters;
           ++total_iters;
           moved = R.cnt->movers[par ^ 1] + R.cnt->long_movers[par ^ 1];
-          if (cfg.single && R.tid == 0) {
-            const uint32_t t = C->trace_len;
-            if (t < kTraceCap) {
-              TraceRec rec;
-              rec.level = level; rec.iteration = iters - 1; rec.n_moved = moved; rec.pad = 0;
-              rec.internal = I; rec.sum_a2 = S; rec.modularity = Q; rec.delta = dq;
-              C->trace[t] = rec;
-              C->trace_len = t + 1;
-            }
-          }
           if (!(dq > C->threshold) || iters > C->max_iterations) break;
           if (total_iters > kGuardPasses) { R.err |= kErrLoop; break; }
         }
