@@ -287,17 +287,11 @@ static T* dalloc(lv_context* ctx, std::vector<Block>& owned, size_t count, cudaS
 }
 
 // Whether kernels on `device` can read `bytes` bytes at p as elements of `align` bytes where they are: an
-// aligned address in that device's own memory, all of it inside one allocation. Everything else
-// that a copy takes, or refuses with an error -- another GPU's memory, pinned or managed memory, an odd
-// address, an array that ends early -- is left to a copy.
+// aligned address in that device's own memory, all of it allocated (an allocator that grows its
+// segments may have mapped them in many pieces, one behind the other). Everything else that a copy
+// takes, or refuses with an error -- another GPU's memory, pinned or managed memory, an odd address, an
+// array that ends early -- is left to a copy.
 static bool readable_in_place(int device, const void* p, size_t bytes, size_t align) {
-  if (reinterpret_cast<uintptr_t>(p) % align != 0) return false;
-  cudaPointerAttributes a{};
-  if (cudaPointerGetAttributes(&a, p) != cudaSuccess) {
-    cudaGetLastError();
-    return false;
-  }
-  if (a.type != cudaMemoryTypeDevice || a.device != device) return false;
   using RangeFn = CUresult (*)(CUdeviceptr*, size_t*, CUdeviceptr);
   static const RangeFn range_of = [] {
     void* fn = nullptr;
@@ -309,10 +303,22 @@ static bool readable_in_place(int device, const void* p, size_t bytes, size_t al
     }
     return reinterpret_cast<RangeFn>(fn);
   }();
-  CUdeviceptr base = 0;
-  size_t size = 0;
-  const CUdeviceptr at = reinterpret_cast<CUdeviceptr>(p);
-  return range_of && range_of(&base, &size, at) == CUDA_SUCCESS && at - base <= size && bytes <= size - (at - base);
+  CUdeviceptr at = reinterpret_cast<CUdeviceptr>(p);
+  if (at % align != 0 || !range_of) return false;
+  const CUdeviceptr end = at + bytes;
+  for (int pieces = 0; at < end; ++pieces) {
+    cudaPointerAttributes a{};
+    if (cudaPointerGetAttributes(&a, reinterpret_cast<const void*>(at)) != cudaSuccess) {
+      cudaGetLastError();
+      return false;
+    }
+    if (a.type != cudaMemoryTypeDevice || a.device != device || pieces == 4096) return false;
+    CUdeviceptr base = 0;
+    size_t size = 0;
+    if (range_of(&base, &size, at) != CUDA_SUCCESS || base + size <= at) return false;
+    at = base + size;
+  }
+  return true;
 }
 
 // Raises a kernel's dynamic shared-memory limit to at least `bytes` on the current device.

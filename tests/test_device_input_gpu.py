@@ -1,6 +1,9 @@
 """Device inputs that kernels cannot read where they lie -- at odd addresses, in pinned host memory beside
 device arrays -- give what the same arrays give from aligned device memory: they are copied first."""
 import importlib
+import os
+import subprocess
+import sys
 
 import numpy as np
 import pytest
@@ -81,3 +84,30 @@ def test_batch(row, col, lv):
     np.testing.assert_array_equal(out, want)
     np.testing.assert_array_equal(qs, q)
     np.testing.assert_array_equal(ks, k)
+
+
+SCRIPT = """
+import importlib, numpy as np, torch
+lv = importlib.import_module("louvain-fast-move-cuda_b200")
+n = 3_000_000                                       # (24 MB of row offsets and of columns)
+i = torch.arange(n, dtype=torch.int32, device="cuda")
+row = torch.arange(n + 1, dtype=torch.int64, device="cuda") * 2
+col = torch.stack([(i - 1) % n, (i + 1) % n], 1).reshape(-1).int().contiguous()
+out = torch.empty(n, dtype=torch.int32, device="cuda")
+torch.cuda.synchronize()
+eng = lv.Engine(0)
+for _ in range(2):
+    eng.run_csr(n, row, col, out=out)
+host = eng.run_csr(n, row.cpu().numpy(), col.cpu().numpy())[0]
+assert (out.cpu().numpy() == host).all()
+print("same")
+"""
+
+
+@pytest.mark.parametrize("conf", ["expandable_segments:True", "backend:cudaMallocAsync"])
+def test_allocators(conf):
+    """Arrays from allocators that map a segment in pieces, or take it from a stream-ordered pool."""
+    root = os.path.dirname(os.path.dirname(os.path.abspath(__file__)))
+    r = subprocess.run([sys.executable, "-c", SCRIPT], cwd=root, env=dict(os.environ, PYTORCH_CUDA_ALLOC_CONF=conf),
+                       capture_output=True, text=True, timeout=300)
+    assert r.returncode == 0 and r.stdout.strip() == "same", r.stderr[-2000:]
