@@ -1300,9 +1300,10 @@ constexpr uint32_t kApplyShort = 32;
 // level -- is applied by k_apply_full, which walks every row instead of the movers'. A pushed entry
 // costs 9-16 ps while the per-vertex state stays in L2 and about 33 ps beyond (kL2Vertices: 20 bytes
 // of it per vertex against 126 MB), a walked one 4-8 ps. Pushed -> walked, us: R-MAT scale 22 at 55 %
-// of the entries 1145 -> 590, at 24 % 482 -> 580; planted partition at 50 % 125 -> 180; 768 graphs
-// with 20 M vertices at 35 % 2500 -> 1540, at 19 % 1560 -> 1370, at 13 % 1100 -> 1240. Below kFullMinE
-// entries the walk's own latency (about 40 us) is not worth it.
+// of the entries 1145 -> 590, at 24 % 482 -> 580; 768 graphs with 20 M vertices at 35 % 2500 -> 1540,
+// at 19 % 1560 -> 1370, at 13 % 1100 -> 1240. Both limits come from whole-number weights; with fp32
+// weights (sums in double) the walk breaks even later than at half: planted partition at 50 % 125 ->
+// 180. Below kFullMinE entries the walk's own latency (about 40 us) is not worth it.
 constexpr uint32_t kFullMinE = 1u << 22;
 constexpr uint32_t kL2Vertices = 6000000;
 __device__ __forceinline__ bool heavy_pass(const Ctrl* C) {

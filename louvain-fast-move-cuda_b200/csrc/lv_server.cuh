@@ -41,8 +41,8 @@ struct Request {
 };
 
 // Device bytes that a request is admitted for: 16 B per CSR entry (two entry buffers of destination
-// and weight) and 124 B per vertex of state and scratch, plus the control block. (What hash tables a
-// level turns out to need comes on top; what a run would like to have ahead of that need is taken
+// and weight) and 124 B per vertex of state and scratch, plus the control block. (An estimate: the
+// vertex arrays are 168 B, 180 B in a batch; the hash tables that a level turns out to need come on top; what a run would like to have ahead of that need is taken
 // only as far as the budget has room: lv_server::spare.)
 inline size_t footprint(int64_t n, int64_t E) {
   return (size_t)E * 16 + (size_t)n * 124 + (size_t)(1u << 20) + sizeof(Ctrl);
